@@ -8,8 +8,8 @@
 //   1. a prologue kernel classifies each problem by max(m, n) into a size class, takes
 //      that class's tile configuration from the tuning table (chosen by the autotuner,
 //      gb_autotune_grouped), counts its tiles and writes the exclusive prefix sum;
-//   2. the persistent kernel (grid = SMs x resident CTAs) strides over the global tile
-//      index, finds its problem by binary search in the prefix sums and runs that
+//   2. the CTAs of the persistent kernel (grid = SMs x resident CTAs) take one global tile
+//      index after another, find its problem by a search in the prefix sums and run that
 //      configuration's tile routine.
 // Both kernels read only device memory, so a call can be captured in a CUDA graph.
 #include <cuda_runtime.h>
@@ -20,6 +20,7 @@
 #include <mutex>
 #include <vector>
 
+#include "f64_tile.cuh"
 #include "gb_common.cuh"
 #include "grouped.cuh"
 #include "profile.cuh"
@@ -30,8 +31,9 @@ namespace gb {
 struct TileCfg {
   int bm, bn, bk, tm, tn;
 };
-// Every configuration runs on 256 threads: (bm / tm) * (bn / tn) == 256.  0-3 serve both
-// element types; 4-9 (FP32 only) are the larger and rectangular tiles of the FP32 tile loop.
+// FP32 runs every configuration on 256 threads, (bm / tm) * (bn / tn) == 256; 4-9, the larger and
+// rectangular tiles, are FP32 only.  FP64 takes bm and bn of 0-3 as the largest extents of its
+// tiles (f64_tile.cuh).
 __host__ __device__ constexpr TileCfg tile_cfg(int c) {
   return c == 0 ? TileCfg{16, 16, 16, 1, 1}
        : c == 1 ? TileCfg{32, 32, 16, 2, 2}
@@ -52,21 +54,56 @@ __host__ __device__ inline int size_class(int64_t m, int64_t n) {
   return d <= 16 ? 0 : d <= 32 ? 1 : d <= 64 ? 2 : d <= 128 ? 3 : d <= 256 ? 4 : 5;
 }
 
-// Per-problem choice (GB_GROUPED_AUTO): the configuration with the least modelled time
+// Per-problem choice (GB_GROUPED_AUTO) in FP32: the configuration with the least modelled time
 //   tiles x (bm bn max(k, 1) / eff(tm tn) + overhead)
 // where eff is the measured FMA efficiency of a register tile of tm x tn elements per thread
 // relative to the 8 x 8 tile, and overhead the fixed cost of one tile (its first panel's load
 // latency, index set-up and epilogue) in the same units.  Padding rows and columns of a tile
 // cost as much as real ones, so tall and wide problems take rectangular tiles.
-__host__ __device__ inline int auto_config(int64_t m, int64_t n, int64_t k, int nconfigs) {
+__host__ __device__ inline int auto_config_f32(int64_t m, int64_t n, int64_t k) {
   float best = 3.4e38f;
   int arg = 0;
-  for (int c = 0; c < nconfigs; ++c) {
+  for (int c = 0; c < GROUPED_CONFIGS_F32; ++c) {
     const TileCfg t = tile_cfg(c);
     const int e = t.tm * t.tn;
     const float eff = e >= 64 ? 1.0f : e >= 32 ? 0.9f : e >= 16 ? 0.75f : e >= 8 ? 0.55f : e >= 4 ? 0.35f : 0.1f;
     const float tiles = static_cast<float>((m + t.bm - 1) / t.bm) * static_cast<float>((n + t.bn - 1) / t.bn);
     const float cost = tiles * (static_cast<float>(t.bm * t.bn) * static_cast<float>(k > 1 ? k : 1) / eff + 32768.0f);
+    if (cost < best) {
+      best = cost;
+      arg = c;
+    }
+  }
+  return arg;
+}
+
+// Extents of an FP64 problem's tiles under a configuration: equal tiles as large as the
+// configuration allows (33 rows on 32-row tiles: 17 + 16, not 32 + 1).
+struct F64Tiles {
+  int tm, tn, fm, fn;
+};
+__host__ __device__ inline F64Tiles f64_tiles(const TileCfg& c, int64_t m, int64_t n) {
+  F64Tiles t;
+  t.tm = static_cast<int>((m + c.bm - 1) / c.bm);
+  t.tn = static_cast<int>((n + c.bn - 1) / c.bn);
+  t.fm = t.tm > 0 ? static_cast<int>((m + t.tm - 1) / t.tm) : 0;
+  t.fn = t.tn > 0 ? static_cast<int>((n + t.tn - 1) / t.tn) : 0;
+  return t;
+}
+
+// The same in FP64, where the DFMA pipe bounds everything (f64_tile.cuh): the configuration with
+// the fewest units of 32 elements, a tile's barriers, first loads and stores counting as 26 unit-k
+// (measured on 8192 problems of 32 x 32 x 64: 1.01 ms on 16 x 16 tiles, 0.96 on 32 x 32), among those
+// whose tiles hold at most F64_MAX_ELEMS (larger ones run in strips and re-read A).
+__host__ __device__ inline int auto_config_f64(int64_t m, int64_t n, int64_t k) {
+  float best = 3.4e38f;
+  int arg = 0;
+  for (int c = 0; c < GROUPED_CONFIGS_F64; ++c) {
+    const F64Tiles t = f64_tiles(tile_cfg(c), m, n);
+    if (t.fm * t.fn > F64_MAX_ELEMS) continue;
+    const float units = static_cast<float>((t.fm * t.fn + 31) / 32);
+    const float cost = static_cast<float>(t.tm) * static_cast<float>(t.tn) *
+                       (units * static_cast<float>(k > 1 ? k : 1) + 26.0f);
     if (cost < best) {
       best = cost;
       arg = c;
@@ -83,24 +120,11 @@ __device__ __forceinline__ int config_of(const gb_grouped_tuning_t& t, int cls) 
   return v;
 }
 
-// The configuration one problem runs under (the table's, or the per-problem choice).
-template <int NCFG>
-__host__ __device__ inline int problem_config(int table_cfg, int64_t m, int64_t n, int64_t k) {
-  return table_cfg == GB_GROUPED_AUTO ? auto_config(m, n, k, NCFG) : table_cfg;
-}
 
-template <typename T>
-__device__ __forceinline__ T fmad(T a, T b, T c);
-template <>
-__device__ __forceinline__ double fmad<double>(double a, double b, double c) { return fma(a, b, c); }
-template <>
-__device__ __forceinline__ float fmad<float>(float a, float b, float c) { return fmaf(a, b, c); }
-
-constexpr int GROUPED_THREADS = 256;
-// largest shared memory of any tile routine (bytes): the double-buffered 128 x 128 x 16 FP32
-// panels of the SIMT mainloop (the FP64 16 x 64 + 16 x 65 panels take 16.5 KB)
+constexpr int GROUPED_THREADS = 256;   // FP32 (FP64: F64_THREADS)
+// largest shared memory of any FP32 tile routine (bytes): the double-buffered 128 x 128 x 16
+// panels of the SIMT mainloop
 constexpr int GROUPED_SMEM = SimtSmem<float, 128, 128, 16>::ELEMS * 4;
-static_assert(GROUPED_SMEM >= (16 * 64 + 16 * 65) * 8, "FP64 tile panels");
 
 // jmul!'s FMA chain with the alpha/beta epilogue of the grouped call (alpha != 0 here).
 template <typename T>
@@ -120,115 +144,49 @@ struct GroupedChainOp {
   __device__ __forceinline__ bool reads_c() const { return beta != T(0); }
 };
 
-// One BM x BN tile of problem `p` (column-major, no transposes).  Per element the FMA chain
-// runs k = 0..K-1 in order from -0.0 (equal to jmul!'s a1*x1 first step, bit for bit).
-// The next K slab is loaded into registers while the current one is multiplied from shared
-// memory; B's slab is stored [k][n] with rows padded by one word, so the k-fastest global
-// reads land in distinct banks.
-template <typename T, int BM, int BN, int BK, int TM, int TN>
-__device__ __forceinline__ void grouped_tile(const gb_problem_t& p, int tm, int tn, unsigned char* smem) {
-  static_assert((BM / TM) * (BN / TN) == GROUPED_THREADS, "configuration must use 256 threads");
-  constexpr int LA = (BM * BK + GROUPED_THREADS - 1) / GROUPED_THREADS;   // A elements per thread
-  constexpr int LB = (BK * BN + GROUPED_THREADS - 1) / GROUPED_THREADS;   // B elements per thread
-  constexpr int BNP = BN + 1;
-  T* As = reinterpret_cast<T*>(smem);   // [BK][BM]
-  T* Bs = As + BK * BM;                 // [BK][BN + 1]
+// One 16 x 16 FP32 tile of problem `p` (column-major, no transposes), one element a thread.  The FMA
+// chain runs k = 0..K-1 in order from -0.0 (equal to jmul!'s a1*x1 first step, bit for bit).  The
+// next 16 k are loaded into registers while the current ones are multiplied from shared memory; B's
+// slab is stored [k][n] with rows padded by one word, so the k-fastest global reads land in
+// distinct banks.
+__device__ __forceinline__ void grouped_tile_16(const gb_problem_t& p, int tm, int tn, float* smem) {
+  constexpr int D = 16;
+  float* As = smem;           // [k][m]
+  float* Bs = As + D * D;     // [k][n], rows of D + 1
   const int tid = threadIdx.x;
-  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+  const int tx = tid % D, ty = tid / D;
   const int64_t M = p.m, N = p.n, K = p.k;
-  const int64_t m0 = static_cast<int64_t>(tm) * BM, n0 = static_cast<int64_t>(tn) * BN;
-  const T* __restrict__ A = static_cast<const T*>(p.A);
-  const T* __restrict__ B = static_cast<const T*>(p.B);
-  T acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = T(-0.0);
-
-  // alpha and beta decoded once per warp (FP64 compares and conversions run on the narrow
-  // FP64 pipe) and broadcast
-  T alpha, beta;
-  bool alpha_zero, unit;   // alpha == 0; alpha == 1 and beta == 0 (C = the chain itself)
-  {
-    const int lane = threadIdx.x & 31;
-    float2 ab = make_float2(0.0f, 0.0f);
-    double ad = 0.0, bd = 0.0;
-    if (sizeof(T) == 8) {
-      ad = p.alpha;
-      bd = p.beta;
-    } else if (lane == 0) {
-      ab = make_float2(static_cast<float>(p.alpha), static_cast<float>(p.beta));
-    }
-    if (sizeof(T) == 4) {
-      ab.x = __shfl_sync(0xffffffffu, ab.x, 0);
-      ab.y = __shfl_sync(0xffffffffu, ab.y, 0);
-    }
-    alpha = (sizeof(T) == 8) ? static_cast<T>(ad) : static_cast<T>(ab.x);
-    beta = (sizeof(T) == 8) ? static_cast<T>(bd) : static_cast<T>(ab.y);
-    alpha_zero = ((__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0);
-    unit = __double_as_longlong(p.alpha) == 0x3FF0000000000000ll && __double_as_longlong(p.beta) == 0ll;
-  }
+  const int64_t m0 = static_cast<int64_t>(tm) * D, n0 = static_cast<int64_t>(tn) * D;
+  const float* __restrict__ A = static_cast<const float*>(p.A);
+  const float* __restrict__ B = static_cast<const float*>(p.B);
+  // alpha and beta converted once per warp (on the narrow FP64 pipe) and broadcast
+  float2 ab = make_float2(0.0f, 0.0f);
+  if ((tid & 31) == 0) ab = make_float2(static_cast<float>(p.alpha), static_cast<float>(p.beta));
+  const float alpha = __shfl_sync(0xffffffffu, ab.x, 0), beta = __shfl_sync(0xffffffffu, ab.y, 0);
+  const bool alpha_zero = (__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0;
+  const bool unit = __double_as_longlong(p.alpha) == 0x3FF0000000000000ll && __double_as_longlong(p.beta) == 0ll;
   const int64_t Kc = alpha_zero ? 0 : K;   // alpha == 0: A and B are not read
-  T ra[LA], rb[LB];
-  auto load = [&](int64_t k0) {
-#pragma unroll
-    for (int l = 0; l < LA; ++l) {
-      const int e = tid + l * GROUPED_THREADS;
-      const int ml = e % BM, kl = e / BM;
-      const int64_t m = m0 + ml, k = k0 + kl;
-      ra[l] = (e < BM * BK && m < M && k < K) ? A[m + k * p.lda] : T(0);
-    }
-#pragma unroll
-    for (int l = 0; l < LB; ++l) {
-      const int e = tid + l * GROUPED_THREADS;
-      const int kl = e % BK, nl = e / BK;
-      const int64_t n = n0 + nl, k = k0 + kl;
-      rb[l] = (e < BK * BN && n < N && k < K) ? B[k + n * p.ldb] : T(0);
-    }
+  float acc = -0.0f, ra = 0.0f, rb = 0.0f;
+  auto load = [&](int64_t k0) {   // A: tx along m, ty along k; B: tx along k, ty along n
+    ra = (m0 + tx < M && k0 + ty < K) ? A[(m0 + tx) + (k0 + ty) * p.lda] : 0.0f;
+    rb = (n0 + ty < N && k0 + tx < K) ? B[(k0 + tx) + (n0 + ty) * p.ldb] : 0.0f;
   };
   if (Kc > 0) load(0);
-  for (int64_t k0 = 0; k0 < Kc; k0 += BK) {
-    const int kc = static_cast<int>(K - k0 < BK ? K - k0 : BK);
-#pragma unroll
-    for (int l = 0; l < LA; ++l) {
-      const int e = tid + l * GROUPED_THREADS;
-      if (e < BM * BK) As[(e / BM) * BM + e % BM] = ra[l];
-    }
-#pragma unroll
-    for (int l = 0; l < LB; ++l) {
-      const int e = tid + l * GROUPED_THREADS;
-      if (e < BK * BN) Bs[(e % BK) * BNP + e / BK] = rb[l];
-    }
+  for (int64_t k0 = 0; k0 < Kc; k0 += D) {
+    const int kc = static_cast<int>(K - k0 < D ? K - k0 : D);
+    As[ty * D + tx] = ra;
+    Bs[tx * (D + 1) + ty] = rb;
     __syncthreads();
-    if (k0 + BK < Kc) load(k0 + BK);   // in flight while this slab is multiplied
-    for (int kk = 0; kk < kc; ++kk) {
-      T a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk * BM + ty + i * (BM / TM)];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Bs[kk * BNP + tx + j * (BN / TN)];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmad<T>(a[i], b[j], acc[i][j]);
-    }
+    if (k0 + D < Kc) load(k0 + D);   // in flight while this slab is multiplied
+    for (int kk = 0; kk < kc; ++kk) acc = fmaf(As[kk * D + ty], Bs[kk * (D + 1) + tx], acc);
     __syncthreads();
   }
-  T* __restrict__ C = static_cast<T*>(p.C);
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int64_t m = m0 + ty + i * (BM / TM);
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int64_t n = n0 + tx + j * (BN / TN);
-      if (n >= N) continue;
-      T* c = &C[m + n * p.ldc];
-      if (alpha == T(0)) *c = (beta == T(0)) ? T(0) : beta * *c;   // A, B not read
-      else if (unit) *c = acc[i][j];   // jmul!'s result, without a multiply on the FP64 pipe
-      else *c = (beta == T(0)) ? alpha * acc[i][j] : fmad<T>(alpha, acc[i][j], beta * *c);
-    }
-  }
+  const int64_t m = m0 + ty, n = n0 + tx;
+  if (m >= M || n >= N) return;
+  float* c = static_cast<float*>(p.C) + m + n * p.ldc;
+  if (alpha == 0.0f) *c = (beta == 0.0f) ? 0.0f : beta * *c;
+  else if (unit) *c = acc;
+  else *c = (beta == 0.0f) ? alpha * acc : fmaf(alpha, acc, beta * *c);
 }
 
 // alpha = 0: C = beta C on one bm x bn tile (beta = 0 writes zeros without reading C; A and B
@@ -237,7 +195,7 @@ template <typename T>
 __device__ __forceinline__ void scale_tile(const gb_problem_t& p, int64_t m0, int64_t n0, int bm, int bn) {
   T* __restrict__ C = static_cast<T*>(p.C);
   const T beta = static_cast<T>(p.beta);
-  for (int e = threadIdx.x; e < bm * bn; e += GROUPED_THREADS) {
+  for (int e = threadIdx.x; e < bm * bn; e += static_cast<int>(blockDim.x)) {
     const int64_t m = m0 + e % bm, n = n0 + e / bm;
     if (m < p.m && n < p.n) {
       T* c = &C[m + n * p.ldc];
@@ -246,15 +204,18 @@ __device__ __forceinline__ void scale_tile(const gb_problem_t& p, int64_t m0, in
   }
 }
 
+// The configuration one problem runs under (the table's, or the per-problem choice).
 __device__ __forceinline__ int prologue_config(const gb_grouped_tuning_t& tuning, const gb_problem_t& p, bool f32) {
   const int c = config_of(tuning, size_class(p.m, p.n));
-  return f32 ? problem_config<GROUPED_CONFIGS_F32>(c, p.m, p.n, p.k) : problem_config<GROUPED_CONFIGS_F64>(c, p.m, p.n, p.k);
+  if (c != GB_GROUPED_AUTO) return c;
+  return f32 ? auto_config_f32(p.m, p.n, p.k) : auto_config_f64(p.m, p.n, p.k);
 }
 
 // Workspace of a call over `count` problems (int64 words): the tile prefix sums in schedule
 // order offsets[0..count], then the schedule order (count int32 entries: the problem index,
 // and for count <= 2^24 its tile configuration in bits 24-30, so the tile loop need not
-// evaluate the per-problem choice again for every tile).
+// evaluate the per-problem choice again for every tile).  The first problem's tiles start at 0, so
+// the tile loop takes that as known and counts the tiles it has handed out in offsets[0].
 __host__ __device__ inline long long* grouped_order_words(long long* ws, int count) { return ws + count + 1; }
 constexpr int GROUPED_PACK_LIMIT = 1 << 24;
 __host__ __device__ inline int grouped_order_entry(int i, int cfg, int count) {
@@ -262,9 +223,8 @@ __host__ __device__ inline int grouped_order_entry(int i, int cfg, int count) {
 }
 
 // Prologue (one block): the schedule orders the problems by the work of one of their tiles
-// (tile rows x tile columns x k, in 32 power-of-two buckets, heaviest first), so that the CTAs,
-// striding over the schedule, take tiles of similar length side by side and the short ones
-// fill the tail; it writes the order and the exclusive prefix sums of the tiles in that order.
+// (tile rows x tile columns x k, in 32 power-of-two buckets, heaviest first), so that the CTAs
+// take tiles of similar length side by side and the short ones fill the tail; it writes the order and the exclusive prefix sums of the tiles in that order.
 // The order inside a bucket depends on timing, which changes no result (each tile is
 // independent).
 __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_problem_t* __restrict__ probs, int count,
@@ -278,7 +238,12 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   if (t < 32) hist[t] = 0;
   __syncthreads();
   auto bucket_of = [&](const gb_problem_t& p, const TileCfg& c) {
-    const long long w = static_cast<long long>(c.bm) * c.bn * (p.k > 1 ? p.k : 1);
+    long long w = static_cast<long long>(c.bm) * c.bn * (p.k > 1 ? p.k : 1);
+    if (!f32) {   // FP64 tiles cost what is in them
+      const F64Tiles t = f64_tiles(c, p.m, p.n);
+      w = static_cast<long long>(t.fm) * t.fn * (p.k > 1 ? p.k : 1);
+      if (w < 1) w = 1;
+    }
     const int lg = 63 - __clzll(w);                 // w >= 1
     return 31 - (lg > 31 ? 31 : lg);                 // heavy first
   };
@@ -322,7 +287,7 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   }
   long long run = (t == 0) ? 0 : part[t - 1];
   for (int i = b; i < e; ++i) {
-    offsets[i] = run;
+    offsets[i] = run;   // offsets[0] = 0: the tile counter's start
     run += tiles_of(i);
   }
   if (t == 1023) offsets[count] = part[1023];
@@ -332,7 +297,7 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
 // tiles share their successor's offset), searched from `from` (a position with
 // offsets[from] <= w: a CTA's tiles come in increasing order, so its previous tile's position).
 // Each warp searches on its own: its 32 lanes probe 32 points of the remaining interval at
-// once, so 4096 problems take at most 3 rounds of loads instead of the 12 dependent loads of a
+// once (never offsets[0]), so 4096 problems take at most 3 rounds of loads instead of the 12 dependent loads of a
 // binary search.  Every warp reaches the same position.
 __device__ __forceinline__ int schedule_pos(const long long* __restrict__ offsets, int count, long long w, int from) {
   const int lane = threadIdx.x & 31;
@@ -354,17 +319,34 @@ __device__ __forceinline__ int schedule_pos(const long long* __restrict__ offset
   return lo;
 }
 
-// Persistent tile loop: CTA b takes tiles b, b + grid, ... of the schedule.
 template <typename T>
-__global__ void __launch_bounds__(GROUPED_THREADS, 2) grouped_gemm_kernel(const gb_problem_t* __restrict__ probs,
-                                                                       int count, gb_grouped_tuning_t tuning,
-                                                                       long long* __restrict__ ws) {
-  __shared__ __align__(16) unsigned char smem[GROUPED_SMEM];
+constexpr int grouped_threads() { return sizeof(T) == 8 ? F64_THREADS : GROUPED_THREADS; }
+
+// Persistent tile loop: CTA b takes tile b of the schedule, then the next one that no CTA has taken
+// (a counter in offsets[0]; its answer is fetched while the tile runs).  Against a fixed stride, where
+// the busiest SM of 4096 log-uniform problems gets 3.5% more than its share.
+template <typename T>
+__global__ void __launch_bounds__(grouped_threads<T>(), sizeof(T) == 8 ? F64_CTAS : 2)
+    grouped_gemm_kernel(const gb_problem_t* __restrict__ probs, int count, gb_grouped_tuning_t tuning,
+                        long long* __restrict__ ws) {
+  __shared__ __align__(16) unsigned char smem[sizeof(T) == 8 ? F64_SMEM_ELEMS * 8 : GROUPED_SMEM];
+  __shared__ long long next_tile[2];
   const long long* offsets = ws;
   const int* order = reinterpret_cast<const int*>(grouped_order_words(ws, count));
   const long long total = offsets[count];
-  int lo = 0;   // offsets[0] = 0 <= w
-  for (long long w = blockIdx.x; w < total; w += gridDim.x) {
+  int lo = 0;   // the first problem's tiles start at 0 <= w
+  long long next = 0;
+  long long w = blockIdx.x;
+  // The tile after this one, handed to all threads; the barrier also frees the shared panels.  Two
+  // slots: a slot is written again only after another such barrier.
+  auto advance = [&](int slot) {
+    if (threadIdx.x == 0) next_tile[slot] = next;
+    __syncthreads();
+    w = next_tile[slot];
+  };
+  for (int slot = 0; w < total; advance(slot), slot ^= 1) {
+    if (threadIdx.x == 0)
+      next = gridDim.x + static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(ws), 1ull));
     lo = schedule_pos(offsets, count, w, lo);
     const int e = order[lo];
     const bool packed = count <= GROUPED_PACK_LIMIT;
@@ -373,20 +355,30 @@ __global__ void __launch_bounds__(GROUPED_THREADS, 2) grouped_gemm_kernel(const 
     const TileCfg c = tile_cfg(cfg);
     // tile rows of the problem and the tile's place in it, in 32-bit arithmetic (a problem's
     // tile count is below 2^31)
-    const int local = static_cast<int>(w - offsets[lo]);
+    const int local = static_cast<int>(lo ? w - offsets[lo] : w);
     const int tiles_m = static_cast<int>((p.m + c.bm - 1) / c.bm);
     const int tn = local / tiles_m, tm = local - tn * tiles_m;
     if constexpr (sizeof(T) == 8) {
-      // FP64 runs at the DFMA rate whatever the tile: the small configurations keep the
-      // register count (and so the resident CTAs per SM) low.
-      switch (cfg) {
-        case 0: grouped_tile<T, 16, 16, 16, 1, 1>(p, tm, tn, smem); break;
-        case 1: grouped_tile<T, 32, 32, 16, 2, 2>(p, tm, tn, smem); break;
-        case 2: grouped_tile<T, 64, 32, 16, 4, 2>(p, tm, tn, smem); break;
-        default: grouped_tile<T, 64, 64, 16, 4, 4>(p, tm, tn, smem); break;
+      const F64Tiles ft = f64_tiles(c, p.m, p.n);
+      const int64_t m0 = static_cast<int64_t>(tm) * ft.fm, n0 = static_cast<int64_t>(tn) * ft.fn;
+      const int r = static_cast<int>(p.m - m0 < ft.fm ? p.m - m0 : ft.fm);
+      const int cc = static_cast<int>(p.n - n0 < ft.fn ? p.n - n0 : ft.fn);
+      if (r <= 0 || cc <= 0) continue;   // equal tiles can need one fewer
+      if ((__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0) {
+        scale_tile<T>(p, m0, n0, r, cc);
+        continue;
+      }
+      const bool unit = __double_as_longlong(p.alpha) == 0x3FF0000000000000ll && __double_as_longlong(p.beta) == 0ll;
+      const int cols = min(32, F64_MAX_ELEMS / r);   // larger tiles run in column strips
+      for (int j0 = 0; j0 < cc; j0 += cols) {
+        if (j0) __syncthreads();   // the strip reuses the shared panels
+        f64_tile_any<false>(r, min(cols, cc - j0), p.k, static_cast<const double*>(p.A) + m0, 1, p.lda,
+                            static_cast<const double*>(p.B) + (n0 + j0) * p.ldb, 1, p.ldb, p.alpha, p.beta, unit,
+                            static_cast<double*>(p.C) + m0 + (n0 + j0) * p.ldc, p.ldc, static_cast<int>(w ^ (w >> 2)),
+                            reinterpret_cast<double*>(smem));
       }
     } else if (cfg == 0) {
-      grouped_tile<T, 16, 16, 16, 1, 1>(p, tm, tn, smem);   // one element a thread
+      grouped_tile_16(p, tm, tn, reinterpret_cast<float*>(smem));
     } else if ((__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0) {
       scale_tile<T>(p, static_cast<int64_t>(tm) * c.bm, static_cast<int64_t>(tn) * c.bn, c.bm, c.bn);
     } else {
@@ -413,7 +405,6 @@ __global__ void __launch_bounds__(GROUPED_THREADS, 2) grouped_gemm_kernel(const 
         default: GB_GTILE(32, 128, 16, 2, 8); break;
       }
 #undef GB_GTILE
-      __syncthreads();   // the next tile reuses the shared panels
     }
   }
 }
@@ -422,11 +413,10 @@ gb_grouped_tuning_t grouped_default_tuning(int dtype_bytes) {
   gb_grouped_tuning_t t;
   std::memset(&t, 0, sizeof(t));
   // classes: <=16, <=32, <=64, <=128, <=256, >256
-  // FP32: the per-problem choice in every class (rectangular tiles for tall and wide problems).
-  // FP64: 16 x 16 tiles everywhere: the DFMA pipe, not the register tile, bounds FP64, and the
-  // smallest tiles pad least (the autotuner picks them in every class; 1.0 TFLOP/s against 0.71
-  // for larger tiles in the larger classes, 4096 log-uniform problems).
-  for (int c = 0; c < GB_GROUPED_CLASSES; ++c) t.config[c] = dtype_bytes == 8 ? 0 : GB_GROUPED_AUTO;
+  // The per-problem choice in every class (rectangular FP32 tiles for tall and wide problems; the
+  // FP64 tiles that pad least).
+  (void)dtype_bytes;
+  for (int c = 0; c < GB_GROUPED_CLASSES; ++c) t.config[c] = GB_GROUPED_AUTO;
   return t;
 }
 
@@ -454,7 +444,7 @@ static int grid_for(int sms) {
   }
   int per_sm = dev >= 0 ? per_sm_of[dev].load(std::memory_order_relaxed) : 0;
   if (per_sm < 1) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_gemm_kernel<T>, GROUPED_THREADS, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_gemm_kernel<T>, grouped_threads<T>(), 0) !=
             cudaSuccess ||
         per_sm < 1) {
       cudaGetLastError();
@@ -474,7 +464,7 @@ int grouped_launch(int dtype_bytes, const gb_problem_t* d_probs, int count, cons
   if (dtype_bytes == 8) {
     const int grid = grid_for<double>(sms);
     GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
-              (grouped_gemm_kernel<double><<<grid, GROUPED_THREADS, 0, s>>>(d_probs, count, tuning, d_offsets)));
+              (grouped_gemm_kernel<double><<<grid, F64_THREADS, 0, s>>>(d_probs, count, tuning, d_offsets)));
   } else {
     const int grid = grid_for<float>(sms);
     GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
@@ -624,7 +614,7 @@ int grouped_f64_noalloc(const gb_problem_t* d_probs, int count, const gb_grouped
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return gb_set_cuda_error(e, "grouped prologue launch");
   prof_count(GB_KERNEL_GROUPED_GEMM);
-  grouped_gemm_kernel<double><<<grid_for<double>(sms), GROUPED_THREADS, 0, s>>>(d_probs, count, t, offsets);
+  grouped_gemm_kernel<double><<<grid_for<double>(sms), F64_THREADS, 0, s>>>(d_probs, count, t, offsets);
   e = cudaGetLastError();
   if (e != cudaSuccess) return gb_set_cuda_error(e, "grouped launch");
   prof_count(GB_KERNEL_GROUPED_GEMM);
