@@ -954,8 +954,8 @@ static int kernel_entry(Onto onto, Init init_fn, T* D, const T* A, const T* X, i
   if (Mk == 0 || Pk == 0) return GB_OK;
   if (!is_device_ptr(D) || (N > 0 && (!is_device_ptr(A) || !is_device_ptr(X)))) return GB_ERR_INVALID_VALUE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (init) return init_fn(0, 0, Mk, Pk, N, T(1), A, sAD, X, sX, T(0), D, sAD, dev->sms, s);
-  return onto(Mk, Pk, N, A, sAD, X, sX, D, sAD, dev->sms, s);
+  if (init) return init_fn(dev, Mk, Pk, N, A, sAD, X, sX, D, sAD, s);
+  return onto(dev, Mk, Pk, N, A, sAD, X, sX, D, sAD, s);
 }
 
 // Host-buffer products: upload the stored operands (packed, leading dimension = rows), run the
@@ -1193,7 +1193,7 @@ int gb_gemm_f32(int transA, int transB, int64_t M, int64_t N, int64_t K, float a
   if (rc) return rc;
   rc = check_gemm_args(transA, transB, M, N, K, lda, ldb, ldc, A, B, C, alpha != 0.0f);
   if (rc) return rc;
-  return native_gemm_f32(transA, transB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, dev->sms,
+  return native_gemm_f32(transA, transB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, dev->sms, dev->pool,
                          static_cast<cudaStream_t>(stream));
 }
 
@@ -1209,7 +1209,7 @@ int gb_gemm_f32_ex(int transA, int transB, int64_t M, int64_t N, int64_t K, floa
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // no product to form (alpha = 0, K = 0): C = beta C exactly as the native mode does it
   if (mode == GB_MODE_NATIVE || M == 0 || N == 0 || K == 0 || alpha == 0.0f)
-    return native_gemm_f32(transA, transB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, dev->sms, s);
+    return native_gemm_f32(transA, transB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, dev->sms, dev->pool, s);
   if (tc_pair_tiles(M, N) > 0x7FFFFFFF / 2 || tc_tiles(M, N) > 0x7FFFFFFF / 2) return GB_ERR_UNSUPPORTED;
   const int nterms = (mode == GB_MODE_BF16X3) ? 2 : 3;
   void* ws = nullptr;
@@ -1222,14 +1222,28 @@ int gb_gemm_f32_ex(int transA, int transB, int64_t M, int64_t N, int64_t K, floa
 
 int gb_kernel_f64(double* pD, const double* pA, const double* pX, int64_t Mk, int64_t Pk, int64_t stride_AD,
                   int64_t stride_X, int64_t N, int init, void* stream) {
-  return kernel_entry<double>(native_kernel_onto_f64, native_gemm_f64, pD, pA, pX, Mk, Pk, stride_AD, stride_X, N,
-                              init, stream);
+  auto jmul = [](DeviceInfo* d, int64_t m, int64_t p, int64_t n, const double* A, int64_t la, const double* X,
+                 int64_t lx, double* D, int64_t ld, cudaStream_t s) {
+    return native_gemm_f64(0, 0, m, p, n, 1.0, A, la, X, lx, 0.0, D, ld, d->sms, s);
+  };
+  auto onto = [](DeviceInfo* d, int64_t m, int64_t p, int64_t n, const double* A, int64_t la, const double* X,
+                 int64_t lx, double* D, int64_t ld, cudaStream_t s) {
+    return native_kernel_onto_f64(m, p, n, A, la, X, lx, D, ld, d->sms, s);
+  };
+  return kernel_entry<double>(onto, jmul, pD, pA, pX, Mk, Pk, stride_AD, stride_X, N, init, stream);
 }
 
 int gb_kernel_f32(float* pD, const float* pA, const float* pX, int64_t Mk, int64_t Pk, int64_t stride_AD,
                   int64_t stride_X, int64_t N, int init, void* stream) {
-  return kernel_entry<float>(native_kernel_onto_f32, native_gemm_f32, pD, pA, pX, Mk, Pk, stride_AD, stride_X, N,
-                             init, stream);
+  auto jmul = [](DeviceInfo* d, int64_t m, int64_t p, int64_t n, const float* A, int64_t la, const float* X,
+                 int64_t lx, float* D, int64_t ld, cudaStream_t s) {
+    return native_gemm_f32(0, 0, m, p, n, 1.0f, A, la, X, lx, 0.0f, D, ld, d->sms, d->pool, s);
+  };
+  auto onto = [](DeviceInfo* d, int64_t m, int64_t p, int64_t n, const float* A, int64_t la, const float* X,
+                 int64_t lx, float* D, int64_t ld, cudaStream_t s) {
+    return native_kernel_onto_f32(m, p, n, A, la, X, lx, D, ld, d->sms, d->pool, s);
+  };
+  return kernel_entry<float>(onto, jmul, pD, pA, pX, Mk, Pk, stride_AD, stride_X, N, init, stream);
 }
 
 int gb_gemm_adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B,

@@ -1,5 +1,5 @@
-// Register-blocked GEMM mainloop on the CUDA cores, shared by the native FP64/FP32 GEMM
-// (GB_MODE_NATIVE) and the semiring GEMM.
+// Register-blocked GEMM mainloop on the CUDA cores, shared by the FP32 grouped GEMM and the
+// semiring GEMM.
 //
 // Restates jBLAS's register-blocked driver (src/gemm.jl:244-348) for the GPU: each
 // thread owns a TM x TN register tile of C (the reference's rows x cols tile from
