@@ -1345,11 +1345,9 @@ static int strided_batched(int dtype_bytes, int64_t M, int64_t N, int64_t K, dou
   char* ws = nullptr;
   GB_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), tab_bytes + ws_bytes, dev->pool, s));
   gb_problem_t* tab = reinterpret_cast<gb_problem_t*>(ws);
-  rc = grouped_fill_strided(tab, n, M, N, K, lda, ldb, ldc, A, B, C, sa * dtype_bytes, sb * dtype_bytes,
-                            sc * dtype_bytes, alpha, beta, s);
-  if (!rc)
-    rc = grouped_launch(dtype_bytes, tab, n, grouped_default_tuning(dtype_bytes),
-                        reinterpret_cast<long long*>(ws + tab_bytes), dev->sms, s);
+  rc = grouped_strided_launch(dtype_bytes, tab, reinterpret_cast<long long*>(ws + tab_bytes), n, M, N, K, lda, ldb,
+                              ldc, A, B, C, sa * dtype_bytes, sb * dtype_bytes, sc * dtype_bytes, alpha, beta,
+                              dev->sms, s);
   cudaFreeAsync(ws, s);
   return rc;
 }

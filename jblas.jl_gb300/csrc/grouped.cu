@@ -24,27 +24,26 @@
 #include "gb_common.cuh"
 #include "grouped.cuh"
 #include "profile.cuh"
-#include "simt_gemm.cuh"
+#include "simt4_tile.cuh"
 
 namespace gb {
 
 struct TileCfg {
-  int bm, bn, bk, tm, tn;
+  int bm, bn;
 };
-// FP32 runs every configuration on 256 threads, (bm / tm) * (bn / tn) == 256; 4-9, the larger and
-// rectangular tiles, are FP32 only.  FP64 takes bm and bn of 0-3 as the largest extents of its
-// tiles (f64_tile.cuh).
+// 0-3 serve both element types; 4-9, the larger and rectangular tiles, are FP32 only.  FP64 takes bm
+// and bn as the largest extents of its tiles (f64_tile.cuh); FP32 runs a tile in pieces of 64 x 64.
 __host__ __device__ constexpr TileCfg tile_cfg(int c) {
-  return c == 0 ? TileCfg{16, 16, 16, 1, 1}
-       : c == 1 ? TileCfg{32, 32, 16, 2, 2}
-       : c == 2 ? TileCfg{64, 32, 16, 4, 2}
-       : c == 3 ? TileCfg{64, 64, 16, 4, 4}
-       : c == 4 ? TileCfg{128, 64, 16, 8, 4}
-       : c == 5 ? TileCfg{128, 128, 16, 8, 8}
-       : c == 6 ? TileCfg{32, 64, 16, 2, 4}
-       : c == 7 ? TileCfg{64, 128, 16, 4, 8}
-       : c == 8 ? TileCfg{128, 32, 16, 8, 2}
-                : TileCfg{32, 128, 16, 2, 8};
+  return c == 0 ? TileCfg{16, 16}
+       : c == 1 ? TileCfg{32, 32}
+       : c == 2 ? TileCfg{64, 32}
+       : c == 3 ? TileCfg{64, 64}
+       : c == 4 ? TileCfg{128, 64}
+       : c == 5 ? TileCfg{128, 128}
+       : c == 6 ? TileCfg{32, 64}
+       : c == 7 ? TileCfg{64, 128}
+       : c == 8 ? TileCfg{128, 32}
+                : TileCfg{32, 128};
 }
 constexpr int GROUPED_CONFIGS_F64 = 4;
 constexpr int GROUPED_CONFIGS_F32 = 10;
@@ -54,28 +53,9 @@ __host__ __device__ inline int size_class(int64_t m, int64_t n) {
   return d <= 16 ? 0 : d <= 32 ? 1 : d <= 64 ? 2 : d <= 128 ? 3 : d <= 256 ? 4 : 5;
 }
 
-// Per-problem choice (GB_GROUPED_AUTO) in FP32: the configuration with the least modelled time
-//   tiles x (bm bn max(k, 1) / eff(tm tn) + overhead)
-// where eff is the measured FMA efficiency of a register tile of tm x tn elements per thread
-// relative to the 8 x 8 tile, and overhead the fixed cost of one tile (its first panel's load
-// latency, index set-up and epilogue) in the same units.  Padding rows and columns of a tile
-// cost as much as real ones, so tall and wide problems take rectangular tiles.
-__host__ __device__ inline int auto_config_f32(int64_t m, int64_t n, int64_t k) {
-  float best = 3.4e38f;
-  int arg = 0;
-  for (int c = 0; c < GROUPED_CONFIGS_F32; ++c) {
-    const TileCfg t = tile_cfg(c);
-    const int e = t.tm * t.tn;
-    const float eff = e >= 64 ? 1.0f : e >= 32 ? 0.9f : e >= 16 ? 0.75f : e >= 8 ? 0.55f : e >= 4 ? 0.35f : 0.1f;
-    const float tiles = static_cast<float>((m + t.bm - 1) / t.bm) * static_cast<float>((n + t.bn - 1) / t.bn);
-    const float cost = tiles * (static_cast<float>(t.bm * t.bn) * static_cast<float>(k > 1 ? k : 1) / eff + 32768.0f);
-    if (cost < best) {
-      best = cost;
-      arg = c;
-    }
-  }
-  return arg;
-}
+// Per-problem choice (GB_GROUPED_AUTO) in FP32: 64 x 64 pieces, or 32 x 32 ones where all problems
+// together have too few of the larger for every CTA of the grid to take several.
+__host__ __device__ inline int auto_config_f32(bool large) { return large ? 3 : 1; }
 
 // Extents of an FP64 problem's tiles under a configuration: equal tiles as large as the
 // configuration allows (33 rows on 32-row tiles: 17 + 16, not 32 + 1).
@@ -121,81 +101,15 @@ __device__ __forceinline__ int config_of(const gb_grouped_tuning_t& t, int cls) 
 }
 
 
-constexpr int GROUPED_THREADS = 256;   // FP32 (FP64: F64_THREADS)
-// largest shared memory of any FP32 tile routine (bytes): the double-buffered 128 x 128 x 16
-// panels of the SIMT mainloop
-constexpr int GROUPED_SMEM = SimtSmem<float, 128, 128, 16>::ELEMS * 4;
-
-// jmul!'s FMA chain with the alpha/beta epilogue of the grouped call (alpha != 0 here).
-template <typename T>
-struct GroupedChainOp {
-  static constexpr bool kInitFromC = false;
-  static constexpr bool kPairs = false;
-  static constexpr bool kVecStore = true;   // short K loops: the epilogue's stores matter
-  T alpha, beta;
-  static __device__ __forceinline__ T init() { return T(-0.0); }
-  static __device__ __forceinline__ T step(T acc, T a, T b) { return fma_t<T>(a, b, acc); }
-  __device__ __forceinline__ void store(T* c, T acc) const {
-    *c = (beta == T(0)) ? alpha * acc : fma_t<T>(alpha, acc, beta * *c);
-  }
-  __device__ __forceinline__ T value(T c, T acc) const {
-    return (beta == T(0)) ? alpha * acc : fma_t<T>(alpha, acc, beta * c);
-  }
-  __device__ __forceinline__ bool reads_c() const { return beta != T(0); }
-};
-
-// One 16 x 16 FP32 tile of problem `p` (column-major, no transposes), one element a thread.  The FMA
-// chain runs k = 0..K-1 in order from -0.0 (equal to jmul!'s a1*x1 first step, bit for bit).  The
-// next 16 k are loaded into registers while the current ones are multiplied from shared memory; B's
-// slab is stored [k][n] with rows padded by one word, so the k-fastest global reads land in
-// distinct banks.
-__device__ __forceinline__ void grouped_tile_16(const gb_problem_t& p, int tm, int tn, float* smem) {
-  constexpr int D = 16;
-  float* As = smem;           // [k][m]
-  float* Bs = As + D * D;     // [k][n], rows of D + 1
-  const int tid = threadIdx.x;
-  const int tx = tid % D, ty = tid / D;
-  const int64_t M = p.m, N = p.n, K = p.k;
-  const int64_t m0 = static_cast<int64_t>(tm) * D, n0 = static_cast<int64_t>(tn) * D;
-  const float* __restrict__ A = static_cast<const float*>(p.A);
-  const float* __restrict__ B = static_cast<const float*>(p.B);
-  // alpha and beta converted once per warp (on the narrow FP64 pipe) and broadcast
-  float2 ab = make_float2(0.0f, 0.0f);
-  if ((tid & 31) == 0) ab = make_float2(static_cast<float>(p.alpha), static_cast<float>(p.beta));
-  const float alpha = __shfl_sync(0xffffffffu, ab.x, 0), beta = __shfl_sync(0xffffffffu, ab.y, 0);
-  const bool alpha_zero = (__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0;
-  const bool unit = __double_as_longlong(p.alpha) == 0x3FF0000000000000ll && __double_as_longlong(p.beta) == 0ll;
-  const int64_t Kc = alpha_zero ? 0 : K;   // alpha == 0: A and B are not read
-  float acc = -0.0f, ra = 0.0f, rb = 0.0f;
-  auto load = [&](int64_t k0) {   // A: tx along m, ty along k; B: tx along k, ty along n
-    ra = (m0 + tx < M && k0 + ty < K) ? A[(m0 + tx) + (k0 + ty) * p.lda] : 0.0f;
-    rb = (n0 + ty < N && k0 + tx < K) ? B[(k0 + tx) + (n0 + ty) * p.ldb] : 0.0f;
-  };
-  if (Kc > 0) load(0);
-  for (int64_t k0 = 0; k0 < Kc; k0 += D) {
-    const int kc = static_cast<int>(K - k0 < D ? K - k0 : D);
-    As[ty * D + tx] = ra;
-    Bs[tx * (D + 1) + ty] = rb;
-    __syncthreads();
-    if (k0 + D < Kc) load(k0 + D);   // in flight while this slab is multiplied
-    for (int kk = 0; kk < kc; ++kk) acc = fmaf(As[kk * D + ty], Bs[kk * (D + 1) + tx], acc);
-    __syncthreads();
-  }
-  const int64_t m = m0 + ty, n = n0 + tx;
-  if (m >= M || n >= N) return;
-  float* c = static_cast<float*>(p.C) + m + n * p.ldc;
-  if (alpha == 0.0f) *c = (beta == 0.0f) ? 0.0f : beta * *c;
-  else if (unit) *c = acc;
-  else *c = (beta == 0.0f) ? alpha * acc : fmaf(alpha, acc, beta * *c);
-}
-
 // alpha = 0: C = beta C on one bm x bn tile (beta = 0 writes zeros without reading C; A and B
 // are not read), as jBLAS's alpha/beta extension of gb_gemm_* defines it.
+// Run by `threads` threads numbered `tid`.
 template <typename T>
-__device__ __forceinline__ void scale_tile(const gb_problem_t& p, int64_t m0, int64_t n0, int bm, int bn) {
+__device__ __forceinline__ void scale_tile(const gb_problem_t& p, int64_t m0, int64_t n0, int bm, int bn, int tid,
+                                           int threads) {
   T* __restrict__ C = static_cast<T*>(p.C);
   const T beta = static_cast<T>(p.beta);
-  for (int e = threadIdx.x; e < bm * bn; e += static_cast<int>(blockDim.x)) {
+  for (int e = tid; e < bm * bn; e += threads) {
     const int64_t m = m0 + e % bm, n = n0 + e / bm;
     if (m < p.m && n < p.n) {
       T* c = &C[m + n * p.ldc];
@@ -204,11 +118,12 @@ __device__ __forceinline__ void scale_tile(const gb_problem_t& p, int64_t m0, in
   }
 }
 
-// The configuration one problem runs under (the table's, or the per-problem choice).
-__device__ __forceinline__ int prologue_config(const gb_grouped_tuning_t& tuning, const gb_problem_t& p, bool f32) {
+// The configuration one problem runs under: the table's, or the per-problem choice (`large`: auto_config_f32).
+__device__ __forceinline__ int prologue_config(const gb_grouped_tuning_t& tuning, const gb_problem_t& p, bool f32,
+                                               bool large) {
   const int c = config_of(tuning, size_class(p.m, p.n));
   if (c != GB_GROUPED_AUTO) return c;
-  return f32 ? auto_config_f32(p.m, p.n, p.k) : auto_config_f64(p.m, p.n, p.k);
+  return f32 ? auto_config_f32(large) : auto_config_f64(p.m, p.n, p.k);
 }
 
 // Workspace of a call over `count` problems (int64 words): the tile prefix sums in schedule
@@ -223,33 +138,48 @@ __host__ __device__ inline int grouped_order_entry(int i, int cfg, int count) {
 }
 
 // Prologue (one block): the schedule orders the problems by the work of one of their tiles
-// (tile rows x tile columns x k, in 32 power-of-two buckets, heaviest first), so that the CTAs
-// take tiles of similar length side by side and the short ones fill the tail; it writes the order and the exclusive prefix sums of the tiles in that order.
+// (rows x columns x k of what a tile holds, in 32 power-of-two buckets, heaviest first), so that the
+// CTAs take tiles of similar length side by side and the short ones fill the tail; it writes the order and the exclusive prefix sums of the tiles in that order.
 // The order inside a bucket depends on timing, which changes no result (each tile is
 // independent).
 __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_problem_t* __restrict__ probs, int count,
                                                               gb_grouped_tuning_t tuning, bool f32,
-                                                              long long* __restrict__ ws) {
+                                                              int enough, long long* __restrict__ ws) {
   __shared__ long long part[1024];
   __shared__ int hist[32], start[32];
   long long* offsets = ws;
   int* order = reinterpret_cast<int*>(grouped_order_words(ws, count));
   const int t = threadIdx.x;
   if (t < 32) hist[t] = 0;
-  __syncthreads();
-  auto bucket_of = [&](const gb_problem_t& p, const TileCfg& c) {
-    long long w = static_cast<long long>(c.bm) * c.bn * (p.k > 1 ? p.k : 1);
-    if (!f32) {   // FP64 tiles cost what is in them
-      const F64Tiles t = f64_tiles(c, p.m, p.n);
-      w = static_cast<long long>(t.fm) * t.fn * (p.k > 1 ? p.k : 1);
-      if (w < 1) w = 1;
+  bool large = true;   // (a table too long to pack keeps the larger tiles)
+  if (f32 && count <= GROUPED_PACK_LIMIT) {
+    int pieces = 0;   // 64 x 64 pieces of all problems, up to the threshold
+    for (int i = t; i < count && pieces < enough; i += 1024) {
+      const gb_problem_t& p = probs[i];
+      if (p.m > 0 && p.n > 0) pieces += static_cast<int>(min(static_cast<int64_t>(enough), ((p.m + 63) / 64) * ((p.n + 63) / 64)));
     }
-    const int lg = 63 - __clzll(w);                 // w >= 1
+    part[t] = pieces;
+    __syncthreads();
+    for (int off = 512; off > 0; off >>= 1) {
+      if (t < off) part[t] += part[t + off];
+      __syncthreads();
+    }
+    large = part[0] >= enough;
+  }
+  __syncthreads();
+  auto bucket_of = [&](const gb_problem_t& p, int cfg) {
+    const long long k = p.k > 1 ? p.k : 1;
+    const TileCfg c = tile_cfg(cfg);
+    const F64Tiles t = f64_tiles(c, p.m, p.n);
+    const long long held = f32 ? min(p.m, static_cast<int64_t>(c.bm)) * min(p.n, static_cast<int64_t>(c.bn))
+                               : static_cast<long long>(t.fm) * t.fn;
+    const long long w = held * k;
+    const int lg = 63 - __clzll(w > 1 ? w : 1);
     return 31 - (lg > 31 ? 31 : lg);                 // heavy first
   };
   for (int i = t; i < count; i += 1024) {
     const gb_problem_t& p = probs[i];
-    atomicAdd(&hist[bucket_of(p, tile_cfg(prologue_config(tuning, p, f32)))], 1);
+    atomicAdd(&hist[bucket_of(p, prologue_config(tuning, p, f32, large))], 1);
   }
   __syncthreads();
   if (t == 0) {
@@ -262,8 +192,8 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   __syncthreads();
   for (int i = t; i < count; i += 1024) {
     const gb_problem_t& p = probs[i];
-    const int cfg = prologue_config(tuning, p, f32);
-    order[atomicAdd(&start[bucket_of(p, tile_cfg(cfg))], 1)] = grouped_order_entry(i, cfg, count);
+    const int cfg = prologue_config(tuning, p, f32, large);
+    order[atomicAdd(&start[bucket_of(p, cfg)], 1)] = grouped_order_entry(i, cfg, count);
   }
   __syncthreads();
   const int per = (count + 1023) / 1024;
@@ -272,7 +202,7 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   auto tiles_of = [&](int pos) -> long long {
     const int e = order[pos];
     const gb_problem_t& p = probs[packed ? (e & 0xFFFFFF) : e];
-    const TileCfg c = tile_cfg(packed ? (e >> 24) : prologue_config(tuning, p, f32));
+    const TileCfg c = tile_cfg(packed ? (e >> 24) : prologue_config(tuning, p, f32, large));
     return (p.m <= 0 || p.n <= 0) ? 0 : ((p.m + c.bm - 1) / c.bm) * ((p.n + c.bn - 1) / c.bn);
   };
   long long sum = 0;
@@ -319,94 +249,116 @@ __device__ __forceinline__ int schedule_pos(const long long* __restrict__ offset
   return lo;
 }
 
-template <typename T>
-constexpr int grouped_threads() { return sizeof(T) == 8 ? F64_THREADS : GROUPED_THREADS; }
+// A tile of the schedule: its problem and its place in it.  `lo` is the caller's schedule position.
+struct GroupedTile {
+  gb_problem_t p;
+  TileCfg c;
+  int64_t tm, tn;   // tile row and column
+};
+__device__ __forceinline__ void grouped_find(const gb_problem_t* __restrict__ probs, int count,
+                                             const gb_grouped_tuning_t& tuning, bool f32,
+                                             const long long* __restrict__ offsets, const int* __restrict__ order,
+                                             long long w, int& lo, GroupedTile& t) {
+  lo = schedule_pos(offsets, count, w, lo);
+  const int e = order[lo];
+  const bool packed = count <= GROUPED_PACK_LIMIT;
+  t.p = probs[packed ? (e & 0xFFFFFF) : e];
+  t.c = tile_cfg(packed ? (e >> 24) : prologue_config(tuning, t.p, f32, true));
+  // in 32-bit arithmetic (a problem's tile count is below 2^31); the first problem's tiles start at 0
+  const int local = static_cast<int>(lo ? w - offsets[lo] : w);
+  const int tiles_m = static_cast<int>((t.p.m + t.c.bm - 1) / t.c.bm);
+  const int tn = local / tiles_m;
+  t.tm = local - tn * tiles_m;
+  t.tn = tn;
+}
+__device__ __forceinline__ bool alpha_is_zero(const gb_problem_t& p) {
+  return (__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0;
+}
 
-// Persistent tile loop: CTA b takes tile b of the schedule, then the next one that no CTA has taken
-// (a counter in offsets[0]; its answer is fetched while the tile runs).  Against a fixed stride, where
-// the busiest SM of 4096 log-uniform problems gets 3.5% more than its share.
-template <typename T>
-__global__ void __launch_bounds__(grouped_threads<T>(), sizeof(T) == 8 ? F64_CTAS : 2)
-    grouped_gemm_kernel(const gb_problem_t* __restrict__ probs, int count, gb_grouped_tuning_t tuning,
-                        long long* __restrict__ ws) {
-  __shared__ __align__(16) unsigned char smem[sizeof(T) == 8 ? F64_SMEM_ELEMS * 8 : GROUPED_SMEM];
-  __shared__ long long next_tile[2];
+// Persistent tile loop: CTA b takes tile b of the schedule, then the next one that no CTA has taken (a
+// counter in offsets[0]; its answer is fetched while the tile runs).  Against a fixed stride, where
+// the busiest SM of 4096 log-uniform problems gets 3.5% more than its share.  run(tile, index) may leave
+// its shared memory without a barrier: one follows.
+template <class Run>
+__device__ __forceinline__ void grouped_loop(const gb_problem_t* __restrict__ probs, int count,
+                                             const gb_grouped_tuning_t& tuning, bool f32, long long* __restrict__ ws,
+                                             const Run& run) {
+  __shared__ long long next_tile[2];   // two slots: one is written again only after another barrier
   const long long* offsets = ws;
   const int* order = reinterpret_cast<const int*>(grouped_order_words(ws, count));
   const long long total = offsets[count];
-  int lo = 0;   // the first problem's tiles start at 0 <= w
-  long long next = 0;
-  long long w = blockIdx.x;
-  // The tile after this one, handed to all threads; the barrier also frees the shared panels.  Two
-  // slots: a slot is written again only after another such barrier.
-  auto advance = [&](int slot) {
+  int lo = 0, slot = 0;
+  for (long long w = blockIdx.x; w < total; slot ^= 1) {
+    long long next = 0;
+    if (threadIdx.x == 0)
+      next = gridDim.x + static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(ws), 1ull));
+    GroupedTile t;
+    grouped_find(probs, count, tuning, f32, offsets, order, w, lo, t);
+    run(t, w);
     if (threadIdx.x == 0) next_tile[slot] = next;
     __syncthreads();
     w = next_tile[slot];
-  };
-  for (int slot = 0; w < total; advance(slot), slot ^= 1) {
-    if (threadIdx.x == 0)
-      next = gridDim.x + static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(ws), 1ull));
-    lo = schedule_pos(offsets, count, w, lo);
-    const int e = order[lo];
-    const bool packed = count <= GROUPED_PACK_LIMIT;
-    const gb_problem_t p = probs[packed ? (e & 0xFFFFFF) : e];
-    const int cfg = packed ? (e >> 24) : prologue_config(tuning, p, sizeof(T) == 4);
-    const TileCfg c = tile_cfg(cfg);
-    // tile rows of the problem and the tile's place in it, in 32-bit arithmetic (a problem's
-    // tile count is below 2^31)
-    const int local = static_cast<int>(lo ? w - offsets[lo] : w);
-    const int tiles_m = static_cast<int>((p.m + c.bm - 1) / c.bm);
-    const int tn = local / tiles_m, tm = local - tn * tiles_m;
-    if constexpr (sizeof(T) == 8) {
-      const F64Tiles ft = f64_tiles(c, p.m, p.n);
-      const int64_t m0 = static_cast<int64_t>(tm) * ft.fm, n0 = static_cast<int64_t>(tn) * ft.fn;
-      const int r = static_cast<int>(p.m - m0 < ft.fm ? p.m - m0 : ft.fm);
-      const int cc = static_cast<int>(p.n - n0 < ft.fn ? p.n - n0 : ft.fn);
-      if (r <= 0 || cc <= 0) continue;   // equal tiles can need one fewer
-      if ((__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0) {
-        scale_tile<T>(p, m0, n0, r, cc);
-        continue;
-      }
-      const bool unit = __double_as_longlong(p.alpha) == 0x3FF0000000000000ll && __double_as_longlong(p.beta) == 0ll;
-      const int cols = min(32, F64_MAX_ELEMS / r);   // larger tiles run in column strips
-      for (int j0 = 0; j0 < cc; j0 += cols) {
-        if (j0) __syncthreads();   // the strip reuses the shared panels
-        f64_tile_any<false>(r, min(cols, cc - j0), p.k, static_cast<const double*>(p.A) + m0, 1, p.lda,
-                            static_cast<const double*>(p.B) + (n0 + j0) * p.ldb, 1, p.ldb, p.alpha, p.beta, unit,
-                            static_cast<double*>(p.C) + m0 + (n0 + j0) * p.ldc, p.ldc, static_cast<int>(w ^ (w >> 2)),
-                            reinterpret_cast<double*>(smem));
-      }
-    } else if (cfg == 0) {
-      grouped_tile_16(p, tm, tn, reinterpret_cast<float*>(smem));
-    } else if ((__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0) {
-      scale_tile<T>(p, static_cast<int64_t>(tm) * c.bm, static_cast<int64_t>(tn) * c.bn, c.bm, c.bn);
-    } else {
-      // FP32 register tiles of two or more rows and columns: the double-buffered SIMT mainloop
-      // of the native GEMM (simt_gemm.cuh) on this problem's tile
-      const GroupedChainOp<T> op{static_cast<T>(p.alpha), static_cast<T>(p.beta)};
-      const T* A = static_cast<const T*>(p.A);
-      const T* B = static_cast<const T*>(p.B);
-      T* C = static_cast<T*>(p.C);
-      T* sm = reinterpret_cast<T*>(smem);
-      const int64_t m0 = static_cast<int64_t>(tm) * c.bm, n0 = static_cast<int64_t>(tn) * c.bn;
-#define GB_GTILE(BM_, BN_, BK_, TM_, TN_)                                                                    \
-  simt_tile<T, GroupedChainOp<T>, BM_, BN_, BK_, TM_, TN_, false, false>(p.m, p.n, p.k, op, A, p.lda, B, p.ldb, C, \
-                                                                        p.ldc, m0, n0, sm)
-      switch (cfg) {
-        case 1: GB_GTILE(32, 32, 16, 2, 2); break;
-        case 2: GB_GTILE(64, 32, 16, 4, 2); break;
-        case 3: GB_GTILE(64, 64, 16, 4, 4); break;
-        case 4: GB_GTILE(128, 64, 16, 8, 4); break;
-        case 5: GB_GTILE(128, 128, 16, 8, 8); break;
-        case 6: GB_GTILE(32, 64, 16, 2, 4); break;
-        case 7: GB_GTILE(64, 128, 16, 4, 8); break;
-        case 8: GB_GTILE(128, 32, 16, 8, 2); break;
-        default: GB_GTILE(32, 128, 16, 2, 8); break;
-      }
-#undef GB_GTILE
-    }
   }
+}
+
+__global__ void __launch_bounds__(F64_THREADS, F64_CTAS)
+    grouped_f64_kernel(const gb_problem_t* __restrict__ probs, int count, gb_grouped_tuning_t tuning,
+                       long long* __restrict__ ws) {
+  __shared__ __align__(16) double smem[F64_SMEM_ELEMS];
+  grouped_loop(probs, count, tuning, false, ws, [&](const GroupedTile& t, long long w) {
+    const gb_problem_t& p = t.p;
+    const F64Tiles ft = f64_tiles(t.c, p.m, p.n);
+    const int64_t m0 = t.tm * ft.fm, n0 = t.tn * ft.fn;
+    const int r = static_cast<int>(p.m - m0 < ft.fm ? p.m - m0 : ft.fm);
+    const int c = static_cast<int>(p.n - n0 < ft.fn ? p.n - n0 : ft.fn);
+    if (r <= 0 || c <= 0) return;   // equal tiles can need one fewer
+    if (alpha_is_zero(p)) {
+      scale_tile<double>(p, m0, n0, r, c, threadIdx.x, F64_THREADS);
+      return;
+    }
+    const bool unit = __double_as_longlong(p.alpha) == 0x3FF0000000000000ll && __double_as_longlong(p.beta) == 0ll;
+    const int cols = min(32, F64_MAX_ELEMS / r);   // larger tiles run in column strips
+    for (int j0 = 0; j0 < c; j0 += cols) {
+      if (j0) __syncthreads();   // the strip reuses the shared panels
+      f64_tile_any<false>(r, min(cols, c - j0), p.k, static_cast<const double*>(p.A) + m0, 1, p.lda,
+                          static_cast<const double*>(p.B) + (n0 + j0) * p.ldb, 1, p.ldb, p.alpha, p.beta, unit,
+                          static_cast<double*>(p.C) + m0 + (n0 + j0) * p.ldc, p.ldc, static_cast<int>(w ^ (w >> 2)),
+                          smem);
+    }
+  });
+}
+
+// FP32: CTAs of four warps run a tile in pieces of up to 64 x 64 on the packed pairs of
+// simt4_tile.cuh: a warp takes a 32 x 32 part, so a piece pads to multiples of 32, and the operands are
+// read once per 64 rows or columns.  Independent warps on tiles of their own, as native FP32 runs
+// them, were slower here (start: 0.88 ms, now 0.66): warps on tiles of different extents execute different code, and with 64 x 64
+// tiles three quarters of their time was waiting for instructions (4096 log-uniform problems 1.1 to
+// 1.8 ms; 32 x 32 tiles 0.85 ms, bound by their 4-byte copies).
+using GroupedPiece = S4Shape<8, 4, 2, 2>;
+constexpr int GROUPED_F32_CTAS = 4;
+__global__ void __launch_bounds__(GroupedPiece::THREADS, GROUPED_F32_CTAS)
+    grouped_f32_kernel(const gb_problem_t* __restrict__ probs, int count, gb_grouped_tuning_t tuning,
+                       long long* __restrict__ ws) {
+  __shared__ __align__(16) uint32_t smem[GroupedPiece::SMEM_BYTES / 4];
+  grouped_loop(probs, count, tuning, true, ws, [&](const GroupedTile& t, long long) {
+    const gb_problem_t& p = t.p;
+    const int64_t m0 = t.tm * t.c.bm, n0 = t.tn * t.c.bn;
+    const int rows = static_cast<int>(p.m - m0 < t.c.bm ? p.m - m0 : t.c.bm);
+    const int cols = static_cast<int>(p.n - n0 < t.c.bn ? p.n - n0 : t.c.bn);
+    if (alpha_is_zero(p)) {
+      scale_tile<float>(p, m0, n0, rows, cols, threadIdx.x, GroupedPiece::THREADS);
+      return;
+    }
+    const F32Chain op{static_cast<float>(p.alpha), static_cast<float>(p.beta)};
+    for (int j0 = 0; j0 < cols; j0 += 64) {
+      for (int i0 = 0; i0 < rows; i0 += 64) {
+        const int r = min(64, rows - i0), c = min(64, cols - j0);
+        simt4_tile<GroupedPiece, true>(r, c, r, c, p.k, op, static_cast<const uint32_t*>(p.A) + m0 + i0, 1, p.lda,
+                                       static_cast<const uint32_t*>(p.B) + (n0 + j0) * p.ldb, 1, p.ldb,
+                                       static_cast<uint32_t*>(p.C) + m0 + i0 + (n0 + j0) * p.ldc, 1, p.ldc, smem);
+      }
+    }
+  });
 }
 
 gb_grouped_tuning_t grouped_default_tuning(int dtype_bytes) {
@@ -429,49 +381,35 @@ int grouped_validate_tuning(int dtype_bytes, const gb_grouped_tuning_t& t) {
   return GB_OK;
 }
 
-// Resident CTAs per SM of grouped_gemm_kernel<T>, looked up once per device (the occupancy
-// query runs against the current device's context); concurrent first calls may both query,
-// and both store the same value.
-constexpr int GROUPED_MAX_DEVICES = 64;
+// 64 x 64 pieces from which FP32's per-problem choice takes them (auto_config_f32): three a CTA.
+static int f32_enough(int sms) { return 3 * GROUPED_F32_CTAS * sms; }
 
-template <typename T>
-static int grid_for(int sms) {
-  static std::atomic<int> per_sm_of[GROUPED_MAX_DEVICES];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= GROUPED_MAX_DEVICES) {
-    cudaGetLastError();
-    dev = -1;
-  }
-  int per_sm = dev >= 0 ? per_sm_of[dev].load(std::memory_order_relaxed) : 0;
-  if (per_sm < 1) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_gemm_kernel<T>, grouped_threads<T>(), 0) !=
-            cudaSuccess ||
-        per_sm < 1) {
-      cudaGetLastError();
-      per_sm = 1;
-    } else if (dev >= 0) {
-      per_sm_of[dev].store(per_sm, std::memory_order_relaxed);
-    }
-  }
-  return sms * per_sm;
+static int launch_f64_tiles(const gb_problem_t* d_probs, int count, const gb_grouped_tuning_t& tuning, long long* ws,
+                            int sms, cudaStream_t s) {
+  grouped_f64_kernel<<<sms * F64_CTAS, F64_THREADS, 0, s>>>(d_probs, count, tuning, ws);
+  return GB_OK;
+}
+
+static int launch_tiles(int dtype_bytes, const gb_problem_t* d_probs, int count, const gb_grouped_tuning_t& tuning,
+                        long long* d_ws, int sms, cudaStream_t s) {
+  if (dtype_bytes == 8)
+    GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s, launch_f64_tiles(d_probs, count, tuning, d_ws, sms, s));
+  else
+    GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
+              (grouped_f32_kernel<<<sms * GROUPED_F32_CTAS, GroupedPiece::THREADS, 0, s>>>(d_probs, count, tuning,
+                                                                                           d_ws)));
+  GB_CUDA_TRY(cudaGetLastError());
+  return GB_OK;
 }
 
 int grouped_launch(int dtype_bytes, const gb_problem_t* d_probs, int count, const gb_grouped_tuning_t& tuning,
                    long long* d_offsets, int sms, cudaStream_t s) {
   if (count <= 0) return GB_OK;
   GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
-            (grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, tuning, dtype_bytes == 4, d_offsets)));
-  if (dtype_bytes == 8) {
-    const int grid = grid_for<double>(sms);
-    GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
-              (grouped_gemm_kernel<double><<<grid, F64_THREADS, 0, s>>>(d_probs, count, tuning, d_offsets)));
-  } else {
-    const int grid = grid_for<float>(sms);
-    GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
-              (grouped_gemm_kernel<float><<<grid, GROUPED_THREADS, 0, s>>>(d_probs, count, tuning, d_offsets)));
-  }
+            (grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, tuning, dtype_bytes == 4, f32_enough(sms),
+                                                      d_offsets)));
   GB_CUDA_TRY(cudaGetLastError());
-  return GB_OK;
+  return launch_tiles(dtype_bytes, d_probs, count, tuning, d_offsets, sms, s);
 }
 
 size_t grouped_workspace_bytes(int count) {
@@ -610,11 +548,11 @@ int grouped_f64_noalloc(const gb_problem_t* d_probs, int count, const gb_grouped
   // clearing.
   // Launched directly, not through the timing hooks (which create CUDA events while profiling
   // is on); gb_launch_counts still counts both launches.
-  grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, t, false, offsets);
+  grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, t, false, 0, offsets);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return gb_set_cuda_error(e, "grouped prologue launch");
   prof_count(GB_KERNEL_GROUPED_GEMM);
-  grouped_gemm_kernel<double><<<grid_for<double>(sms), F64_THREADS, 0, s>>>(d_probs, count, t, offsets);
+  launch_f64_tiles(d_probs, count, t, offsets, sms, s);
   e = cudaGetLastError();
   if (e != cudaSuccess) return gb_set_cuda_error(e, "grouped launch");
   prof_count(GB_KERNEL_GROUPED_GEMM);
@@ -623,10 +561,12 @@ int grouped_f64_noalloc(const gb_problem_t* d_probs, int count, const gb_grouped
 
 
 // ------------------------------------------------------------------ strided batches
+// The table of a strided batch and, as all its problems have one configuration of `tiles` tiles, its
+// schedule: the offsets and the order that the prologue would write (`cfg` < 0: the prologue runs).
 __global__ void grouped_fill_strided_kernel(gb_problem_t* __restrict__ probs, int count, int64_t M, int64_t N,
                                             int64_t K, int64_t lda, int64_t ldb, int64_t ldc, const char* A,
                                             const char* B, char* C, int64_t sa, int64_t sb, int64_t sc, double alpha,
-                                            double beta) {
+                                            double beta, int cfg, long long tiles, long long* __restrict__ ws) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   gb_problem_t p;
@@ -642,18 +582,36 @@ __global__ void grouped_fill_strided_kernel(gb_problem_t* __restrict__ probs, in
   p.alpha = alpha;
   p.beta = beta;
   probs[i] = p;
+  if (cfg >= 0) {
+    ws[i] = i * tiles;
+    if (i == count - 1) ws[count] = count * tiles;
+    reinterpret_cast<int*>(grouped_order_words(ws, count))[i] = grouped_order_entry(i, cfg, count);
+  }
 }
 
-int grouped_fill_strided(gb_problem_t* d_probs, int count, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
-                         int64_t ldc, const void* A, const void* B, void* C, int64_t strideA_bytes,
-                         int64_t strideB_bytes, int64_t strideC_bytes, double alpha, double beta, cudaStream_t s) {
+// `count` products of one shape under the default tuning: one launch fills the table and the schedule
+// (the one-block prologue took 8 us of a call on 668 products of 10 x 35 x 19), one runs it.
+int grouped_strided_launch(int dtype_bytes, gb_problem_t* d_probs, long long* d_ws, int count, int64_t M, int64_t N,
+                           int64_t K, int64_t lda, int64_t ldb, int64_t ldc, const void* A, const void* B, void* C,
+                           int64_t strideA_bytes, int64_t strideB_bytes, int64_t strideC_bytes, double alpha,
+                           double beta, int sms, cudaStream_t s) {
   if (count <= 0) return GB_OK;
+  int cfg = -1;
+  long long tiles = 0;
+  if (count <= GROUPED_PACK_LIMIT) {
+    const int64_t pieces = ((M + 63) / 64) * ((N + 63) / 64);
+    cfg = dtype_bytes == 8 ? auto_config_f64(M, N, K) : auto_config_f32(pieces >= f32_enough(sms) / count + 1);
+    const TileCfg c = tile_cfg(cfg);
+    tiles = ((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
+  }
   const int blocks = (count + 255) / 256;
   grouped_fill_strided_kernel<<<blocks, 256, 0, s>>>(d_probs, count, M, N, K, lda, ldb, ldc,
                                                       static_cast<const char*>(A), static_cast<const char*>(B),
                                                       static_cast<char*>(C), strideA_bytes, strideB_bytes,
-                                                      strideC_bytes, alpha, beta);
+                                                      strideC_bytes, alpha, beta, cfg, tiles, d_ws);
   GB_CUDA_TRY(cudaGetLastError());
-  return GB_OK;
+  const gb_grouped_tuning_t tuning = grouped_default_tuning(dtype_bytes);
+  return cfg < 0 ? grouped_launch(dtype_bytes, d_probs, count, tuning, d_ws, sms, s)
+                 : launch_tiles(dtype_bytes, d_probs, count, tuning, d_ws, sms, s);
 }
 }  // namespace gb

@@ -5,9 +5,9 @@
 // a1*x1 bit for bit; every tile shape, operand layout and packing runs the same chain.
 //
 // Measured in alternation with 128 x 128 / 64 x 64 scalar register tiles (FFMA peak 78 TFLOP/s):
-// 256^3 16.6 -> 13.3 us a call, 1536^3 217 -> 163 us, 2048^3 404 -> 350 us, 4096^3 2.73 -> 2.41 ms
-// (alpha = 1.5, beta = 0.5), 4097 x 4095 x 4001 2.67 -> 2.40, 8192 x 8192 x 4096 10.4 -> 9.05
-// (61 TFLOP/s), 16384 x 64 x 16384 1.11 -> 0.86; kernel! at 2048^3 519 -> 369 us.
+// 256^3 16.6 -> 13 us a call, 1536^3 217 -> 172 us, 2048^3 404 -> 336 us, 4096^3 2.70 -> 2.31 ms,
+// 4097 x 4095 x 4001 2.67 -> 2.30, 8192 x 8192 x 4096 10.4 -> 8.66 (63 TFLOP/s), 16384 x 64 x 16384
+// 1.11 -> 0.91; kernel! at 2048^3 519 -> 369 us.
 #include <algorithm>
 
 #include "gb_common.cuh"
@@ -16,19 +16,6 @@
 #include "simt4_tile.cuh"
 
 namespace gb {
-
-// jmul!'s chain with the BLAS alpha/beta epilogue (beta == 0: C is not read).
-struct F32Chain {
-  static constexpr bool kInitFromC = false;
-  float alpha, beta;
-  static __device__ __forceinline__ uint32_t init() { return 0x80000000u; }   // -0.0
-  static __device__ __forceinline__ pair4 step(pair4 acc, pair4 a, pair4 b) { return fma_f32x2(a, b, acc); }
-  __device__ __forceinline__ bool reads_c() const { return beta != 0.0f; }
-  __device__ __forceinline__ uint32_t value(uint32_t acc) const { return __float_as_uint(alpha * __uint_as_float(acc)); }
-  __device__ __forceinline__ uint32_t value(uint32_t c, uint32_t acc) const {
-    return __float_as_uint(fmaf(alpha, __uint_as_float(acc), beta * __uint_as_float(c)));
-  }
-};
 
 // jBLAS's kernel! (src/kernels.jl:212-238): the chain starts from D's value and is stored as is.
 struct F32Onto {

@@ -1,5 +1,5 @@
-// Tile of C for 4-byte elements on the CUDA cores, for native FP32: register tiles on packed
-// pairs of rows.
+// Tile of C for 4-byte elements on the CUDA cores, for native and grouped FP32: register tiles
+// on packed pairs of rows.
 //
 // What bounds it: with one multiply-add per instruction the FMA pipe (one warp instruction per
 // clock and SM partition) shares its issue slots with shared-memory reads and address arithmetic;
@@ -11,13 +11,15 @@
 //  - a pair is two consecutive rows: A's rows lie side by side in shared memory and are read as
 //    pairs; B's element is duplicated in registers (two moves for 4 or 8 packed operations);
 //  - up to 16 x 8 elements a thread, so that a k takes 6 16-byte reads for 64 packed operations,
-//    and a tile is one warp's alone: nothing waits at a barrier (two
-//    warps a tile: 38 TFLOP/s on 16384 x 64 x 16384, one: 43);
+//    and natively a tile is one warp's alone: nothing waits at a barrier
+//    (two warps a tile: 38 TFLOP/s on 16384 x 64 x 16384, one: 40);
 //  - panels come through cp.async: 16 bytes a copy where rows are contiguous and aligned, else 4 (any
 //    alignment, either orientation), S4_STAGES - 1 panels ahead, without bounds checks inside the
 //    matrix;
-//  - the k loop is unrolled by 8 (16 overflowed the instruction cache: 128 x 128 tiles 49 -> 34
-//    TFLOP/s in the scalar form).
+//  - the code stays small, as every warp fetches it at a place of its own: the k loop is unrolled by
+//    8 (by 16, 128 x 128 tiles fell from 49 to 34 TFLOP/s in the scalar form), and the 64 x 64 tile
+//    loads its panels from one place (with the first panels' loads written out before the loop,
+//    8192 x 8192 x 4096 took 9.0 ms instead of 8.6; the smaller tiles are the faster for it).
 // C has a row and a column stride, so a caller may exchange the operands' roles (C^T = B^T A^T).
 // Measured (native FP32, in alternation with the 8 x 8 scalar tile): see native_f32.cu.
 #pragma once
@@ -52,41 +54,47 @@ __device__ __forceinline__ pair4 fma_f32x2(pair4 a, pair4 b, pair4 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
-// Tile of one warp: 4 x 8 lanes of TM x TN elements.
-template <int TM_, int TN_>
+// Tile of WM x WN warps, each 4 x 8 lanes of TM x TN elements.
+template <int TM_, int TN_, int WM_ = 1, int WN_ = 1>
 struct S4Shape {
-  static constexpr int TM = TM_, TN = TN_;
-  static constexpr int BM = 4 * TM, BN = 8 * TN;
+  static constexpr int TM = TM_, TN = TN_, WM = WM_, WN = WN_, THREADS = 32 * WM * WN;
+  static constexpr int BM = WM * 4 * TM, BN = WN * 8 * TN;
   static constexpr int LDA = BM + 4, LDB = BN + 4;   // words; rows 16-byte aligned, k on distinct banks
   static constexpr int PANEL = S4_BK * (LDA + LDB);
-  static constexpr int SMEM_BYTES = S4_STAGES * PANEL * 4;   // of one warp
+  static constexpr int SMEM_BYTES = S4_STAGES * PANEL * 4;
   static_assert(TM % 4 == 0 && TN % 2 == 0, "vector operand reads");
+  // A one-warp tile has other warps beside it, a larger one is its CTA's.
+  static __device__ __forceinline__ int tid() { return THREADS == 32 ? threadIdx.x & 31 : threadIdx.x; }
+  static __device__ __forceinline__ void sync() {
+    if constexpr (THREADS == 32) __syncwarp();
+    else __syncthreads();
+  }
 };
 
-// One lane's share of an operand's panels: element (x, k), x < extent <= X, is src[x * xs + k * ks]
+// One thread's share of an operand's panels: element (x, k), x < extent <= X, is src[x * xs + k * ks]
 // and goes to word k * LD + x of the panel.  Three ways: XV four x a copy (xs = 1, aligned, full
 // extent), XF the lanes along x, KF the lanes along k (8 k x 4 x a warp: distinct banks).  Without
 // ANY the operand has xs = 1 and KF is not compiled (the code of the three ways and their registers
 // cost the largest tile 5%).
-template <int X, int LD, bool ANY>
+template <int X, int LD, int THREADS, bool ANY>
 struct S4Loader {
+  static constexpr int UNROLL = X > 32 ? 8 : 16;
   static constexpr int XV = 0, XF = 1, KF = 2;
-  static constexpr int VX = X / 4, VN = X * S4_BK / 4 / 32, VK = 32 / VX;
-  static constexpr int FX = X < 32 ? X : 32, FNX = X / FX, FK = 32 / FX, FN = S4_BK / FK;
-  static constexpr int KX = 4, KN = X / KX;
-  static_assert(32 % VX == 0 && S4_BK % VK == 0 && X % FX == 0 && 32 % FX == 0 && S4_BK % FK == 0 && X % KX == 0,
-                "panel loads");
+  static constexpr int VX = X / 4, VN = X * S4_BK / 4 / THREADS, VK = THREADS / VX;
+  static constexpr int FX = X < THREADS ? X : THREADS, FNX = X / FX, FK = THREADS / FX, FN = S4_BK / FK;
+  static constexpr int KX = THREADS / 8, KN = X / KX;
+  static_assert(THREADS % VX == 0 && S4_BK % VK == 0 && X % FX == 0 && THREADS % FX == 0 && S4_BK % FK == 0 &&
+                X % KX == 0, "panel loads");
   const uint32_t* p;
   int64_t str, adv, xstep;
   uint32_t dst;
   int way, x, k;
 
-  __device__ __forceinline__ void init(const uint32_t* src, int64_t xs, int64_t ks, int extent) {
-    const int lane = threadIdx.x & 31;
+  __device__ __forceinline__ void init(const uint32_t* src, int64_t xs, int64_t ks, int extent, int tid) {
     way = (ANY && ks == 1 && xs != 1) ? KF
         : (xs == 1 && extent == X && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (ks & 3) == 0) ? XV : XF;
-    x = way == XV ? lane % VX * 4 : way == XF ? lane % FX : lane / 8;
-    k = way == XV ? lane / VX : way == XF ? lane / FX : lane % 8;
+    x = way == XV ? tid % VX * 4 : way == XF ? tid % FX : tid / 8;
+    k = way == XV ? tid / VX : way == XF ? tid / FX : tid % 8;
     p = src + x * xs + k * ks;
     str = way == XV ? VK * ks : way == XF ? FK * ks : KX * xs;
     xstep = ANY ? FX * xs : FX;
@@ -94,21 +102,22 @@ struct S4Loader {
     dst = static_cast<uint32_t>(k * LD + x) * 4u;
   }
 
+  // (loops unrolled in part: their code is fetched by warps at many different places)
   template <bool CHECK>
   __device__ __forceinline__ void copy(uint32_t d, int extent, int kc) {
     const uint32_t* q = p;
     if (way == XV) {
-#pragma unroll
+#pragma unroll UNROLL
       for (int l = 0; l < VN; ++l, q += str)
         if (!CHECK || k + l * VK < kc) cp_async_16(d + l * (VK * LD * 4), q);
     } else if (!ANY || way == XF) {
-#pragma unroll
+#pragma unroll UNROLL
       for (int l = 0; l < FN; ++l, q += str)
 #pragma unroll
         for (int h = 0; h < FNX; ++h)
           if (!CHECK || (x + h * FX < extent && k + l * FK < kc)) cp_async_4(d + (l * FK * LD + h * FX) * 4, q + h * xstep);
     } else {
-#pragma unroll
+#pragma unroll UNROLL
       for (int l = 0; l < KN; ++l, q += str)
 #pragma unroll
         for (int h = 0; h < S4_BK; h += 8)
@@ -131,7 +140,8 @@ struct S4Loader {
 //   op.reads_c(), op.value(c, acc), op.value(acc)   the element of C, from its old value or without
 // k runs 1..K in order; no padded k is folded in.  Rows and columns past the edge compute on stale
 // shared memory and are not stored.  A's element (i, k) is A[i * ars + k * aks], B's (k, j) is
-// B[k * bks + j * bcs].  The last shared-memory reads are not followed by a barrier.
+// B[k * bks + j * bcs].  Run by S::THREADS threads in shared memory of their own: one warp, or (THREADS >
+// 32) the whole CTA.
 template <class S, bool ANY, class Op>
 __device__ __forceinline__ void simt4_tile(int r, int c, int ra, int cb, int64_t K, const Op& op, const uint32_t* __restrict__ A,
                                            int64_t ars, int64_t aks, const uint32_t* __restrict__ B, int64_t bks,
@@ -139,29 +149,18 @@ __device__ __forceinline__ void simt4_tile(int r, int c, int ra, int cb, int64_t
                                            uint32_t* smem) {
   constexpr int TM = S::TM, TN = S::TN, BK = S4_BK;
   constexpr int CV = TN % 4 == 0 ? 4 : 2;   // columns per shared-memory read
-  const int lane = threadIdx.x & 31;
-  const int row0 = (lane >> 3) * 4;     // + 16 per four rows
-  const int col0 = (lane & 7) * CV;     // + 8 CV per CV columns
+  const int tid = S::tid(), lane = tid & 31, warp = tid >> 5;
+  const int row0 = (warp % S::WM) * 4 * TM + (lane >> 3) * 4;     // + 16 per four rows
+  const int col0 = (warp / S::WM) * 8 * TN + (lane & 7) * CV;     // + 8 CV per CV columns
+  // a warp whose part lies outside the tile only helps to load
+  const bool idle = S::THREADS > 32 && ((warp % S::WM) * 4 * TM >= r || (warp / S::WM) * 8 * TN >= c);
 
-  S4Loader<S::BM, S::LDA, ANY> la;
-  S4Loader<S::BN, S::LDB, ANY> lb;
-  la.init(A, ars, aks, ra);
-  lb.init(B, bcs, bks, cb);
+  S4Loader<S::BM, S::LDA, S::THREADS, ANY> la;
+  S4Loader<S::BN, S::LDB, S::THREADS, ANY> lb;
+  la.init(A, ars, aks, ra, tid);
+  lb.init(B, bcs, bks, cb, tid);
   const uint32_t smem_u = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   const int64_t panels = (K + BK - 1) / BK;
-  auto load = [&](int64_t p, int stage) {   // panel p into a stage (panels are loaded in order)
-    const int64_t left = K - p * BK;
-    const int kc = static_cast<int>(left < BK ? left : BK);
-    const uint32_t dst = smem_u + static_cast<uint32_t>(stage * (S::PANEL * 4));
-    la.load(dst, ra, kc);
-    lb.load(dst + BK * S::LDA * 4, cb, kc);
-  };
-#pragma unroll
-  for (int p = 0; p < S4_STAGES - 1; ++p) {
-    if (p < panels) load(p, p);
-    cp_async_commit();
-  }
-
   pair4 acc[TM / 2][TN];
 #pragma unroll
   for (int i = 0; i < TM / 2; ++i) {
@@ -210,19 +209,40 @@ __device__ __forceinline__ void simt4_tile(int r, int c, int ra, int cb, int64_t
     }
   };
 
-  int stage = 0;
-  for (int64_t p = 0; p < panels; ++p) {
-    cp_async_wait<S4_STAGES - 2>();
-    __syncwarp();   // panel p is in place, and every lane has left panel p - 1's stage
-    if (p + S4_STAGES - 1 < panels) load(p + S4_STAGES - 1, (stage + S4_STAGES - 1) % S4_STAGES);
+  int stage = 0, load_stage = 0;
+  auto load = [&](int64_t q) {   // panels are loaded in order
+    const int64_t left = K - q * BK;
+    const int kc = static_cast<int>(left < BK ? left : BK);
+    const uint32_t dst = smem_u + static_cast<uint32_t>(load_stage * (S::PANEL * 4));
+    la.load(dst, ra, kc);
+    lb.load(dst + BK * S::LDA * 4, cb, kc);
+    load_stage = (load_stage + 1) % S4_STAGES;
+  };
+  // Panel q is loaded S4_STAGES - 1 panels before it is used.  The largest tile's copies are written
+  // out in one place only, the others' also before the loop (see above).
+  int64_t q = 0;
+  if constexpr (TM <= 8) {
+#pragma unroll
+    for (; q < S4_STAGES - 1; ++q) {
+      if (q < panels) load(q);
+      cp_async_commit();
+    }
+  }
+  for (; q < panels + S4_STAGES - 1; ++q) {
+    cp_async_wait<S4_STAGES - 2>();   // panel q - (S4_STAGES - 1), the oldest but S4_STAGES - 2, is in place
+    S::sync();                        // for every thread, and all have left the stage to be loaded
+    if (q < panels) load(q);
     cp_async_commit();
+    const int64_t p = q - (S4_STAGES - 1);
+    if (p < 0) continue;
     const uint32_t* pa = smem + stage * S::PANEL;
     const uint32_t* pb = pa + BK * S::LDA;
     stage = (stage + 1) % S4_STAGES;
     const int64_t left = K - p * BK;
     pair4 a0[TM / 2], a1[TM / 2];
     uint32_t b0[TN], b1[TN];
-    if (left >= BK) {
+    if (idle) {
+    } else if (left >= BK) {
       read(pa, pb, 0, a0, b0);
 #pragma unroll 4
       for (int k = 0; k < BK; k += 2) {   // the next k's operands are read before this one's FMAs
@@ -239,7 +259,8 @@ __device__ __forceinline__ void simt4_tile(int r, int c, int ra, int cb, int64_t
     }
   }
   cp_async_wait<0>();   // (only empty groups are left)
-  __syncwarp();         // the warp's next tile reuses the stages
+  S::sync();            // the next tile reuses the stages
+  if (idle) return;
 
   // A column of the lane's rows at a time: C's old values, where the epilogue reads them, are all
   // requested before the first is used (one at a time cost 2% at 4096^3).
@@ -268,5 +289,18 @@ __device__ __forceinline__ void simt4_tile(int r, int c, int ra, int cb, int64_t
     }
   }
 }
+
+// jmul!'s chain with the BLAS alpha/beta epilogue (beta == 0: C is not read).
+struct F32Chain {
+  static constexpr bool kInitFromC = false;
+  float alpha, beta;
+  static __device__ __forceinline__ uint32_t init() { return 0x80000000u; }   // -0.0
+  static __device__ __forceinline__ pair4 step(pair4 acc, pair4 a, pair4 b) { return fma_f32x2(a, b, acc); }
+  __device__ __forceinline__ bool reads_c() const { return beta != 0.0f; }
+  __device__ __forceinline__ uint32_t value(uint32_t acc) const { return __float_as_uint(alpha * __uint_as_float(acc)); }
+  __device__ __forceinline__ uint32_t value(uint32_t c, uint32_t acc) const {
+    return __float_as_uint(fmaf(alpha, __uint_as_float(acc), beta * __uint_as_float(c)));
+  }
+};
 
 }  // namespace gb
