@@ -939,7 +939,7 @@ static int semiring_entry(Fn fn, int sr, int ta, int tb, int64_t M, int64_t N, i
   if (sr < 0 || sr >= GB_SEMIRINGS || (accumulate != 0 && accumulate != 1)) return GB_ERR_INVALID_VALUE;
   rc = check_gemm_args(ta, tb, M, N, K, lda, ldb, ldc, A, B, C, true);
   if (rc || M == 0 || N == 0) return rc;
-  return fn(sr, ta, tb, M, N, K, A, lda, B, ldb, accumulate, C, ldc, static_cast<cudaStream_t>(stream));
+  return fn(sr, ta, tb, M, N, K, A, lda, B, ldb, accumulate, C, ldc, dev->sms, static_cast<cudaStream_t>(stream));
 }
 
 // kernel! / initkernel! entry points: argument checks, then the onto-D chain or jmul!'s chain.

@@ -4,7 +4,8 @@
 namespace gb {
 
 int semiring_gemm_f64(int sr, int ta, int tb, int64_t M, int64_t N, int64_t K, const double* A, int64_t lda,
-                      const double* B, int64_t ldb, int accumulate, double* C, int64_t ldc, cudaStream_t s) {
+                      const double* B, int64_t ldb, int accumulate, double* C, int64_t ldc, int sms, cudaStream_t s) {
+  (void)sms;
   return semiring_gemm<double, 64, 64, 16, 4, 4>(sr, ta, tb, M, N, K, A, lda, B, ldb, accumulate, C, ldc, s);
 }
 
