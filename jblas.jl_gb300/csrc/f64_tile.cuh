@@ -1,5 +1,6 @@
 // One FP64 tile of C on the CUDA cores, shared by the native GEMM (native_gemm.cu) and the
-// grouped GEMM (grouped.cu): jmul!'s per-element FMA chain (src/gemm.jl:76-89, 154-168).
+// grouped GEMM (grouped.cu), jmul!'s per-element FMA chain (src/gemm.jl:76-89, 154-168), and by the
+// FP64 semirings (semiring_f64.cu).  What an element does with each k is a policy (F64Chain below).
 //
 // What bounds it: GB300 executes half an FP64 lane per clock and SM partition, so a warp's DFMA
 // holds its partition's FP64 pipe for 64 cycles (measured; the same for 1 or 32 active lanes, and
@@ -83,6 +84,15 @@ struct F64Loader {
     dst = static_cast<uint32_t>(k * (X + 1) + x) * 8u;
     ddst = static_cast<uint32_t>(dk * (X + 1) + dx) * 8u;
   }
+  // Rewrites the elements of a panel that this thread loaded (its copies have arrived).
+  template <class Op>
+  __device__ __forceinline__ void encode(unsigned long long* panel, int extent, int kc) const {
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+      unsigned long long* e = panel + (dst + l * ddst) / 8;
+      if (x + l * dx < extent && k + l * dk < kc) *e = Op::encode(*e);
+    }
+  }
   // Loads the panel of kc k to the shared address `panel`.
   __device__ __forceinline__ void load(uint32_t panel, int extent, int kc) {
     const double* q = p;
@@ -95,25 +105,47 @@ struct F64Loader {
   }
 };
 
+// The policy of the FMA chains:
+//   ONTO = false   the chain starts at -0.0 (fma(a1, x1, -0.0) is the rounded product a1 x1) and
+//                  C = alpha * chain [+ beta * C], written without a multiply when unit (alpha = 1,
+//                  beta = 0: the multiply would run on the FP64 pipe)
+//   ONTO = true    the chain starts at C's value and is stored as it is (jBLAS's kernel!)
+template <bool ONTO>
+struct F64Chain {
+  using Elem = double;   // an element in shared memory, and
+  using Acc = double;    // what a lane keeps for an element of C
+  static constexpr bool ENCODE = false;   // no rewriting of the panels
+  double alpha, beta;
+  bool unit;
+  __device__ __forceinline__ double init(const double* c, bool in) const { return (ONTO && in) ? *c : -0.0; }
+  static __device__ __forceinline__ double step(double acc, double a, double b) { return fma(a, b, acc); }
+  __device__ __forceinline__ void store(double* c, double acc) const {
+    if (ONTO || unit) *c = acc;
+    else *c = (beta == 0.0) ? alpha * acc : fma(alpha, acc, beta * *c);
+  }
+};
+
 // NU chains per lane over the kc k of one panel; off[i] holds the byte offsets of the lane's row
 // of A (low half) and column of B (high half) inside a panel row.  The operands of the next k are
 // read before the DFMAs of this one: with one CTA on an SM nothing else hides the reads' latency.
 // (16 chains, which leave no registers for that, ran at 73% of the pipe on a ragged product.)
-template <int NU, int LDA, int LDB>
+template <class Op, int NU, int LDA, int LDB>
 __device__ __forceinline__ void f64_panel(const char* __restrict__ pa, const char* __restrict__ pb, int kc,
-                                          const uint32_t (&off)[F64_MAX_UNITS], double (&acc)[F64_MAX_UNITS]) {
-  auto read = [&](int k, double (&a)[NU], double (&b)[NU]) {
+                                          const uint32_t (&off)[F64_MAX_UNITS],
+                                          typename Op::Acc (&acc)[F64_MAX_UNITS]) {
+  using E = typename Op::Elem;
+  auto read = [&](int k, E (&a)[NU], E (&b)[NU]) {
 #pragma unroll
     for (int i = 0; i < NU; ++i) {
-      a[i] = *reinterpret_cast<const double*>(pa + k * (LDA * 8) + (off[i] & 0xFFFFu));
-      b[i] = *reinterpret_cast<const double*>(pb + k * (LDB * 8) + (off[i] >> 16));
+      a[i] = *reinterpret_cast<const E*>(pa + k * (LDA * 8) + (off[i] & 0xFFFFu));
+      b[i] = *reinterpret_cast<const E*>(pb + k * (LDB * 8) + (off[i] >> 16));
     }
   };
-  auto step = [&](const double (&a)[NU], const double (&b)[NU]) {
+  auto step = [&](const E (&a)[NU], const E (&b)[NU]) {
 #pragma unroll
-    for (int i = 0; i < NU; ++i) acc[i] = fma(a[i], b[i], acc[i]);
+    for (int i = 0; i < NU; ++i) acc[i] = Op::step(acc[i], a[i], b[i]);
   };
-  double a0[NU], b0[NU], a1[NU], b1[NU];
+  E a0[NU], b0[NU], a1[NU], b1[NU];
   read(0, a0, b0);
   int k = 0;
   for (; k + 2 < kc; k += 2) {
@@ -132,19 +164,13 @@ __device__ __forceinline__ void f64_panel(const char* __restrict__ pa, const cha
 }
 
 // The r x c tile of C at C (its first element; leading dimension ldc), 1 <= r <= XA, 1 <= c <= XB,
-// r c <= F64_MAX_ELEMS:
-//   ONTO = false   the chain starts at -0.0 (fma(a1, x1, -0.0) is the rounded product a1 x1) and
-//                  C = alpha * chain [+ beta * C], written without a multiply when unit (alpha = 1,
-//                  beta = 0: the multiply would run on the FP64 pipe)
-//   ONTO = true    the chain starts at C's value and is stored as it is (jBLAS's kernel!)
-// A's element (i, k) is A[i * ars + k * aks], B's (k, j) is B[k * bks + j * bcs].  `rot` deals the
+// r c <= F64_MAX_ELEMS.  A's element (i, k) is A[i * ars + k * aks], B's (k, j) is B[k * bks + j * bcs].  `rot` deals the
 // units from another warp in each tile, so the partitions share the remainders.  K >= 0.
 // The tile's last shared-memory reads are not followed by a barrier.
-template <bool ONTO, int XA, int XB>
+template <int XA, int XB, class Op>
 __device__ __forceinline__ void f64_tile(int r, int c, int64_t K, const double* __restrict__ A, int64_t ars,
                                          int64_t aks, const double* __restrict__ B, int64_t bks, int64_t bcs,
-                                         double alpha, double beta, bool unit, double* __restrict__ C, int64_t ldc,
-                                         int rot, double* smem) {
+                                         const Op& op, double* __restrict__ C, int64_t ldc, int rot, double* smem) {
   using S = F64Shape<XA, XB>;
   constexpr int BK = S::BK;
   constexpr int MAXU = XA * XB < F64_MAX_ELEMS ? XA * XB / 32 / F64_WARPS : F64_MAX_UNITS;
@@ -176,7 +202,7 @@ __device__ __forceinline__ void f64_tile(int r, int c, int64_t K, const double* 
   // Row and column of each of the lane's elements v * 32 + lane, + 128, ...; past the last element
   // the lane repeats it (and does not store).
   uint32_t off[F64_MAX_UNITS];
-  double acc[F64_MAX_UNITS];
+  typename Op::Acc acc[F64_MAX_UNITS];
   {
     const int e0 = v * 32 + lane;
     int col = e0 / r, row = e0 - col * r;
@@ -187,7 +213,7 @@ __device__ __forceinline__ void f64_tile(int r, int c, int64_t K, const double* 
       const bool in = e0 + i * F64_THREADS < elems;
       const int rr = in ? row : r - 1, cc = in ? col : c - 1;
       off[i] = static_cast<uint32_t>(rr * 8) | (static_cast<uint32_t>(cc * 8) << 16);
-      acc[i] = (ONTO && in) ? C[rr + cc * ldc] : -0.0;
+      acc[i] = op.init(C + rr + cc * ldc, in);
       row += drow;
       col += dcol;
       if (row >= r) {
@@ -199,18 +225,23 @@ __device__ __forceinline__ void f64_tile(int r, int c, int64_t K, const double* 
 
   int stage = 0;
   for (int64_t p = 0; p < panels; ++p) {
+    const int64_t left = K - p * BK;
+    const int kc = static_cast<int>(left < BK ? left : BK);
     cp_async_wait<F64_STAGES - 2>();
+    if constexpr (Op::ENCODE) {
+      unsigned long long* panel = reinterpret_cast<unsigned long long*>(smem) + stage * S::PANEL;
+      la.template encode<Op>(panel, r, kc);
+      lb.template encode<Op>(panel + BK * S::LDA, c, kc);
+    }
     __syncthreads();   // panel p is in place, and every warp has left panel p - 1's stage
     if (p + F64_STAGES - 1 < panels) load(p + F64_STAGES - 1, (stage + F64_STAGES - 1) % F64_STAGES);
     cp_async_commit();
-    const int64_t left = K - p * BK;
-    const int kc = static_cast<int>(left < BK ? left : BK);
     const char* pa = reinterpret_cast<const char*>(smem + stage * S::PANEL);
     const char* pb = pa + BK * S::LDA * 8;
     stage = (stage + 1) % F64_STAGES;
     switch (nu) {   // uniform in the warp
 #define GB_F64_CASE(n_) \
-  case n_: if constexpr (n_ <= MAXU) f64_panel<n_, S::LDA, S::LDB>(pa, pb, kc, off, acc); break;
+  case n_: if constexpr (n_ <= MAXU) f64_panel<Op, n_, S::LDA, S::LDB>(pa, pb, kc, off, acc); break;
       GB_F64_CASE(1) GB_F64_CASE(2) GB_F64_CASE(3) GB_F64_CASE(4) GB_F64_CASE(5) GB_F64_CASE(6) GB_F64_CASE(7)
       GB_F64_CASE(8)
 #undef GB_F64_CASE
@@ -223,26 +254,24 @@ __device__ __forceinline__ void f64_tile(int r, int c, int64_t K, const double* 
   for (int i = 0; i < MAXU; ++i) {
     if (i >= nu) break;
     if (v * 32 + lane + i * F64_THREADS < elems) {
-      double* p = C + (off[i] & 0xFFFFu) / 8 + static_cast<int64_t>(off[i] >> 19) * ldc;
-      if (ONTO || unit) *p = acc[i];
-      else *p = (beta == 0.0) ? alpha * acc[i] : fma(alpha, acc[i], beta * *p);
+      op.store(C + (off[i] & 0xFFFFu) / 8 + static_cast<int64_t>(off[i] >> 19) * ldc, acc[i]);
     }
   }
 }
 
 // The tile on the panel shape that fits it (64 x 32, 32 x 32 or 16 x 16: the smaller ones take
 // fewer barriers per k).
-template <bool ONTO>
+template <class Op>
 __device__ __forceinline__ void f64_tile_any(int r, int c, int64_t K, const double* __restrict__ A, int64_t ars,
                                              int64_t aks, const double* __restrict__ B, int64_t bks, int64_t bcs,
-                                             double alpha, double beta, bool unit, double* __restrict__ C,
-                                             int64_t ldc, int rot, double* smem) {
+                                             const Op& op, double* __restrict__ C, int64_t ldc, int rot,
+                                             double* smem) {
   if (r <= 16 && c <= 16)
-    f64_tile<ONTO, 16, 16>(r, c, K, A, ars, aks, B, bks, bcs, alpha, beta, unit, C, ldc, rot, smem);
+    f64_tile<16, 16>(r, c, K, A, ars, aks, B, bks, bcs, op, C, ldc, rot, smem);
   else if (r <= 32)
-    f64_tile<ONTO, 32, 32>(r, c, K, A, ars, aks, B, bks, bcs, alpha, beta, unit, C, ldc, rot, smem);
+    f64_tile<32, 32>(r, c, K, A, ars, aks, B, bks, bcs, op, C, ldc, rot, smem);
   else
-    f64_tile<ONTO, 64, 32>(r, c, K, A, ars, aks, B, bks, bcs, alpha, beta, unit, C, ldc, rot, smem);
+    f64_tile<64, 32>(r, c, K, A, ars, aks, B, bks, bcs, op, C, ldc, rot, smem);
 }
 
 }  // namespace gb

@@ -317,13 +317,13 @@ __global__ void __launch_bounds__(F64_THREADS, F64_CTAS)
       return;
     }
     const bool unit = __double_as_longlong(p.alpha) == 0x3FF0000000000000ll && __double_as_longlong(p.beta) == 0ll;
+    const F64Chain<false> chain{p.alpha, p.beta, unit};
     const int cols = min(32, F64_MAX_ELEMS / r);   // larger tiles run in column strips
     for (int j0 = 0; j0 < c; j0 += cols) {
       if (j0) __syncthreads();   // the strip reuses the shared panels
-      f64_tile_any<false>(r, min(cols, c - j0), p.k, static_cast<const double*>(p.A) + m0, 1, p.lda,
-                          static_cast<const double*>(p.B) + (n0 + j0) * p.ldb, 1, p.ldb, p.alpha, p.beta, unit,
-                          static_cast<double*>(p.C) + m0 + (n0 + j0) * p.ldc, p.ldc, static_cast<int>(w ^ (w >> 2)),
-                          smem);
+      f64_tile_any(r, min(cols, c - j0), p.k, static_cast<const double*>(p.A) + m0, 1, p.lda,
+                   static_cast<const double*>(p.B) + (n0 + j0) * p.ldb, 1, p.ldb, chain,
+                   static_cast<double*>(p.C) + m0 + (n0 + j0) * p.ldc, p.ldc, static_cast<int>(w ^ (w >> 2)), smem);
     }
   });
 }

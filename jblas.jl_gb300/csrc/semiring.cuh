@@ -64,8 +64,6 @@ struct SrArith<double> {
   static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
   static __device__ __forceinline__ double canon(double v) { return v == 0.0 ? 0.0 : v; }
   static constexpr bool kHas3 = false;
-  static __device__ __forceinline__ double min3(double a, double b, double c) { return fmin(fmin(a, b), c); }
-  static __device__ __forceinline__ double max3(double a, double b, double c) { return fmax(fmax(a, b), c); }
 };
 
 template <>
