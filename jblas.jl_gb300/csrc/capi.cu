@@ -57,10 +57,9 @@ static std::atomic<int> g_ozaki_min_chunks{1};
 // and reconstructs the previous one.  A second stream copies the finished blocks of C of a
 // host-buffer call to the host.  One call holds a lane at a time.
 struct Lane {
-  // fork and join per block of C; the statistics' fork and join; the plan; one for errors;
-  // one per block for its copy to the host and the copies' join
-  static constexpr int STATS_FORK = 2 * TC_MAX_PANELS, STATS_JOIN = STATS_FORK + 1, PLAN = STATS_FORK + 2,
-                       ERROR_JOIN = STATS_FORK + 3, COPY = STATS_FORK + 4, COPY_JOIN = COPY + TC_MAX_PANELS,
+  // fork and join per block of C; one for errors; one per block for its copy to the host and the
+  // copies' join
+  static constexpr int ERROR_JOIN = 2 * TC_MAX_PANELS, COPY = ERROR_JOIN + 1, COPY_JOIN = COPY + TC_MAX_PANELS,
                        EVENTS = COPY_JOIN + 1;
   cudaStream_t stream = nullptr;
   cudaStream_t copy = nullptr;
@@ -363,20 +362,20 @@ static inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 struct OperandStats {
   char* ws = nullptr;
   OzRowStats a{}, b{};
+  unsigned int* counter = nullptr;   // a zeroed word for the planner
 };
 
-// With a lane (and no host copies), B's statistics run on the lane beside A's on `s`, and `s`
-// waits for them before it returns.
 static int run_stats(DeviceInfo* dev, const double* A, int64_t M, int64_t a_rs, int64_t a_ks, const double* B,
                      int64_t N, int64_t b_rs, int64_t b_ks, int64_t K, bool sums, bool host, OperandStats* os,
-                     HostStats* h, cudaStream_t s, Lane* lane = nullptr) {
+                     HostStats* h, cudaStream_t s) {
   const int Sa = oz_stats_kslices(M, K, a_ks, dev->sms), Sb = oz_stats_kslices(N, K, b_ks, dev->sms);
   const int64_t pa = Sa * M, pb = Sb * N;
-  const size_t amax_bytes = align256((M + N) * sizeof(unsigned long long));
+  const size_t amax_bytes = align256((M + N + 1) * sizeof(unsigned long long));   // and the planner's word
   const size_t part_bytes = align256((pa + pb) * sizeof(int32_t));
   GB_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&os->ws), amax_bytes + 3 * part_bytes, dev->pool, s));
   os->a.amax_bits = reinterpret_cast<unsigned long long*>(os->ws);
   os->b.amax_bits = os->a.amax_bits + M;
+  os->counter = reinterpret_cast<unsigned int*>(os->b.amax_bits + N);
   os->a.part_e = reinterpret_cast<int32_t*>(os->ws + amax_bytes);
   os->b.part_e = os->a.part_e + pa;
   os->a.part_sa = reinterpret_cast<float*>(os->ws + amax_bytes + part_bytes);
@@ -385,20 +384,8 @@ static int run_stats(DeviceInfo* dev, const double* A, int64_t M, int64_t a_rs, 
   os->b.part_sq = os->a.part_sq + pa;
   os->a.kslices = Sa;
   os->b.kslices = Sb;
-  if (lane && !host) {
-    cudaError_t e = cudaEventRecord(lane->ev[Lane::STATS_FORK], s);   // after the workspace allocation
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(lane->stream, lane->ev[Lane::STATS_FORK], 0);
-    if (e != cudaSuccess) return gb_set_cuda_error(e, "ozaki statistics fork");
-    int rc = oz_row_stats(A, M, K, a_rs, a_ks, os->a, sums, s);
-    const int rcb = oz_row_stats(B, N, K, b_rs, b_ks, os->b, sums, lane->stream);
-    e = cudaEventRecord(lane->ev[Lane::STATS_JOIN], lane->stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, lane->ev[Lane::STATS_JOIN], 0);
-    if (!rc) rc = rcb;
-    if (!rc && e != cudaSuccess) rc = gb_set_cuda_error(e, "ozaki statistics join");
-    return rc;
-  }
-  int rc = oz_row_stats(A, M, K, a_rs, a_ks, os->a, sums || host, s);
-  if (!rc) rc = oz_row_stats(B, N, K, b_rs, b_ks, os->b, sums || host, s);
+  GB_CUDA_TRY(cudaMemsetAsync(os->ws, 0, amax_bytes, s));
+  const int rc = oz_stats(A, M, a_rs, a_ks, os->a, B, N, b_rs, b_ks, os->b, K, sums || host, s);
   if (rc || !host) return rc;
   std::vector<unsigned long long> amax(M + N);
   std::vector<int32_t> pe(pa + pb);
@@ -690,8 +677,7 @@ static int crt_gemm(DeviceInfo* dev, int ta, int tb, int64_t M, int64_t N, int64
   const bool sums = (moduli == 0 || err_bound_out);
   // Blocks of C: the residue products of block b run on a high-priority lane while this stream
   // splits the operand panels of block b + 1 and reconstructs block b - 1, on the SMs' spare
-  // registers and issue slots beside the tensor-core kernel; before the first products, B's
-  // statistics and first panel split run on the lane beside A's.  One block (the plain
+  // registers and issue slots beside the tensor-core kernel.  One block (the plain
   // sequence on this stream) when the tuning asks for one and under stream capture; at most
   // one block column per 256 columns.
   const TcTuning tune = tc_tuning_for(TC_KIND_CRT, M, N);
@@ -708,7 +694,7 @@ static int crt_gemm(DeviceInfo* dev, int ta, int tb, int64_t M, int64_t N, int64
   } lane_return{dev, lane};
   OperandStats os;
   HostStats h;
-  rc = run_stats(dev, A, M, a_rs, a_ks, B, N, b_rs, b_ks, K, sums, false, &os, &h, s, lane);
+  rc = run_stats(dev, A, M, a_rs, a_ks, B, N, b_rs, b_ks, K, sums, false, &os, &h, s);
   if (rc) {
     if (os.ws) cudaFreeAsync(os.ws, s);
     return rc;
@@ -727,35 +713,24 @@ static int crt_gemm(DeviceInfo* dev, int ta, int tb, int64_t M, int64_t N, int64
     pp.tk[n] = crt_bits_for(K, n);
   }
   // The call's workspace: its plan record (read by its kernels only), residue planes of A and
-  // B, residue-product planes and the row/column exponents.
+  // B, residue-product planes, the row/column exponents and the planner's scratch.
   const int64_t mpad = (M + 255) / 256 * 256, npad = (N + 255) / 256 * 256;
   const size_t plan_bytes = align256(sizeof(CrtDevicePlan));
   const size_t pa_bytes = align256(static_cast<size_t>(n_ws) * M * pitch * 2);
   const size_t pb_bytes = align256(static_cast<size_t>(n_ws) * N * pitch * 2);
   const size_t res_bytes = align256(static_cast<size_t>(n_ws) * mpad * npad);
   const size_t ex_bytes = align256((M + N) * sizeof(int32_t));
+  const size_t ws_bytes = plan_bytes + pa_bytes + pb_bytes + res_bytes + ex_bytes + crt_plan_scratch_bytes();
   char* ws = nullptr;
-  cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws),
-                                          plan_bytes + pa_bytes + pb_bytes + res_bytes + ex_bytes, dev->pool, s);
+  cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), ws_bytes, dev->pool, s);
   if (e != cudaSuccess) {
     cudaFreeAsync(os.ws, s);
     return gb_set_cuda_error(e, "ozaki crt workspace");
   }
   CrtDevicePlan* plan_d = reinterpret_cast<CrtDevicePlan*>(ws);
   char* wsp = ws + plan_bytes;
-  void* scratch = nullptr;
-  e = cudaMallocFromPoolAsync(&scratch, crt_plan_scratch_bytes(), dev->pool, s);
-  if (e != cudaSuccess) {
-    cudaFreeAsync(ws, s);
-    cudaFreeAsync(os.ws, s);
-    return gb_set_cuda_error(e, "ozaki crt planner scratch");
-  }
-  rc = crt_plan_device(os.a, os.b, pp, plan_d, record, seq, scratch, s);
-  cudaFreeAsync(scratch, s);
-  if (!rc && lane) {   // the lane's first split reads the plan
-    const cudaError_t e = cudaEventRecord(lane->ev[Lane::PLAN], s);
-    if (e != cudaSuccess) rc = gb_set_cuda_error(e, "ozaki crt plan event");
-  }
+  rc = crt_plan_device(os.a, os.b, pp, plan_d, record, seq, wsp + pa_bytes + pb_bytes + res_bytes + ex_bytes, os.counter,
+                       s);
   if (!rc && err_bound_out) {
     CrtDevicePlan hp;
     e = cudaMemcpyAsync(&hp, plan_d, sizeof(hp), cudaMemcpyDeviceToHost, s);
@@ -809,9 +784,15 @@ static int crt_gemm(DeviceInfo* dev, int ta, int tb, int64_t M, int64_t N, int64
     if (ctas * moduli_seen <= cap * (moduli_seen - 1)) ctas *= n_ws;
     return static_cast<int>(ctas < cap ? ctas : cap);
   };
+  auto a_rows = [&](int64_t r0, int64_t r1) {
+    return CrtSplitSide{A + r0 * a_rs, r1 - r0, a_rs, a_ks, os.a.amax_bits + r0, pa + r0 * pitch, M, ea + r0};
+  };
+  auto b_rows = [&](int64_t r0, int64_t r1) {
+    return CrtSplitSide{B + r0 * b_rs, r1 - r0, b_rs, b_ks, os.b.amax_bits + r0, pb + r0 * pitch, N, eb + r0};
+  };
   if (!lane) {
-    rc = crt_split(A, M, K, a_rs, a_ks, os.a.amax_bits, plan_d, pa, pitch, M, ea, s);
-    if (!rc) rc = crt_split(B, N, K, b_rs, b_ks, os.b.amax_bits, plan_d, pb, pitch, N, eb, s);
+    const CrtSplitSide sa = a_rows(0, M), sb = b_rows(0, N);
+    rc = crt_split(&sa, &sb, K, plan_d, pitch, s);
     if (!rc) {
       ga.grid = grid_for(M, N);
       rc = crt_mma_launch(ga, plan, s);
@@ -845,19 +826,9 @@ static int crt_gemm(DeviceInfo* dev, int ta, int tb, int64_t M, int64_t N, int64
     const int nblocks = prow * pcol;
     for (int b = 0; b < nblocks && !rc; ++b) {
       const int r = b / pcol, c = b % pcol;
-      if (!rc && !b_done[c]) {   // the first block's B panel on the lane, beside A's split here
-        cudaStream_t bs = (b == 0) ? hs : s;
-        if (b == 0) cu(cudaStreamWaitEvent(hs, lane->ev[Lane::PLAN], 0));
-        if (!rc)
-          rc = crt_split(B + n0[c] * b_rs, n0[c + 1] - n0[c], K, b_rs, b_ks, os.b.amax_bits + n0[c], plan_d,
-                         pb + n0[c] * pitch, pitch, N, eb + n0[c], bs);
-        b_done[c] = true;
-      }
-      if (!rc && !a_done[r]) {
-        rc = crt_split(A + m0[r] * a_rs, m0[r + 1] - m0[r], K, a_rs, a_ks, os.a.amax_bits + m0[r], plan_d,
-                       pa + m0[r] * pitch, pitch, M, ea + m0[r], s);
-        a_done[r] = true;
-      }
+      const CrtSplitSide sa = a_rows(m0[r], m0[r + 1]), sb = b_rows(n0[c], n0[c + 1]);
+      if (!a_done[r] || !b_done[c]) rc = crt_split(a_done[r] ? nullptr : &sa, b_done[c] ? nullptr : &sb, K, plan_d, pitch, s);
+      a_done[r] = b_done[c] = true;
       if (!rc) cu(cudaEventRecord(lane->ev[2 * b], s));
       if (!rc) cu(cudaStreamWaitEvent(hs, lane->ev[2 * b], 0));
       if (!rc) rc = crt_mma_launch(block_args(r, c), plan, hs);

@@ -226,24 +226,62 @@ __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsig
   return a > b ? a : b;
 }
 
-// k contiguous (ks == 1): one warp per row, one K slice.
+// One operand of the statistics launch: element (r, k) at X[r rs + k ks]; the body that fits its
+// layout and alignment, with gx blocks along the rows (times st.kslices K slices of kslice).
+struct StatsSide {
+  const double* X;
+  int64_t R, K, rs, ks, kslice;
+  OzRowStats st;
+  uint32_t gx;
+  int32_t way;
+};
+enum { STATS_KC, STATS_KC2, STATS_RC, STATS_RC2 };
+
+struct StatsShared {
+  unsigned long long mx[8][64];
+  float sa[8][64], sq[8][64];
+  int e[64];
+};
+
+// k contiguous (ks == 1): one warp per row, one K slice.  The next eight loads are in flight while
+// the current eight are folded in.
 template <bool SUMS>
-__global__ void __launch_bounds__(256) stats_kc_kernel(const double* __restrict__ X, int64_t R, int64_t K,
-                                                       int64_t rs, OzRowStats st) {
+__device__ __forceinline__ void stats_kc(const StatsSide& sd, uint32_t block) {
+  const double* __restrict__ X = sd.X;
+  const int64_t R = sd.R, K = sd.K, rs = sd.rs;
+  const OzRowStats& st = sd.st;
   const int lane = threadIdx.x & 31;
-  const int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5);
+  const int64_t r = static_cast<int64_t>(block) * 8 + (threadIdx.x >> 5);
   if (r >= R) return;
   const unsigned long long* row = reinterpret_cast<const unsigned long long*>(X + r * rs);
   RunStats rs_;
   int64_t k = lane;
-  for (; k + 96 < K; k += 128) {
-    const unsigned long long b0 = row[k], b1 = row[k + 32], b2 = row[k + 64], b3 = row[k + 96];
-    rs_.add(b0, SUMS);
-    rs_.add(b1, SUMS);
-    rs_.add(b2, SUMS);
-    rs_.add(b3, SUMS);
+  if (k + 224 < K) {
+    unsigned long long b[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) b[q] = row[k + 32 * q];
+    for (; k + 256 + 224 < K; k += 256) {
+      unsigned long long n[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) n[q] = row[k + 256 + 32 * q];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        rs_.add(b[q], SUMS);
+        b[q] = n[q];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) rs_.add(b[q], SUMS);
+    k += 256;
   }
-  for (; k < K; k += 32) rs_.add(row[k], SUMS);
+  {   // fewer than eight are left
+    unsigned long long b[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) b[q] = k + 32 * q < K ? row[k + 32 * q] : 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (k + 32 * q < K) rs_.add(b[q], SUMS);
+  }
   unsigned long long mx = rs_.mx;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = umax64(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -270,13 +308,16 @@ __global__ void __launch_bounds__(256) stats_kc_kernel(const double* __restrict_
 
 // rows contiguous (rs == 1): 32 rows x one K slice per block, 8 warps stride over k.
 template <bool SUMS>
-__global__ void __launch_bounds__(256) stats_rc_kernel(const double* __restrict__ X, int64_t R, int64_t K,
-                                                       int64_t ks, int64_t kslice, OzRowStats st) {
-  __shared__ unsigned long long smx[8][32];
-  __shared__ float ssa[8][32], ssq[8][32];
+__device__ __forceinline__ void stats_rc(const StatsSide& sd, uint32_t bx, uint32_t by, StatsShared& sh) {
+  const double* __restrict__ X = sd.X;
+  const int64_t R = sd.R, K = sd.K, ks = sd.ks, kslice = sd.kslice;
+  const OzRowStats& st = sd.st;
+  auto& smx = sh.mx;
+  auto& ssa = sh.sa;
+  auto& ssq = sh.sq;
   const int tr = threadIdx.x & 31, tk = threadIdx.x >> 5;
-  const int64_t r = static_cast<int64_t>(blockIdx.x) * 32 + tr;
-  const int64_t k0 = static_cast<int64_t>(blockIdx.y) * kslice;
+  const int64_t r = static_cast<int64_t>(bx) * 32 + tr;
+  const int64_t k0 = static_cast<int64_t>(by) * kslice;
   const int64_t k1 = (k0 + kslice < K) ? k0 + kslice : K;
   const unsigned long long* Xb = reinterpret_cast<const unsigned long long*>(X);
   RunStats rs_;
@@ -309,7 +350,7 @@ __global__ void __launch_bounds__(256) stats_rc_kernel(const double* __restrict_
       sa += ssa[w][tr];
       sq += ssq[w][tr];
     }
-    const int64_t o = static_cast<int64_t>(blockIdx.y) * R + r;
+    const int64_t o = static_cast<int64_t>(by) * R + r;
     st.part_e[o] = e;
     st.part_sa[o] = sa;
     st.part_sq[o] = sq;
@@ -321,10 +362,12 @@ __global__ void __launch_bounds__(256) stats_rc_kernel(const double* __restrict_
 // k contiguous: one warp per row, lane l reads the pairs (k, k + 1) with k = 2 (l + 32 i).
 // Needs the row starts 16-byte aligned (X aligned, rs even).
 template <bool SUMS>
-__global__ void __launch_bounds__(256) stats_kc2_kernel(const double* __restrict__ X, int64_t R, int64_t K,
-                                                        int64_t rs, OzRowStats st) {
+__device__ __forceinline__ void stats_kc2(const StatsSide& sd, uint32_t block) {
+  const double* __restrict__ X = sd.X;
+  const int64_t R = sd.R, K = sd.K, rs = sd.rs;
+  const OzRowStats& st = sd.st;
   const int lane = threadIdx.x & 31;
-  const int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5);
+  const int64_t r = static_cast<int64_t>(block) * 8 + (threadIdx.x >> 5);
   if (r >= R) return;
   const ulonglong2* row = reinterpret_cast<const ulonglong2*>(X + r * rs);
   const int64_t K2 = K / 2;
@@ -385,22 +428,25 @@ __global__ void __launch_bounds__(256) stats_kc2_kernel(const double* __restrict
 // rows contiguous: 64 rows x one K slice per block, lane l holds rows 2l and 2l + 1 of the
 // block (one 16-byte load per k), 8 warps stride over k.  Needs X aligned, ks even, R even.
 template <bool SUMS>
-__global__ void __launch_bounds__(256) stats_rc2_kernel(const double* __restrict__ X, int64_t R, int64_t K,
-                                                        int64_t ks, int64_t kslice, OzRowStats st) {
-  __shared__ unsigned long long smx[8][64];
-  __shared__ float ssa[8][64], ssq[8][64];
-  __shared__ int sexp[64];
+__device__ __forceinline__ void stats_rc2(const StatsSide& sd, uint32_t bx, uint32_t by, StatsShared& sh) {
+  const double* __restrict__ X = sd.X;
+  const int64_t R = sd.R, K = sd.K, ks = sd.ks, kslice = sd.kslice;
+  const OzRowStats& st = sd.st;
+  auto& smx = sh.mx;
+  auto& ssa = sh.sa;
+  auto& ssq = sh.sq;
+  auto& sexp = sh.e;
   const int lane = threadIdx.x & 31, tk = threadIdx.x >> 5;
-  const int64_t rb = static_cast<int64_t>(blockIdx.x) * 64;
+  const int64_t rb = static_cast<int64_t>(bx) * 64;
   const int64_t r = rb + 2 * lane;   // rows r and r + 1 (R even: both valid or both not)
-  const int64_t k0 = static_cast<int64_t>(blockIdx.y) * kslice;
+  const int64_t k0 = static_cast<int64_t>(by) * kslice;
   const int64_t k1 = (k0 + kslice < K) ? k0 + kslice : K;
   const ulonglong2* Xb = reinterpret_cast<const ulonglong2*>(X);
   RunStats s0, s1;
   if (r < R) {
     const int64_t h = r >> 1, hs = ks >> 1;   // pair index of (r, k): (r + k ks) / 2
     int64_t k = k0 + tk;
-    // software-pipelined as in stats_kc2_kernel
+    // software-pipelined as in stats_kc2
     if (k + 24 < k1) {
       ulonglong2 b[4] = {Xb[h + k * hs], Xb[h + (k + 8) * hs], Xb[h + (k + 16) * hs], Xb[h + (k + 24) * hs]};
       for (; k + 32 + 24 < k1; k += 32) {
@@ -460,11 +506,29 @@ __global__ void __launch_bounds__(256) stats_rc2_kernel(const double* __restrict
         sa += ssa[w][rr];
         sq += ssq[w][rr];
       }
-      const int64_t o = static_cast<int64_t>(blockIdx.y) * R + row;
+      const int64_t o = static_cast<int64_t>(by) * R + row;
       st.part_e[o] = sexp[rr];
       st.part_sa[o] = sa;
       st.part_sq[o] = sq;
     }
+  }
+}
+
+// Both operands in one launch: A's blocks, then B's.  Alone, an operand of a mid-size product leaves
+// most of the chip idle for as long as one row takes.  1531 x 1999 x 1021, rows of 1021 unaligned
+// doubles: two launches of 15 us on four loads a lane, 18 us in one on eight.
+template <bool SUMS>
+__global__ void __launch_bounds__(256) stats_kernel(const __grid_constant__ StatsSide a,
+                                                    const __grid_constant__ StatsSide b, uint32_t blocks_a) {
+  __shared__ StatsShared sh;
+  const bool second = blockIdx.x >= blocks_a;
+  const StatsSide& sd = second ? b : a;
+  const uint32_t block = second ? blockIdx.x - blocks_a : blockIdx.x;
+  switch (sd.way) {
+    case STATS_KC: stats_kc<SUMS>(sd, block); break;
+    case STATS_KC2: stats_kc2<SUMS>(sd, block); break;
+    case STATS_RC: stats_rc<SUMS>(sd, block % sd.gx, block / sd.gx, sh); break;
+    default: stats_rc2<SUMS>(sd, block % sd.gx, block / sd.gx, sh); break;
   }
 }
 
@@ -480,43 +544,37 @@ int oz_stats_kslices(int64_t R, int64_t K, int64_t ks, int sms) {
   return static_cast<int>((K + kslice - 1) / kslice);
 }
 
-int oz_row_stats(const double* X, int64_t R, int64_t K, int64_t rs, int64_t ks, OzRowStats st, bool sums,
-                 cudaStream_t s) {
-  if (R <= 0) return GB_OK;
-  GB_CUDA_TRY(cudaMemsetAsync(st.amax_bits, 0, R * sizeof(unsigned long long), s));
-  if (K <= 0) return GB_OK;
+// One operand's side of the launch and its number of blocks.
+static int64_t stats_side(const double* X, int64_t R, int64_t K, int64_t rs, int64_t ks, const OzRowStats& st,
+                          StatsSide* sd) {
   const bool aligned = (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-  if (ks == 1 && aligned && (rs & 1) == 0) {
-    const int64_t blocks = (R + 7) / 8;
-    if (sums)
-      GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s,
-                stats_kc2_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, s>>>(X, R, K, rs, st));
-    else
-      GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s,
-                stats_kc2_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, s>>>(X, R, K, rs, st));
-  } else if (ks != 1 && rs == 1 && aligned && (ks & 1) == 0 && (R & 1) == 0) {
-    const int64_t kslice = (K + st.kslices - 1) / st.kslices;
-    dim3 grid(static_cast<unsigned>((R + 63) / 64), static_cast<unsigned>(st.kslices));
-    if (sums)
-      GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s, stats_rc2_kernel<true><<<grid, 256, 0, s>>>(X, R, K, ks, kslice, st));
-    else
-      GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s, stats_rc2_kernel<false><<<grid, 256, 0, s>>>(X, R, K, ks, kslice, st));
-  } else if (ks == 1) {
-    const int64_t blocks = (R + 7) / 8;
-    if (sums)
-      GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s,
-                stats_kc_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, s>>>(X, R, K, rs, st));
-    else
-      GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s,
-                stats_kc_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, s>>>(X, R, K, rs, st));
-  } else {
-    const int64_t kslice = (K + st.kslices - 1) / st.kslices;
-    dim3 grid(static_cast<unsigned>((R + 31) / 32), static_cast<unsigned>(st.kslices));
-    if (sums)
-      GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s, stats_rc_kernel<true><<<grid, 256, 0, s>>>(X, R, K, ks, kslice, st));
-    else
-      GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s, stats_rc_kernel<false><<<grid, 256, 0, s>>>(X, R, K, ks, kslice, st));
-  }
+  const bool kc = ks == 1;
+  sd->X = X;
+  sd->R = R;
+  sd->K = K;
+  sd->rs = rs;
+  sd->ks = ks;
+  sd->kslice = (K + st.kslices - 1) / st.kslices;
+  sd->st = st;
+  if (kc) sd->way = aligned && (rs & 1) == 0 ? STATS_KC2 : STATS_KC;
+  else sd->way = rs == 1 && aligned && (ks & 1) == 0 && (R & 1) == 0 ? STATS_RC2 : STATS_RC;
+  const int64_t rows = kc ? 8 : sd->way == STATS_RC2 ? 64 : 32;
+  const int64_t gx = (R + rows - 1) / rows;
+  sd->gx = static_cast<uint32_t>(gx);
+  return gx * (kc ? 1 : st.kslices);
+}
+
+int oz_stats(const double* A, int64_t M, int64_t a_rs, int64_t a_ks, const OzRowStats& sa, const double* B, int64_t N,
+             int64_t b_rs, int64_t b_ks, const OzRowStats& sb, int64_t K, bool sums, cudaStream_t s) {
+  if (M <= 0 || N <= 0 || K <= 0) return GB_OK;
+  StatsSide a, b;
+  const int64_t ba = stats_side(A, M, K, a_rs, a_ks, sa, &a), bb = stats_side(B, N, K, b_rs, b_ks, sb, &b);
+  if (ba + bb > 0x7FFFFFFF) return GB_ERR_UNSUPPORTED;
+  const unsigned grid = static_cast<unsigned>(ba + bb), first = static_cast<unsigned>(ba);
+  if (sums)
+    GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s, stats_kernel<true><<<grid, 256, 0, s>>>(a, b, first));
+  else
+    GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s, stats_kernel<false><<<grid, 256, 0, s>>>(a, b, first));
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
 }

@@ -35,7 +35,7 @@ int oz_make_plan_chunks(int64_t M, int64_t N, int64_t K, int slices, int min_chu
 double oz_plan_cost(const OzPlan& p);
 
 // Per-row statistics of op(X) (rows r < R, contraction index k < K), cut into `kslices`
-// K slices: amax bits of |x| per row (uint64, exact; zeroed and filled by oz_row_stats),
+// K slices: amax bits of |x| per row (uint64, exact; zeroed by the caller, filled by oz_stats),
 // and per slice s the exponent e_s of the slice's max (max < 2^e_s) with FP32 sums of
 // |x| 2^-e_s and x^2 2^-2e_s over truncated values ([s][R] arrays; only with sums = true).
 // The host rescales the slice sums to the row exponent and bounds them one-sidedly.
@@ -49,8 +49,9 @@ struct OzRowStats {
 
 // K slices the statistics kernel uses for this layout (1 when k is contiguous).
 int oz_stats_kslices(int64_t R, int64_t K, int64_t ks, int sms);
-int oz_row_stats(const double* X, int64_t R, int64_t K, int64_t rs, int64_t ks, OzRowStats st, bool sums,
-                 cudaStream_t s);
+// Statistics of both operands of a product in one launch; the amax words are zero on entry.
+int oz_stats(const double* A, int64_t M, int64_t a_rs, int64_t a_ks, const OzRowStats& sa, const double* B, int64_t N,
+             int64_t b_rs, int64_t b_ks, const OzRowStats& sb, int64_t K, bool sums, cudaStream_t s);
 // Writes `slices` digit planes (BF16, [slice][row][pitch]) and per-row exponents.
 int oz_split(const double* X, int64_t R, int64_t K, int64_t rs, int64_t ks,
              const unsigned long long* amax_bits, int slices, int bits, __nv_bfloat16* planes,
@@ -164,15 +165,25 @@ int crt_plan_record(CrtPlanRecord** record, unsigned long long* seq);
 // Planner: from the statistics (with sums), the fewest moduli whose bound meets pp.tol (or
 // pp.n_fixed) and the widest t they allow; writes *plan (the call's workspace) and the tagged
 // copy *record on the device.  `scratch` holds crt_plan_scratch_bytes() bytes of stream-ordered
-// workspace.
+// workspace, `counter` is a zeroed word of it.
 size_t crt_plan_scratch_bytes();
 int crt_plan_device(const OzRowStats& sa, const OzRowStats& sb, const CrtPlanParams& pp, CrtDevicePlan* plan,
-                    CrtPlanRecord* record, unsigned long long seq, void* scratch, cudaStream_t s);
-// Residue planes (BF16, [modulus][row][pitch], plan->n of them) and row exponents of rows
-// [0, R) of op(X); the planes belong to an operand of plane_rows >= R rows (a band of rows
-// passes X, amax_bits, planes and exps offset to its first row, and the operand's row count).
-int crt_split(const double* X, int64_t R, int64_t K, int64_t rs, int64_t ks, const unsigned long long* amax_bits,
-              const CrtDevicePlan* plan, __nv_bfloat16* planes, int64_t pitch, int64_t plane_rows, int32_t* exps,
+                    CrtPlanRecord* record, unsigned long long seq, void* scratch, unsigned int* counter,
+                    cudaStream_t s);
+// One operand (or a band of its rows) for crt_split: rows [0, R) of op(X), element (r, k) at
+// X[r rs + k ks], to residue planes (BF16, [modulus][plane_rows][pitch], plan->n of them) and row
+// exponents.  The planes belong to an operand of plane_rows >= R rows: a band passes X, amax_bits,
+// planes and exps offset to its first row, and the operand's row count.
+struct CrtSplitSide {
+  const double* X;
+  int64_t R, rs, ks;
+  const unsigned long long* amax_bits;
+  __nv_bfloat16* planes;
+  int64_t plane_rows;
+  int32_t* exps;
+};
+// Splits A, B or both (null: not that one) in one launch.
+int crt_split(const CrtSplitSide* a, const CrtSplitSide* b, int64_t K, const CrtDevicePlan* plan, int64_t pitch,
               cudaStream_t s);
 
 struct CrtGemmArgs {

@@ -304,6 +304,11 @@ int crt_plan_record(CrtPlanRecord** record, unsigned long long* seq) {
 // Many blocks reduce row ranges (sums relative to the block's largest row exponent); the
 // last block to finish combines them in block order and chooses the plan.  Terms smaller
 // than 2^-1022 of the largest are dropped: far inside the 1.01 slack of the bound.
+//
+// Bound by a chain of FP64 instructions, each of which holds an SM partition for 64 cycles, so they
+// are spread over warps and lanes (a warp sums one operand's partials, a lane one quantity), maxima
+// of non-negative doubles are taken as integers, and a lane's log2 is FP64 only where FP32 cannot
+// decide.  1531 + 1999 rows: 23 -> 14 us.
 constexpr int CRT_PLAN_THREADS = 256;
 constexpr int CRT_PLAN_BLOCKS = 128;   // per operand at most
 
@@ -312,7 +317,7 @@ struct CrtPlanPartial {
   int32_t ref, nonfinite, any, pad;
 };
 
-size_t crt_plan_scratch_bytes() { return sizeof(CrtPlanPartial) * 2 * CRT_PLAN_BLOCKS + 256; }
+size_t crt_plan_scratch_bytes() { return sizeof(CrtPlanPartial) * 2 * CRT_PLAN_BLOCKS; }
 
 __device__ __forceinline__ int exp_of_bits_dev(unsigned long long bits) {
   if (bits >= 0x7FF0000000000000ull) return 0x7FFFFFFF;
@@ -331,6 +336,16 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
+// max of non-negative doubles, on the integer ALUs
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
+__device__ __forceinline__ double warp_max_nonneg(double x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x = max_nonneg(x, __shfl_xor_sync(0xffffffffu, x, o));
+  return x;
+}
+
 __device__ double crt_bound_dev(bool nonfinite, double na, double nb, double EA, double EB, double SA, double SB,
                                 int64_t K, int t) {
   if (nonfinite) return INFINITY;
@@ -344,14 +359,20 @@ __device__ double crt_bound_dev(bool nonfinite, double na, double nb, double EA,
 
 __device__ int crt_bits_dev(double sa_max, double sb_max, int64_t K, double lm) {
   const double Kd = static_cast<double>(K < 1 ? 1 : K);
-  // S(t) >= min(sa_max, sb_max, K): start from the t that bound allows and step down
-  const double ls = log2(fmin(fmin(sa_max, sb_max), Kd));
+  // S(t) >= min(sa_max, sb_max, K): start from the t that bound allows and step down.  log2 in FP32
+  // is within 1e-4 of the FP64 one here (S <= 2^60), so it decides unless a limit is that close.
+  const double lim = fmin(lm - 2.0 - 1e-9, 125.0 - 1e-9);
+  const float flim = static_cast<float>(lim);
+  const float ls = log2f(static_cast<float>(fmin(fmin(sa_max, sb_max), Kd)));
   int t0 = 62;
-  const double cap = fmin(lm - 2.0, 125.0) - ls;
-  if (cap < 124.0) t0 = min(62, static_cast<int>(floor(cap * 0.5)) + 1);
+  const float cap = flim - ls + 1e-3f;
+  if (cap < 124.0f) t0 = min(62, static_cast<int>(floorf(cap * 0.5f)) + 1);
   for (int t = t0; t >= 1; --t) {
     double S = fmin(sa_max, sb_max) + Kd * ldexp(1.0, -t - 1);
     S = fmin(S, Kd) * (1.0 + 1e-12);
+    const float room = flim - 2.0f * t - log2f(static_cast<float>(S));
+    if (room < -1e-3f) continue;
+    if (room > 1e-3f) return t;
     const double need = 2.0 * t + log2(S);
     if (need + 2.0 <= lm - 1e-9 && need <= 125.0 - 1e-9) return t;
   }
@@ -435,14 +456,13 @@ __global__ void __launch_bounds__(CRT_PLAN_THREADS) crt_plan_kernel(const OzRowS
       e2 += sc * sc;
       s2 += (su * sc) * (su * sc);
       n2 += ssq * down * (sc * sc);
-      smax = fmax(smax, su);
+      smax = max_nonneg(smax, su);
     }
   }
   e2 = warp_sum(e2);
   s2 = warp_sum(s2);
   n2 = warp_sum(n2);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) smax = fmax(smax, __shfl_xor_sync(0xffffffffu, smax, o));
+  smax = warp_max_nonneg(smax);
   __syncthreads();
   if (lane == 0) {
     s_acc[0][wid] = e2;
@@ -451,34 +471,33 @@ __global__ void __launch_bounds__(CRT_PLAN_THREADS) crt_plan_kernel(const OzRowS
     s_acc[3][wid] = smax;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (wid == 0) {   // lane q: quantity q over the warps
+    const double* acc = s_acc[lane & 3];
+    double sum = 0.0;
+    for (int w = 0; w < CRT_PLAN_THREADS / 32; ++w) sum = (lane & 3) == 3 ? max_nonneg(sum, acc[w]) : sum + acc[w];
     CrtPlanPartial pt;
-    pt.e2 = pt.s2 = pt.n2 = pt.smax = 0.0;
-    for (int w = 0; w < CRT_PLAN_THREADS / 32; ++w) {
-      pt.e2 += s_acc[0][w];
-      pt.s2 += s_acc[1][w];
-      pt.n2 += s_acc[2][w];
-      pt.smax = fmax(pt.smax, s_acc[3][w]);
-    }
+    pt.e2 = __shfl_sync(0xffffffffu, sum, 0);
+    pt.s2 = __shfl_sync(0xffffffffu, sum, 1);
+    pt.n2 = __shfl_sync(0xffffffffu, sum, 2);
+    pt.smax = __shfl_sync(0xffffffffu, sum, 3);
     pt.ref = ref;
     pt.nonfinite = nf;
     pt.any = (ref > -1100) ? 1 : 0;
     pt.pad = 0;
-    part[blockIdx.x] = pt;
-    __threadfence();
-    s_last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+    if (lane == 0) {
+      part[blockIdx.x] = pt;
+      __threadfence();
+      s_last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+    }
   }
   __syncthreads();
-  if (!s_last || threadIdx.x >= 32) return;
+  if (!s_last || threadIdx.x >= 64) return;
   __threadfence();
-  // last block, warp 0: combine the partials of each operand (lane l takes blocks l, l + 32, ...;
-  // butterfly reductions leave the same sums in every lane), then lane c - 1 evaluates c moduli
-  // and a ballot picks the fewest that pass
-  double nrm[2], E[2], S[2], smx[2];
-  int nonfinite = 0;
-#pragma unroll
-  for (int op = 0; op < 2; ++op) {
-    const int b0 = op ? blocks_a : 0, b1 = op ? static_cast<int>(gridDim.x) : blocks_a;
+  // last block: warps 0 and 1 combine the partials of one operand each (lane l takes blocks l, l + 32,
+  // ...; butterfly reductions leave the same sums in every lane), then lane c - 1 of warp 0 evaluates c
+  // moduli and a ballot picks the fewest that pass
+  {
+    const int b0 = wid ? blocks_a : 0, b1 = wid ? static_cast<int>(gridDim.x) : blocks_a;
     int gref = -1100, nfl = 0;
     for (int b = b0 + lane; b < b1; b += 32) {
       const CrtPlanPartial& q = part[b];
@@ -490,7 +509,6 @@ __global__ void __launch_bounds__(CRT_PLAN_THREADS) crt_plan_kernel(const OzRowS
       gref = max(gref, __shfl_xor_sync(0xffffffffu, gref, o));
       nfl |= __shfl_xor_sync(0xffffffffu, nfl, o);
     }
-    nonfinite |= nfl;
     double ae2 = 0.0, as2 = 0.0, an2 = 0.0, amx = 0.0;
     for (int b = b0 + lane; b < b1; b += 32) {
       const CrtPlanPartial& q = part[b];
@@ -499,26 +517,36 @@ __global__ void __launch_bounds__(CRT_PLAN_THREADS) crt_plan_kernel(const OzRowS
       ae2 += q.e2 * f;
       as2 += q.s2 * f;
       an2 += q.n2 * f;
-      amx = fmax(amx, q.smax);
+      amx = max_nonneg(amx, q.smax);
     }
     ae2 = warp_sum(ae2);
     as2 = warp_sum(as2);
     an2 = warp_sum(an2);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amx = fmax(amx, __shfl_xor_sync(0xffffffffu, amx, o));
-    nrm[op] = sqrt(an2);
-    E[op] = sqrt(ae2);
-    S[op] = sqrt(as2);
-    smx[op] = amx;
+    amx = warp_max_nonneg(amx);
+    const double root = sqrt(lane == 0 ? an2 : lane == 1 ? ae2 : as2);
+    if (lane < 3) s_acc[wid][lane] = root;   // |x| norm, exponent and sum norms
+    if (lane == 3) {
+      s_acc[wid][3] = amx;
+      s_nf[wid] = nfl;
+    }
   }
+  asm volatile("bar.sync 1, 64;" ::: "memory");
+  if (wid != 0) return;
+  const double nrm[2] = {s_acc[0][0], s_acc[1][0]}, E[2] = {s_acc[0][1], s_acc[1][1]};
+  const double S[2] = {s_acc[0][2], s_acc[1][2]}, smx[2] = {s_acc[0][3], s_acc[1][3]};
+  const int nonfinite = s_nf[0] | s_nf[1];
   int n = pp.n_fixed, t = pp.t_fixed;
+  double bound = 0.0;
+  bool known = false;
   if (n == 0) {
     const int c = lane + 1;
     int tc = 0;
     bool ok = false;
+    double mine = 0.0;
     if (c <= TC_MAX_MODULI) {
       tc = nonfinite ? pp.tk[c] : crt_bits_dev(smx[0], smx[1], pp.K, pp.log2m[c]);
-      ok = tc >= 1 && (nonfinite || crt_bound_dev(false, nrm[0], nrm[1], E[0], E[1], S[0], S[1], pp.K, tc) <= pp.tol);
+      mine = crt_bound_dev(nonfinite, nrm[0], nrm[1], E[0], E[1], S[0], S[1], pp.K, tc);
+      ok = tc >= 1 && (nonfinite || mine <= pp.tol);
     }
     const unsigned pass = __ballot_sync(0xffffffffu, ok);
     const int tmax = __shfl_sync(0xffffffffu, tc, TC_MAX_MODULI - 1);
@@ -526,6 +554,8 @@ __global__ void __launch_bounds__(CRT_PLAN_THREADS) crt_plan_kernel(const OzRowS
       const int first = __ffs(pass) - 1;
       n = first + 1;
       t = __shfl_sync(0xffffffffu, tc, first);
+      bound = __shfl_sync(0xffffffffu, mine, first);
+      known = true;
     } else {   // tolerance out of reach: the most moduli
       n = TC_MAX_MODULI;
       t = tmax >= 1 ? tmax : pp.tk[n];
@@ -534,15 +564,15 @@ __global__ void __launch_bounds__(CRT_PLAN_THREADS) crt_plan_kernel(const OzRowS
   if (lane == 0) {
     out->n = n;
     out->t = t;
-    out->bound = crt_bound_dev(nonfinite, nrm[0], nrm[1], E[0], E[1], S[0], S[1], pp.K, t);
+    out->bound = known ? bound : crt_bound_dev(nonfinite, nrm[0], nrm[1], E[0], E[1], S[0], S[1], pp.K, t);
     record->plan = *out;
     record->seq = seq;
-    *counter = 0u;
   }
 }
 
 int crt_plan_device(const OzRowStats& sa, const OzRowStats& sb, const CrtPlanParams& pp, CrtDevicePlan* plan,
-                    CrtPlanRecord* record, unsigned long long seq, void* scratch, cudaStream_t s) {
+                    CrtPlanRecord* record, unsigned long long seq, void* scratch, unsigned int* counter,
+                    cudaStream_t s) {
   auto blocks_for = [](int64_t R) {
     int64_t b = (R + CRT_PLAN_THREADS - 1) / CRT_PLAN_THREADS;
     if (b > CRT_PLAN_BLOCKS) b = CRT_PLAN_BLOCKS;
@@ -550,9 +580,6 @@ int crt_plan_device(const OzRowStats& sa, const OzRowStats& sb, const CrtPlanPar
   };
   const int ba = blocks_for(pp.M), bb = blocks_for(pp.N);
   CrtPlanPartial* part = static_cast<CrtPlanPartial*>(scratch);
-  unsigned int* counter = reinterpret_cast<unsigned int*>(static_cast<char*>(scratch) +
-                                                          sizeof(CrtPlanPartial) * 2 * CRT_PLAN_BLOCKS);
-  GB_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned int), s));
   GB_LAUNCH(GB_KERNEL_OZAKI_STATS, s,
             (crt_plan_kernel<<<ba + bb, CRT_PLAN_THREADS, 0, s>>>(sa, sb, pp, ba, part, counter, plan, record,
                                                                    seq)));
@@ -680,87 +707,88 @@ __device__ __forceinline__ void crt_split8(const double (&x)[8], int e, int tbit
   for (int g = 0; g < nmod; ++g) store_residues(out0 + g * plane_stride, crt_residues8<ND>(d, mod, g), nvalid);
 }
 
-// k contiguous: one thread = one row and 8 consecutive k, neighbouring threads neighbouring k
-// (a warp reads 2 KB and writes 512 B of one row per plane).  One 16-byte store per plane.
-__global__ void __launch_bounds__(256) crt_split_kc_kernel(const double* __restrict__ X, int64_t R, int64_t K,
-                                                           int64_t rs, int64_t ks,
-                                                           const unsigned long long* __restrict__ amax_bits,
-                                                           __nv_bfloat16* __restrict__ planes, int64_t pitch,
-                                                           int64_t plane_stride, int32_t* __restrict__ exps,
-                                                           const __grid_constant__ CrtModuli mod,
-                                                           const CrtDevicePlan* __restrict__ plan) {
-  const int64_t kc = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, r = blockIdx.y;
-  const int64_t k0 = kc * 8;
-  if (r >= R || k0 >= K) return;
-  const int nmod = plan->n, tbits = plan->t;
-  const int e = row_exponent(amax_bits[r]);
-  if (k0 == 0) exps[r] = e;
-  const bool nonfinite = (e == OZ_EXP_NONFINITE);
-  const int nvalid = static_cast<int>(K - k0 < 8 ? K - k0 : 8);
-  const double* src = X + r * rs + k0 * ks;
-  double x[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) x[j] = (j < nvalid) ? src[j * ks] : 0.0;
-  __nv_bfloat16* out0 = planes + r * pitch + k0;
-  if (tbits <= 52) crt_split8<4>(x, e, tbits, nonfinite, nmod, mod, out0, plane_stride, nvalid);
-  else crt_split8<5>(x, e, tbits, nonfinite, nmod, mod, out0, plane_stride, nvalid);
-}
+// Threads of a split launch, 8 consecutive k of one row each, one 16-byte store per plane:
+//   k contiguous      tpr = 2^log_tpr threads along k (as many as a row has chunks, at most 256), the
+//                     other 256 / tpr along rows; a warp reads 2 KB and writes 512 B per plane.  A row
+//                     to a block left half of the threads of a 1021-long row without work.
+//   rows contiguous   warp w of a block owns rows 4w..4w+3 of a 32-row x 64-k tile; lane l takes row
+//                     4w + l / 8 and chunk l % 8.  Each of its 8 loads is one 8-byte element, and a
+//                     warp's load instruction reads 8 whole 32-byte sectors (4 rows of one column, 8
+//                     columns); per modulus a warp stores 4 rows x 128 bytes of the plane, whole lines.
+// No shared memory and no barriers: the residue work of one modulus overlaps the stores of the
+// previous one.  A's blocks come first, then B's.  1531 x 1999 x 1021, both operands k-contiguous, 15
+// moduli: 27 + 31 us in two launches of a row to a block, 37 in one.
+struct CrtSplitPart {
+  CrtSplitSide side;
+  uint32_t gx;   // blocks along k (k contiguous) or along the rows (rows contiguous)
+  int32_t log_tpr, rows_contiguous;
+};
 
-// Rows contiguous (element (r, k) at X[r + k ks]): warp w of a CTA owns rows 4w..4w+3 of a
-// 32-row x 64-k tile; lane l takes row 4w + l / 8 and the 8 consecutive k of chunk l % 8.  Each
-// of its 8 loads is one 8-byte element, and a warp's load instruction reads 8 whole 32-byte
-// sectors (4 rows of one column, 8 columns); per modulus a warp stores 4 rows x 128 bytes of
-// the plane, whole lines.  No shared memory and no barriers: the residue work of one modulus
-// overlaps the stores of the previous one.
-__global__ void __launch_bounds__(256) crt_split_rc_kernel(const double* __restrict__ X, int64_t R, int64_t K,
-                                                           int64_t ks, const unsigned long long* __restrict__ amax_bits,
-                                                           __nv_bfloat16* __restrict__ planes, int64_t pitch,
-                                                           int64_t plane_stride, int32_t* __restrict__ exps,
-                                                           const __grid_constant__ CrtModuli mod,
-                                                           const CrtDevicePlan* __restrict__ plan) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t r = static_cast<int64_t>(blockIdx.x) * 32 + 4 * w + (lane >> 3);
-  const int64_t k0 = static_cast<int64_t>(blockIdx.y) * 64 + 8 * (lane & 7);
-  if (r >= R || k0 >= K) return;
-  const int nmod = plan->n, tbits = plan->t;
-  const int e = row_exponent(amax_bits[r]);
-  if (k0 == 0) exps[r] = e;
-  const bool nonfinite = (e == OZ_EXP_NONFINITE);
-  const int nvalid = static_cast<int>(K - k0 < 8 ? K - k0 : 8);
-  const double* src = X + r + k0 * ks;
-  double x[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) x[j] = (j < nvalid) ? src[j * ks] : 0.0;
-  __nv_bfloat16* out0 = planes + r * pitch + k0;
-  if (tbits <= 52) crt_split8<4>(x, e, tbits, nonfinite, nmod, mod, out0, plane_stride, nvalid);
-  else crt_split8<5>(x, e, tbits, nonfinite, nmod, mod, out0, plane_stride, nvalid);
-}
-
-int crt_split(const double* X, int64_t R, int64_t K, int64_t rs, int64_t ks, const unsigned long long* amax_bits,
-              const CrtDevicePlan* plan, __nv_bfloat16* planes, int64_t pitch, int64_t plane_rows, int32_t* exps,
-              cudaStream_t s) {
-  const CrtModuli& mod = crt_table().mod;
-  if (R <= 0 || K <= 0) return GB_OK;
-  if (plane_rows < R) return GB_ERR_INVALID_VALUE;
-  const int64_t plane_stride = plane_rows * pitch;   // modulus planes of the whole operand
-  if (rs == 1 && R > 1) {
-    const int64_t gy = (K + 63) / 64;
-    if (gy > 65535 || (R + 31) / 32 > 0x7FFFFFFF) return GB_ERR_UNSUPPORTED;
-    dim3 grid(static_cast<unsigned>((R + 31) / 32), static_cast<unsigned>(gy));
-    GB_LAUNCH(GB_KERNEL_OZAKI_SPLIT, s,
-              (crt_split_rc_kernel<<<grid, 256, 0, s>>>(X, R, K, ks, amax_bits, planes, pitch, plane_stride, exps,
-                                                        mod, plan)));
+__global__ void __launch_bounds__(256) crt_split_kernel(const __grid_constant__ CrtSplitPart a,
+                                                        const __grid_constant__ CrtSplitPart b, uint32_t blocks_a,
+                                                        int64_t K, int64_t pitch, const __grid_constant__ CrtModuli mod,
+                                                        const CrtDevicePlan* __restrict__ plan) {
+  const bool second = blockIdx.x >= blocks_a;
+  const CrtSplitPart& part = second ? b : a;
+  const uint32_t block = second ? blockIdx.x - blocks_a : blockIdx.x;
+  const uint32_t by = block / part.gx, bx = block - by * part.gx;
+  int64_t r, k0;
+  if (part.rows_contiguous) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    r = static_cast<int64_t>(bx) * 32 + 4 * w + (lane >> 3);
+    k0 = static_cast<int64_t>(by) * 64 + 8 * (lane & 7);
   } else {
-    const int64_t kchunks = (K + 7) / 8;
-    for (int64_t r0 = 0; r0 < R; r0 += 65535) {   // rows beyond the grid's y range: bands
-      const int64_t rb = (R - r0 < 65535) ? R - r0 : 65535;
-      dim3 grid(static_cast<unsigned>((kchunks + 255) / 256), static_cast<unsigned>(rb));
-      GB_LAUNCH(GB_KERNEL_OZAKI_SPLIT, s,
-                (crt_split_kc_kernel<<<grid, 256, 0, s>>>(X + r0 * rs, rb, K, rs, ks, amax_bits + r0,
-                                                          planes + r0 * pitch, pitch, plane_stride, exps + r0, mod,
-                                                          plan)));
-    }
+    const int lt = part.log_tpr;
+    r = (static_cast<int64_t>(by) << (8 - lt)) + (threadIdx.x >> lt);
+    k0 = ((static_cast<int64_t>(bx) << lt) + (threadIdx.x & ((1 << lt) - 1))) * 8;
   }
+  if (r >= part.side.R || k0 >= K) return;
+  const int nmod = plan->n, tbits = plan->t;
+  const int e = row_exponent(part.side.amax_bits[r]);
+  if (k0 == 0) part.side.exps[r] = e;
+  const bool nonfinite = (e == OZ_EXP_NONFINITE);
+  const int nvalid = static_cast<int>(K - k0 < 8 ? K - k0 : 8);
+  const int64_t ks = part.side.ks, plane_stride = part.side.plane_rows * pitch;
+  const double* __restrict__ src = part.side.X + r * part.side.rs + k0 * ks;
+  double x[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) x[j] = (j < nvalid) ? src[j * ks] : 0.0;
+  __nv_bfloat16* out0 = part.side.planes + r * pitch + k0;
+  if (tbits <= 52) crt_split8<4>(x, e, tbits, nonfinite, nmod, mod, out0, plane_stride, nvalid);
+  else crt_split8<5>(x, e, tbits, nonfinite, nmod, mod, out0, plane_stride, nvalid);
+}
+
+// One operand's part of the launch; its number of blocks, or -1.
+static int64_t crt_split_part(const CrtSplitSide* side, int64_t K, CrtSplitPart* p) {
+  std::memset(p, 0, sizeof(*p));
+  p->gx = 1;
+  if (!side || side->R <= 0 || K <= 0) return 0;
+  if (side->plane_rows < side->R) return -1;
+  p->side = *side;
+  p->rows_contiguous = (side->rs == 1 && side->R > 1) ? 1 : 0;
+  if (p->rows_contiguous) {
+    const int64_t gx = (side->R + 31) / 32;
+    p->gx = static_cast<uint32_t>(gx);
+    return gx * ((K + 63) / 64);
+  }
+  const int64_t chunks = (K + 7) / 8;
+  while (p->log_tpr < 8 && (1 << p->log_tpr) < chunks) ++p->log_tpr;
+  const int64_t gx = (chunks + (1 << p->log_tpr) - 1) >> p->log_tpr, rows = 256 >> p->log_tpr;
+  p->gx = static_cast<uint32_t>(gx);
+  return gx * ((side->R + rows - 1) / rows);
+}
+
+int crt_split(const CrtSplitSide* a, const CrtSplitSide* b, int64_t K, const CrtDevicePlan* plan, int64_t pitch,
+              cudaStream_t s) {
+  CrtSplitPart pa, pb;
+  const int64_t ba = crt_split_part(a, K, &pa), bb = crt_split_part(b, K, &pb);
+  if (ba < 0 || bb < 0) return GB_ERR_INVALID_VALUE;
+  if (ba + bb == 0) return GB_OK;
+  if (((pa.rows_contiguous || pb.rows_contiguous) && (K + 63) / 64 > 65535) || ba + bb > 0x7FFFFFFF)
+    return GB_ERR_UNSUPPORTED;
+  GB_LAUNCH(GB_KERNEL_OZAKI_SPLIT, s,
+            (crt_split_kernel<<<static_cast<unsigned>(ba + bb), 256, 0, s>>>(pa, pb, static_cast<uint32_t>(ba), K, pitch,
+                                                                             crt_table().mod, plan)));
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
 }
