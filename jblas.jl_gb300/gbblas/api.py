@@ -25,17 +25,26 @@ class DimensionMismatch(ValueError):
     """Operand shapes do not conform (Julia's DimensionMismatch)."""
 
 
-def _stream_ptr(t):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+# The small calls are bound by the host: of 11.7 us for a 16 x 14 x 32 jmul_, 3.7 are the C call and its
+# launch.  So the calls below pass integers straight to the C signatures (which convert them), take the
+# current stream as an integer (a torch.cuda.Stream object per call costs 2 us) and read each shape
+# once: 7.0 us.
+def _stream_of(t):
+    """The current stream of t's device (an integer); t is a CUDA tensor."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def _storage(X, name, allow_copy):
     """(tensor, ld, trans) with X == (trans ? S^T : S) for column-major S of leading dim ld."""
     if X.dim() != 2:
         raise DimensionMismatch("%s must be a matrix, got %d dims" % (name, X.dim()))
+    return _layout(X, *X.shape, name, allow_copy)
+
+
+def _layout(X, r, c, name, allow_copy):
+    """_storage of an r x c matrix."""
     if not X.is_cuda:
         raise ValueError("%s must be a CUDA tensor (device memory)" % name)
-    r, c = X.shape
     s0, s1 = X.stride()
     if (s0 == 1 or r <= 1) and (c <= 1 or s1 >= max(1, r)):
         return X, (s1 if c > 1 else max(1, r)), 0
@@ -61,23 +70,21 @@ def gemm_raw(transA, transB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, *, dt
              mode=_lib.MODE_NATIVE, slices=0, want_bound=False, stream=None):
     """Direct C-ABI call on device pointers (ints).  Returns the error bound or None."""
     L = _lib.lib()
-    st = ctypes.c_void_p(stream)
     if dtype == torch.float64:
-        bound = ctypes.c_double(0.0)
-        rc = L.gb_gemm_f64(int(transA), int(transB), M, N, K, float(alpha), ctypes.c_void_p(A), lda,
-                           ctypes.c_void_p(B), ldb, float(beta), ctypes.c_void_p(C), ldc, int(mode),
-                           int(slices), ctypes.byref(bound) if want_bound else None, st)
+        bound = ctypes.c_double(0.0) if want_bound else None
+        rc = L.gb_gemm_f64(int(transA), int(transB), M, N, K, float(alpha), A, lda, B, ldb, float(beta), C, ldc,
+                           int(mode), int(slices), ctypes.byref(bound) if want_bound else None, stream)
         check(rc, "gb_gemm_f64")
         return bound.value if want_bound else None
     if mode in (_lib.MODE_OZAKI_BF16, _lib.MODE_OZAKI_INT8, _lib.MODE_OZAKI_CRT):
         raise ValueError("Ozaki modes emulate float64; float32 runs natively or in a BF16 term mode")
     if mode == _lib.MODE_NATIVE:
-        rc = L.gb_gemm_f32(int(transA), int(transB), M, N, K, float(alpha), ctypes.c_void_p(A), lda,
-                           ctypes.c_void_p(B), ldb, float(beta), ctypes.c_void_p(C), ldc, st)
+        rc = L.gb_gemm_f32(int(transA), int(transB), M, N, K, float(alpha), A, lda, B, ldb, float(beta), C, ldc,
+                           stream)
         check(rc, "gb_gemm_f32")
     else:
-        rc = L.gb_gemm_f32_ex(int(transA), int(transB), M, N, K, float(alpha), ctypes.c_void_p(A), lda,
-                              ctypes.c_void_p(B), ldb, float(beta), ctypes.c_void_p(C), ldc, int(mode), st)
+        rc = L.gb_gemm_f32_ex(int(transA), int(transB), M, N, K, float(alpha), A, lda, B, ldb, float(beta), C, ldc,
+                              int(mode), stream)
         check(rc, "gb_gemm_f32_ex")
     return None
 
@@ -101,13 +108,13 @@ def gemm_(C, A, B, alpha=1.0, beta=0.0, *, mode="native", slices=0, return_bound
     dt = _dtype_of(C, A, B)
     M, K = A.shape
     K2, N = B.shape
-    if K2 != K or tuple(C.shape) != (M, N):
+    if K2 != K or C.shape != (M, N):
         raise DimensionMismatch("A is %dx%d, B is %dx%d, C is %dx%d" % (M, K, K2, N, *C.shape))
     md = _MODES[mode] if isinstance(mode, str) else int(mode)
-    Cs, ldc, tc = _storage(C, "C", allow_copy=False)
-    As, lda, ta = _storage(A, "A", allow_copy=True)
-    Bs, ldb, tb = _storage(B, "B", allow_copy=True)
-    stream = torch.cuda.current_stream(C.device).cuda_stream
+    Cs, ldc, tc = _layout(C, M, N, "C", False)
+    As, lda, ta = _layout(A, M, K, "A", True)
+    Bs, ldb, tb = _layout(B, K, N, "B", True)
+    stream = _stream_of(C)
     if tc == 0:
         bound = gemm_raw(ta, tb, M, N, K, alpha, As.data_ptr(), lda, Bs.data_ptr(), ldb, beta,
                          Cs.data_ptr(), ldc, dtype=dt, mode=md, slices=slices,
@@ -178,6 +185,9 @@ def jmul_host(D, A, X):
     return gemm_host(D, A, X, 1.0, 0.0, mode="native")
 
 
+_PREFETCH, _LOCALITY = 7, 3   # jmul!'s defaults
+
+
 def jmul_(D, A, X, a_prefetch=7, x_prefetch=7, a_loc=3, x_loc=3, d_loc=3):
     """jmul!(D, A, X[, Val(Aprefetch_freq), Val(Xprefetch_freq), Val(A_loc), Val(X_loc), Val(D_loc)]):
     D = A * X with jBLAS's per-element FMA order (src/gemm.jl:244-246).
@@ -185,12 +195,13 @@ def jmul_(D, A, X, a_prefetch=7, x_prefetch=7, a_loc=3, x_loc=3, d_loc=3):
     The trailing arguments are jmul!'s software-prefetch distances and cache localities, CPU
     cache hints; they are checked (non-negative integers, localities 0..3) and have no GPU
     counterpart (the operands stream through shared memory)."""
-    for name, v in (("a_prefetch", a_prefetch), ("x_prefetch", x_prefetch)):
-        if not isinstance(v, int) or v < 0:
-            raise ValueError("%s must be a non-negative integer, got %r" % (name, v))
-    for name, v in (("a_loc", a_loc), ("x_loc", x_loc), ("d_loc", d_loc)):
-        if not isinstance(v, int) or not 0 <= v <= 3:
-            raise ValueError("%s must be a cache locality 0..3, got %r" % (name, v))
+    if not (a_prefetch is x_prefetch is _PREFETCH and a_loc is x_loc is d_loc is _LOCALITY):   # not the defaults
+        for name, v in (("a_prefetch", a_prefetch), ("x_prefetch", x_prefetch)):
+            if not isinstance(v, int) or v < 0:
+                raise ValueError("%s must be a non-negative integer, got %r" % (name, v))
+        for name, v in (("a_loc", a_loc), ("x_loc", x_loc), ("d_loc", d_loc)):
+            if not isinstance(v, int) or not 0 <= v <= 3:
+                raise ValueError("%s must be a cache locality 0..3, got %r" % (name, v))
     return gemm_(D, A, X, 1.0, 0.0, mode="native")
 
 
@@ -263,10 +274,9 @@ def gemm_strided_batched_(C, A, B, alpha=1.0, beta=0.0):
     sb, ldb = batch_cm(B, K, N, "B")
     sc, ldc = batch_cm(C, M, N, "C")
     name = "gb_gemm_strided_batched_f64" if dt == torch.float64 else "gb_gemm_strided_batched_f32"
-    st = torch.cuda.current_stream(C.device).cuda_stream
-    rc = getattr(_lib.lib(), name)(M, N, K, float(alpha), ctypes.c_void_p(A.data_ptr()), max(1, lda), sa,
-                                  ctypes.c_void_p(B.data_ptr()), max(1, ldb), sb, float(beta),
-                                  ctypes.c_void_p(C.data_ptr()), max(1, ldc), sc, cnt, ctypes.c_void_p(st))
+    st = _stream_of(C) if C.is_cuda else torch.cuda.current_stream(C.device).cuda_stream
+    rc = getattr(_lib.lib(), name)(M, N, K, float(alpha), A.data_ptr(), max(1, lda), sa, B.data_ptr(), max(1, ldb), sb,
+                                  float(beta), C.data_ptr(), max(1, ldc), sc, cnt, st)
     check(rc, name)
     return C
 
@@ -294,21 +304,21 @@ def gemm_semiring_(C, A, B, semiring="min_plus", accumulate=False):
         raise ValueError("unknown semiring %r (one of %s)" % (semiring, ", ".join(_lib.SEMIRINGS)))
     M, K = A.shape
     K2, N = B.shape
-    if K2 != K or tuple(C.shape) != (M, N):
+    if K2 != K or C.shape != (M, N):
         raise DimensionMismatch("A is %dx%d, B is %dx%d, C is %dx%d" % (M, K, K2, N, *C.shape))
-    Cs, ldc, tc = _storage(C, "C", allow_copy=False)
-    As, lda, ta = _storage(A, "A", allow_copy=True)
-    Bs, ldb, tb = _storage(B, "B", allow_copy=True)
+    Cs, ldc, tc = _layout(C, M, N, "C", False)
+    As, lda, ta = _layout(A, M, K, "A", True)
+    Bs, ldb, tb = _layout(B, K, N, "B", True)
     fn = getattr(_lib.lib(), _SEMIRING_FN[dt])
     sr = _lib.SEMIRINGS[semiring]
-    st = _stream_ptr(C)
+    st = _stream_of(C)
     if tc == 0:
-        rc = fn(sr, ta, tb, M, N, K, ctypes.c_void_p(As.data_ptr()), lda, ctypes.c_void_p(Bs.data_ptr()), ldb,
-                int(bool(accumulate)), ctypes.c_void_p(Cs.data_ptr()), ldc, st)
+        rc = fn(sr, ta, tb, M, N, K, As.data_ptr(), lda, Bs.data_ptr(), ldb, int(bool(accumulate)), Cs.data_ptr(), ldc,
+                st)
     else:
         # C stored row-major: C^T = B^T (x) A^T ((x) is commutative in every semiring offered)
-        rc = fn(sr, 1 - tb, 1 - ta, N, M, K, ctypes.c_void_p(Bs.data_ptr()), ldb, ctypes.c_void_p(As.data_ptr()),
-                lda, int(bool(accumulate)), ctypes.c_void_p(Cs.data_ptr()), ldc, st)
+        rc = fn(sr, 1 - tb, 1 - ta, N, M, K, Bs.data_ptr(), ldb, As.data_ptr(), lda, int(bool(accumulate)),
+                Cs.data_ptr(), ldc, st)
     check(rc, _SEMIRING_FN[dt])
     return C
 
