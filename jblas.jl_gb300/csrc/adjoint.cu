@@ -18,6 +18,7 @@
 
 #include "gb_common.cuh"
 #include "profile.cuh"
+#include "split_terms.cuh"
 #include "tc_gemm.cuh"
 
 namespace gb {
@@ -36,54 +37,54 @@ __device__ __forceinline__ void split_terms(float x, uint32_t (&t)[NT]) {
   }
 }
 
-// k contiguous or strided (element (r, k) at X[r*rs + k*ks]): one thread = one row r and 16
-// consecutive k, neighbouring threads neighbouring k; writes the NT term planes
-// [term][r][pitch], 32 bytes per plane per thread.  With ks == 1 the 16 values are read as four
-// 16-byte loads when aligned.
-template <int NT>
-__global__ void __launch_bounds__(256) split_kc_kernel(const float* __restrict__ X, int64_t R, int64_t Kd,
-                                                       int64_t rs, int64_t ks, __nv_bfloat16* __restrict__ planes,
-                                                       int64_t pitch, int64_t plane) {
-  const int64_t kc = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, r = blockIdx.y;
-  const int64_t k0 = kc * 16;
-  if (r >= R || k0 >= Kd) return;
-  const int nvalid = static_cast<int>(Kd - k0 < 16 ? Kd - k0 : 16);
-  const float* src = X + r * rs + k0 * ks;
-  float x[16];
-  if (ks == 1 && nvalid == 16 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+// The term planes of up to three operands in one launch, each operand's blocks in turn.  Bound by memory:
+// 4 bytes read and 2 NT written an element.  An operand alone is 8 to 15 us of a mid-size product, much
+// of it the launch and the last wave.
+//   chunks   (element (r, k) at X[r rs + k ks], any strides): a thread takes 8 consecutive k of a
+//            row, a 16-byte store per plane; tpr = 2^log_tpr threads along k (as many as a row has
+//            chunks, at most 256), the other 256 / tpr along rows.  With ks == 1 and an aligned row
+//            the 8 values are two 16-byte loads; an unaligned row costs a warp 8 lines per load (16 k
+//            a thread: 16 lines, and a row to a block left half the threads of 2047 k idle).
+//   tile     (rows contiguous): a 64 x 64 tile through shared memory.  Warp w loads columns
+//            8w..8w+7 (lanes along r: 128-byte loads); a thread then splits 16 k of one row and
+//            stores 32 bytes of every plane, and for the transposed planes 16 rows of one k (whole
+//            lines in both layouts).  The terms stay in registers; keeping them in shared memory
+//            for both layouts cost 48 conflicting 2-byte stores a thread.
+// 3001 x 2047 and 2047 x 2503, three terms: 16 + 15.5 us in two launches, 22 us in one.
+struct SplitPart {
+  SplitOperand op;
+  uint32_t first;   // first block
+  uint32_t gx;      // chunks: blocks along k; tile: blocks along the rows
+  int32_t log_tpr, tile;
+};
+struct SplitParts {
+  SplitPart part[SPLIT_MAX_OPERANDS];
+};
+
+// N consecutive values -> 2 N bytes of each of NT planes at dst + i plane (the first nvalid of them).
+template <int NT, int N>
+__device__ __forceinline__ void store_terms(const float (&x)[N], __nv_bfloat16* dst, int64_t plane, int nvalid) {
+  uint32_t packed[NT][N / 2];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 v = reinterpret_cast<const float4*>(src)[q];
-      x[4 * q] = v.x;
-      x[4 * q + 1] = v.y;
-      x[4 * q + 2] = v.z;
-      x[4 * q + 3] = v.w;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) x[j] = (j < nvalid) ? src[j * ks] : 0.0f;
-  }
-  uint32_t packed[NT][8];
-#pragma unroll
-  for (int j = 0; j < 16; j += 2) {
+  for (int j = 0; j < N; j += 2) {
     uint32_t t0[NT], t1[NT];
     split_terms<NT>(x[j], t0);
     split_terms<NT>(x[j + 1], t1);
 #pragma unroll
     for (int i = 0; i < NT; ++i) packed[i][j / 2] = t0[i] | (t1[i] << 16);
   }
-  __nv_bfloat16* dst = planes + r * pitch + k0;
-  if (nvalid == 16) {
+  if (nvalid == N) {
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
       uint4* d4 = reinterpret_cast<uint4*>(dst + i * plane);
-      d4[0] = make_uint4(packed[i][0], packed[i][1], packed[i][2], packed[i][3]);
-      d4[1] = make_uint4(packed[i][4], packed[i][5], packed[i][6], packed[i][7]);
+#pragma unroll
+      for (int q = 0; q < N / 8; ++q)
+        d4[q] = make_uint4(packed[i][4 * q], packed[i][4 * q + 1], packed[i][4 * q + 2], packed[i][4 * q + 3]);
     }
   } else {   // unrolled with a predicate: the packed terms stay in registers
     unsigned short* d2 = reinterpret_cast<unsigned short*>(dst);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < N; ++j) {
       if (j < nvalid) {
 #pragma unroll
         for (int i = 0; i < NT; ++i)
@@ -93,19 +94,39 @@ __global__ void __launch_bounds__(256) split_kc_kernel(const float* __restrict__
   }
 }
 
-// Rows contiguous (element (r, k) at X[r + k*ks]): a CTA converts a 64 x 64 tile through shared
-// memory.  Warp w loads columns 8w..8w+7 (lanes along r: 128-byte loads); the terms go to
-// [r][k] shared tiles; each warp then stores 8 rows x 128 B of every plane, and with DUAL also
-// 8 k-rows x 128 B of the transposed planes [k][r] — whole lines in both layouts.
-template <int NT, bool DUAL>
-__global__ void __launch_bounds__(256) split_rc_tile_kernel(const float* __restrict__ X, int64_t R, int64_t Kd,
-                                                            int64_t ks, __nv_bfloat16* __restrict__ planes,
-                                                            int64_t pitch, __nv_bfloat16* __restrict__ planes_t,
-                                                            int64_t pitch_t) {
-  __shared__ float tile[64][65];                                 // [k][r]
-  __shared__ __align__(16) unsigned short ts[NT][64][72];       // [term][r][k], 144-byte rows
+template <int NT>
+__device__ __forceinline__ void split_chunks(const SplitPart& p, uint32_t block) {
+  const SplitOperand& o = p.op;
+  const uint32_t by = block / p.gx, bx = block - by * p.gx;
+  const int lt = p.log_tpr;
+  const int64_t r = (static_cast<int64_t>(by) << (8 - lt)) + (threadIdx.x >> lt);
+  const int64_t k0 = ((static_cast<int64_t>(bx) << lt) + (threadIdx.x & ((1 << lt) - 1))) * 8;
+  if (r >= o.R || k0 >= o.K) return;
+  const int nvalid = static_cast<int>(o.K - k0 < 8 ? o.K - k0 : 8);
+  const float* __restrict__ src = o.X + r * o.rs + k0 * o.ks;
+  float x[8];
+  if (o.ks == 1 && nvalid == 8 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float4 v = reinterpret_cast<const float4*>(src)[q];
+      x[4 * q] = v.x;
+      x[4 * q + 1] = v.y;
+      x[4 * q + 2] = v.z;
+      x[4 * q + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = (j < nvalid) ? src[j * o.ks] : 0.0f;
+  }
+  store_terms<NT>(x, o.planes + r * o.pitch + k0, o.R * o.pitch, nvalid);
+}
+
+template <int NT>
+__device__ __forceinline__ void split_tile(const SplitPart& p, uint32_t block, float (&tile)[64][65]) {
+  const SplitOperand& o = p.op;
+  const uint32_t by = block / p.gx, bx = block - by * p.gx;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int64_t r0 = static_cast<int64_t>(blockIdx.x) * 64, k0 = static_cast<int64_t>(blockIdx.y) * 64;
+  const int64_t r0 = static_cast<int64_t>(bx) * 64, k0 = static_cast<int64_t>(by) * 64;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     const int kk = w * 8 + c;
@@ -114,98 +135,80 @@ __global__ void __launch_bounds__(256) split_rc_tile_kernel(const float* __restr
     for (int h = 0; h < 2; ++h) {
       const int rr = lane + 32 * h;
       const int64_t r = r0 + rr;
-      tile[kk][rr] = (r < R && k < Kd) ? X[r + k * ks] : 0.0f;
+      tile[kk][rr] = (r < o.R && k < o.K) ? o.X[r + k * o.ks] : 0.0f;
     }
   }
   __syncthreads();
-  const int rr = tid >> 2, kb = (tid & 3) * 16;   // this thread's row and 16-wide k chunk
+  const int line = tid >> 2, at = (tid & 3) * 16;   // this thread's row (k row) and 16-wide chunk
+  float x[16];
+  if (r0 + line < o.R && k0 + at < o.K) {   // planes [r][k]
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    uint32_t t[NT];
-    split_terms<NT>(tile[kb + j][rr], t);
-#pragma unroll
-    for (int i = 0; i < NT; ++i) ts[i][rr][kb + j] = static_cast<unsigned short>(t[i]);
+    for (int j = 0; j < 16; ++j) x[j] = tile[at + j][line];
+    const int64_t left = o.K - k0 - at;
+    store_terms<NT>(x, o.planes + (r0 + line) * o.pitch + k0 + at, o.R * o.pitch, static_cast<int>(left < 16 ? left : 16));
   }
-  __syncthreads();
-  {   // row-major planes [r][k]
-    const int64_t r = r0 + rr, k = k0 + kb;
-    if (r < R && k < Kd) {
-      const int nvalid = static_cast<int>(Kd - k < 16 ? Kd - k : 16);
+  if (o.planes_t && k0 + line < o.K && r0 + at < o.R) {   // planes [k][r]
 #pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        unsigned short* d = reinterpret_cast<unsigned short*>(planes) + (i * R + r) * pitch + k;
-        if (nvalid == 16) {
-          const uint4* src = reinterpret_cast<const uint4*>(&ts[i][rr][kb]);
-          reinterpret_cast<uint4*>(d)[0] = src[0];
-          reinterpret_cast<uint4*>(d)[1] = src[1];
-        } else {
-          for (int j = 0; j < nvalid; ++j) d[j] = ts[i][rr][kb + j];
-        }
-      }
-    }
-  }
-  if (DUAL) {   // transposed planes [k][r]: this thread's k row (tid >> 2) and 16-wide r chunk
-    const int kk = tid >> 2, rb = (tid & 3) * 16;
-    const int64_t k = k0 + kk, r = r0 + rb;
-    if (k < Kd && r < R) {
-      const int nvalid = static_cast<int>(R - r < 16 ? R - r : 16);
-#pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        unsigned short* d = reinterpret_cast<unsigned short*>(planes_t) + (i * Kd + k) * pitch_t + r;
-        if (nvalid == 16) {
-          uint32_t p[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            p[q] = static_cast<uint32_t>(ts[i][rb + 2 * q][kk]) | (static_cast<uint32_t>(ts[i][rb + 2 * q + 1][kk]) << 16);
-          reinterpret_cast<uint4*>(d)[0] = make_uint4(p[0], p[1], p[2], p[3]);
-          reinterpret_cast<uint4*>(d)[1] = make_uint4(p[4], p[5], p[6], p[7]);
-        } else {
-          for (int q = 0; q < nvalid; ++q) d[q] = ts[i][rb + q][kk];
-        }
-      }
-    }
+    for (int j = 0; j < 16; ++j) x[j] = tile[line][at + j];
+    const int64_t left = o.R - r0 - at;
+    store_terms<NT>(x, o.planes_t + (k0 + line) * o.pitch_t + r0 + at, o.K * o.pitch_t,
+                    static_cast<int>(left < 16 ? left : 16));
   }
 }
 
-// BF16 term planes of the R x Kd operand whose element (r, k) is X[r*rs + k*ks]: planes
-// [term][r][pitch] (and with planes_t, from the same read, [term][k][pitch_t]; rows contiguous
-// only).  nterms = 2 or 3.
-int split_bf16_terms(const float* X, int64_t R, int64_t Kd, int64_t rs, int64_t ks, int nterms,
-                     __nv_bfloat16* planes, int64_t pitch, __nv_bfloat16* planes_t, int64_t pitch_t, int kind,
-                     cudaStream_t s) {
-  if (R <= 0 || Kd <= 0) return GB_OK;
-  if (nterms != 2 && nterms != 3) return GB_ERR_INVALID_VALUE;
-  if (rs == 1 || planes_t) {
-    if (rs != 1) return GB_ERR_UNSUPPORTED;   // the transposed layout is written from row-contiguous X
-    const int64_t ktiles = (Kd + 63) / 64;
-    if (ktiles > 65535 || (R + 63) / 64 > 0x7FFFFFFF) return GB_ERR_UNSUPPORTED;
-    dim3 grid(static_cast<unsigned>((R + 63) / 64), static_cast<unsigned>(ktiles));
-    if (planes_t && nterms == 2)
-      GB_LAUNCH(kind, s, (split_rc_tile_kernel<2, true><<<grid, 256, 0, s>>>(X, R, Kd, ks, planes, pitch, planes_t,
-                                                                               pitch_t)));
-    else if (planes_t)
-      GB_LAUNCH(kind, s, (split_rc_tile_kernel<3, true><<<grid, 256, 0, s>>>(X, R, Kd, ks, planes, pitch, planes_t,
-                                                                               pitch_t)));
-    else if (nterms == 2)
-      GB_LAUNCH(kind, s, (split_rc_tile_kernel<2, false><<<grid, 256, 0, s>>>(X, R, Kd, ks, planes, pitch, nullptr,
-                                                                                0)));
-    else
-      GB_LAUNCH(kind, s, (split_rc_tile_kernel<3, false><<<grid, 256, 0, s>>>(X, R, Kd, ks, planes, pitch, nullptr,
-                                                                                0)));
-  } else {
-    const int64_t kchunks = (Kd + 15) / 16;
-    const int64_t plane = R * pitch;
-    for (int64_t r0 = 0; r0 < R; r0 += 65535) {   // rows beyond the grid's y range: bands
-      const int64_t rb = (R - r0 < 65535) ? R - r0 : 65535;
-      dim3 grid(static_cast<unsigned>((kchunks + 255) / 256), static_cast<unsigned>(rb));
-      if (nterms == 2)
-        GB_LAUNCH(kind, s, (split_kc_kernel<2><<<grid, 256, 0, s>>>(X + r0 * rs, rb, Kd, rs, ks, planes + r0 * pitch,
-                                                                    pitch, plane)));
-      else
-        GB_LAUNCH(kind, s, (split_kc_kernel<3><<<grid, 256, 0, s>>>(X + r0 * rs, rb, Kd, rs, ks, planes + r0 * pitch,
-                                                                    pitch, plane)));
+template <int NT>
+__global__ void __launch_bounds__(256) split_terms_kernel(const __grid_constant__ SplitParts parts) {
+  __shared__ float tile[64][65];   // [k][r]
+  int i = 0;
+#pragma unroll
+  for (int q = 1; q < SPLIT_MAX_OPERANDS; ++q)
+    if (blockIdx.x >= parts.part[q].first) i = q;
+  const SplitPart& p = parts.part[i];
+  const uint32_t block = blockIdx.x - p.first;
+  if (p.tile) split_tile<NT>(p, block, tile);
+  else split_chunks<NT>(p, block);
+}
+
+int split_bf16_terms(const SplitOperand* ops, int count, int nterms, int kind, cudaStream_t s) {
+  if ((nterms != 2 && nterms != 3) || count < 0 || count > SPLIT_MAX_OPERANDS) return GB_ERR_INVALID_VALUE;
+  SplitParts parts;
+  std::memset(&parts, 0, sizeof(parts));
+  int64_t blocks = 0;
+  for (int i = 0; i < SPLIT_MAX_OPERANDS; ++i) {
+    SplitPart& p = parts.part[i];
+    p.first = static_cast<uint32_t>(blocks);
+    p.gx = 1;
+    if (i >= count || ops[i].R <= 0 || ops[i].K <= 0) {
+      // no blocks; one past the last is never reached, and an empty operand before a full one
+      // starts where that one does
+      continue;
     }
+    const SplitOperand& o = ops[i];
+    p.op = o;
+    if (o.planes_t && o.rs != 1) return GB_ERR_UNSUPPORTED;   // the transposed layout is written from row-contiguous X
+    int64_t n;
+    if (o.rs == 1) {
+      const int64_t ktiles = (o.K + 63) / 64, rtiles = (o.R + 63) / 64;
+      if (ktiles > 65535 || rtiles > 0x7FFFFFFF) return GB_ERR_UNSUPPORTED;
+      p.tile = 1;
+      p.gx = static_cast<uint32_t>(rtiles);
+      n = rtiles * ktiles;
+    } else {
+      const int64_t chunks = (o.K + 7) / 8;
+      while (p.log_tpr < 8 && (1 << p.log_tpr) < chunks) ++p.log_tpr;
+      const int64_t gx = (chunks + (1 << p.log_tpr) - 1) >> p.log_tpr, rows = 256 >> p.log_tpr;
+      p.gx = static_cast<uint32_t>(gx);
+      n = gx * ((o.R + rows - 1) / rows);
+    }
+    blocks += n;
+    if (blocks > 0x7FFFFFFF) return GB_ERR_UNSUPPORTED;
   }
+  if (blocks == 0) return GB_OK;
+  const unsigned grid = static_cast<unsigned>(blocks);
+  if (nterms == 2)
+    GB_LAUNCH(kind, s, split_terms_kernel<2><<<grid, 256, 0, s>>>(parts));
+  else
+    GB_LAUNCH(kind, s, split_terms_kernel<3><<<grid, 256, 0, s>>>(parts));
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
 }
@@ -247,12 +250,11 @@ int adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, co
   w += al256(2 * static_cast<size_t>(K) * pM * 2);
   __nv_bfloat16* P4 = reinterpret_cast<__nv_bfloat16*>(w);                      // dC [p][j][i]
 
-  // dC (M x N, column-major): rows i contiguous -> [p][i][j] and, from the same read, [p][j][i]
-  int rc = split_bf16_terms(dC, M, N, 1, lddc, 2, P1, pN, P4, pM, GB_KERNEL_ADJOINT_SPLIT, s);
-  // B (K x N): rows k contiguous -> [p][k][j]
-  if (!rc) rc = split_bf16_terms(B, K, N, 1, ldb, 2, P2, pN, nullptr, 0, GB_KERNEL_ADJOINT_SPLIT, s);
-  // A^T rows k (contraction over i, contiguous in memory) -> [p][k][i]
-  if (!rc) rc = split_bf16_terms(A, K, M, lda, 1, 2, P3, pM, nullptr, 0, GB_KERNEL_ADJOINT_SPLIT, s);
+  const SplitOperand ops[3] = {
+      {dC, M, N, 1, lddc, P1, pN, P4, pM},        // column-major, rows i contiguous: [p][i][j] and [p][j][i]
+      {B, K, N, 1, ldb, P2, pN, nullptr, 0},      // rows k contiguous: [p][k][j]
+      {A, K, M, lda, 1, P3, pM, nullptr, 0}};     // A^T, rows k, contraction over i contiguous: [p][k][i]
+  int rc = split_bf16_terms(ops, 3, 2, GB_KERNEL_ADJOINT_SPLIT, s);
   if (rc) return rc;
 
   CUtensorMap ta0, tb0, ta1, tb1;

@@ -21,13 +21,10 @@
 
 #include "gb_common.cuh"
 #include "profile.cuh"
+#include "split_terms.cuh"
 #include "tc_gemm.cuh"
 
 namespace gb {
-
-int split_bf16_terms(const float* X, int64_t R, int64_t Kd, int64_t rs, int64_t ks, int nterms,
-                     __nv_bfloat16* planes, int64_t pitch, __nv_bfloat16* planes_t, int64_t pitch_t, int kind,
-                     cudaStream_t s);
 
 static inline int64_t pitch64_of(int64_t k) { return ((k + 63) / 64) * 64; }
 static inline size_t align_256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -62,9 +59,9 @@ int gemm_f32_tc(int ta, int tb, int64_t M, int64_t N, int64_t K, float alpha, co
   __nv_bfloat16* PB = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(ws) +
                                                        align_256(static_cast<size_t>(nterms) * M * pk * 2));
   // op(A)[i, k] = ta ? A[k + i lda] : A[i + k lda];  op(B)[k, j] = tb ? B[j + k ldb] : B[k + j ldb]
-  int rc = split_bf16_terms(A, M, K, ta ? lda : 1, ta ? 1 : lda, nterms, PA, pk, nullptr, 0, GB_KERNEL_F32_SPLIT, s);
-  if (!rc)
-    rc = split_bf16_terms(B, N, K, tb ? 1 : ldb, tb ? ldb : 1, nterms, PB, pk, nullptr, 0, GB_KERNEL_F32_SPLIT, s);
+  const SplitOperand ops[2] = {{A, M, K, ta ? lda : 1, ta ? 1 : lda, PA, pk, nullptr, 0},
+                               {B, N, K, tb ? 1 : ldb, tb ? ldb : 1, PB, pk, nullptr, 0}};
+  int rc = split_bf16_terms(ops, 2, nterms, GB_KERNEL_F32_SPLIT, s);
   if (rc) return rc;
   const TcTuning tune = tc_tuning_for(TC_KIND_F32, M, N);
   const bool pair = tune.engine == 2;
