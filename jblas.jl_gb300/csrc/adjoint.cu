@@ -41,10 +41,11 @@ __device__ __forceinline__ void split_terms(float x, uint32_t (&t)[NT]) {
 // 4 bytes read and 2 NT written an element.  An operand alone is 8 to 15 us of a mid-size product, much
 // of it the launch and the last wave.
 //   chunks   (element (r, k) at X[r rs + k ks], any strides): a thread takes 8 consecutive k of a
-//            row, a 16-byte store per plane; tpr = 2^log_tpr threads along k (as many as a row has
-//            chunks, at most 256), the other 256 / tpr along rows.  With ks == 1 and an aligned row
-//            the 8 values are two 16-byte loads; an unaligned row costs a warp 8 lines per load (16 k
-//            a thread: 16 lines, and a row to a block left half the threads of 2047 k idle).
+//            row, a 16-byte store per plane, or 16 where k is contiguous and every row aligned (four
+//            16-byte loads; 8 there: 190 us instead of 185 for a product whose split is 40); tpr =
+//            2^log_tpr threads along k (as many as a row has chunks, at most 256), the other
+//            256 / tpr along rows.  An unaligned row costs a warp 8 lines per load, 16 with 16 k a
+//            thread, and a row to a block left half the threads of 2047 k idle.
 //   tile     (rows contiguous): a 64 x 64 tile through shared memory.  Warp w loads columns
 //            8w..8w+7 (lanes along r: 128-byte loads); a thread then splits 16 k of one row and
 //            stores 32 bytes of every plane, and for the transposed planes 16 rows of one k (whole
@@ -56,9 +57,12 @@ struct SplitPart {
   uint32_t first;   // first block
   uint32_t gx;      // chunks: blocks along k; tile: blocks along the rows
   int32_t log_tpr, tile;
+  int32_t wide;     // chunks of 16
 };
 struct SplitParts {
   SplitPart part[SPLIT_MAX_OPERANDS];
+  unsigned int* zero;   // written by block 0
+  int32_t nzero;
 };
 
 // N consecutive values -> 2 N bytes of each of NT planes at dst + i plane (the first nvalid of them).
@@ -94,20 +98,20 @@ __device__ __forceinline__ void store_terms(const float (&x)[N], __nv_bfloat16* 
   }
 }
 
-template <int NT>
+template <int NT, int N>
 __device__ __forceinline__ void split_chunks(const SplitPart& p, uint32_t block) {
   const SplitOperand& o = p.op;
   const uint32_t by = block / p.gx, bx = block - by * p.gx;
   const int lt = p.log_tpr;
   const int64_t r = (static_cast<int64_t>(by) << (8 - lt)) + (threadIdx.x >> lt);
-  const int64_t k0 = ((static_cast<int64_t>(bx) << lt) + (threadIdx.x & ((1 << lt) - 1))) * 8;
+  const int64_t k0 = ((static_cast<int64_t>(bx) << lt) + (threadIdx.x & ((1 << lt) - 1))) * N;
   if (r >= o.R || k0 >= o.K) return;
-  const int nvalid = static_cast<int>(o.K - k0 < 8 ? o.K - k0 : 8);
+  const int nvalid = static_cast<int>(o.K - k0 < N ? o.K - k0 : N);
   const float* __restrict__ src = o.X + r * o.rs + k0 * o.ks;
-  float x[8];
-  if (o.ks == 1 && nvalid == 8 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+  float x[N];
+  if (o.ks == 1 && nvalid == N && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
+    for (int q = 0; q < N / 4; ++q) {
       const float4 v = reinterpret_cast<const float4*>(src)[q];
       x[4 * q] = v.x;
       x[4 * q + 1] = v.y;
@@ -116,7 +120,7 @@ __device__ __forceinline__ void split_chunks(const SplitPart& p, uint32_t block)
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = (j < nvalid) ? src[j * o.ks] : 0.0f;
+    for (int j = 0; j < N; ++j) x[j] = (j < nvalid) ? src[j * o.ks] : 0.0f;
   }
   store_terms<NT>(x, o.planes + r * o.pitch + k0, o.R * o.pitch, nvalid);
 }
@@ -159,6 +163,8 @@ __device__ __forceinline__ void split_tile(const SplitPart& p, uint32_t block, f
 template <int NT>
 __global__ void __launch_bounds__(256) split_terms_kernel(const __grid_constant__ SplitParts parts) {
   __shared__ float tile[64][65];   // [k][r]
+  if (blockIdx.x == 0)
+    for (int z = threadIdx.x; z < parts.nzero; z += 256) parts.zero[z] = 0;
   int i = 0;
 #pragma unroll
   for (int q = 1; q < SPLIT_MAX_OPERANDS; ++q)
@@ -166,13 +172,17 @@ __global__ void __launch_bounds__(256) split_terms_kernel(const __grid_constant_
   const SplitPart& p = parts.part[i];
   const uint32_t block = blockIdx.x - p.first;
   if (p.tile) split_tile<NT>(p, block, tile);
-  else split_chunks<NT>(p, block);
+  else if (p.wide) split_chunks<NT, 16>(p, block);
+  else split_chunks<NT, 8>(p, block);
 }
 
-int split_bf16_terms(const SplitOperand* ops, int count, int nterms, int kind, cudaStream_t s) {
+int split_bf16_terms(const SplitOperand* ops, int count, int nterms, unsigned int* zero, int nzero, int kind,
+                     cudaStream_t s) {
   if ((nterms != 2 && nterms != 3) || count < 0 || count > SPLIT_MAX_OPERANDS) return GB_ERR_INVALID_VALUE;
   SplitParts parts;
   std::memset(&parts, 0, sizeof(parts));
+  parts.zero = zero;
+  parts.nzero = nzero;
   int64_t blocks = 0;
   for (int i = 0; i < SPLIT_MAX_OPERANDS; ++i) {
     SplitPart& p = parts.part[i];
@@ -194,7 +204,8 @@ int split_bf16_terms(const SplitOperand* ops, int count, int nterms, int kind, c
       p.gx = static_cast<uint32_t>(rtiles);
       n = rtiles * ktiles;
     } else {
-      const int64_t chunks = (o.K + 7) / 8;
+      p.wide = o.ks == 1 && (o.rs & 3) == 0 && (reinterpret_cast<uintptr_t>(o.X) & 15) == 0;
+      const int64_t each = p.wide ? 16 : 8, chunks = (o.K + each - 1) / each;
       while (p.log_tpr < 8 && (1 << p.log_tpr) < chunks) ++p.log_tpr;
       const int64_t gx = (chunks + (1 << p.log_tpr) - 1) >> p.log_tpr, rows = 256 >> p.log_tpr;
       p.gx = static_cast<uint32_t>(gx);
@@ -231,14 +242,21 @@ static void split3_schedule(SliceSchedule& S, int kb_chunk) {
 }
 
 // Workspace layout for an adjoint of A (M x K), B (K x N), dC (M x N).
-size_t adjoint_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+static TcSplit adjoint_split(int64_t M, int64_t N, int64_t K, int sms) {
+  auto t = [](int64_t x) { return (x + 255) / 256; };
+  return tc_split_plan({t(M) * t(K), t(K) * t(N)}, {(N + TC_BK - 1) / TC_BK, (M + TC_BK - 1) / TC_BK}, 3, sms / 2);
+}
+
+size_t adjoint_workspace_bytes(int64_t M, int64_t N, int64_t K, int sms, bool split) {
   const int64_t pN = pitch64(N), pM = pitch64(M);
+  const TcSplit sp = split ? adjoint_split(M, N, K, sms) : TcSplit();
   return al256(2 * static_cast<size_t>(M) * pN * 2) + al256(2 * static_cast<size_t>(K) * pN * 2) +
-         al256(2 * static_cast<size_t>(K) * pM * 2) + al256(2 * static_cast<size_t>(N) * pM * 2);
+         al256(2 * static_cast<size_t>(K) * pM * 2) + al256(2 * static_cast<size_t>(N) * pM * 2) + sp.ws_bytes +
+         sp.counters * sizeof(unsigned int);
 }
 
 int adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B, int64_t ldb,
-                const float* dC, int64_t lddc, float* dA, int64_t ldda, float* dB, int64_t lddb, void* ws,
+                const float* dC, int64_t lddc, float* dA, int64_t ldda, float* dB, int64_t lddb, void* ws, bool split,
                 int sms, DeviceStatus* status, uint64_t wait_limit_ns, cudaStream_t s) {
   const int64_t pN = pitch64(N), pM = pitch64(M);
   char* w = static_cast<char*>(ws);
@@ -254,7 +272,13 @@ int adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, co
       {dC, M, N, 1, lddc, P1, pN, P4, pM},        // column-major, rows i contiguous: [p][i][j] and [p][j][i]
       {B, K, N, 1, ldb, P2, pN, nullptr, 0},      // rows k contiguous: [p][k][j]
       {A, K, M, lda, 1, P3, pM, nullptr, 0}};     // A^T, rows k, contraction over i contiguous: [p][k][i]
-  int rc = split_bf16_terms(ops, 3, 2, GB_KERNEL_ADJOINT_SPLIT, s);
+  w += al256(2 * static_cast<size_t>(N) * pM * 2);
+  const int64_t big = M > N ? (M > K ? M : K) : (N > K ? N : K);
+  const TcTuning tune = tc_tuning_for(TC_KIND_ADJOINT, big, big);
+  const bool pair = tune.engine == 2;
+  const TcSplit sp = pair && split ? adjoint_split(M, N, K, sms) : TcSplit();
+  unsigned int* counters = reinterpret_cast<unsigned int*>(w + sp.ws_bytes);
+  int rc = split_bf16_terms(ops, 3, 2, counters, sp.counters, GB_KERNEL_ADJOINT_SPLIT, s);
   if (rc) return rc;
 
   CUtensorMap ta0, tb0, ta1, tb1;
@@ -264,13 +288,10 @@ int adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, co
   if (!rc) rc = make_plane_tmap(&tb1, P4, M, N, 2, pM, TC_BN);
   if (rc) return rc;
 
-  const int64_t big = M > N ? (M > K ? M : K) : (N > K ? N : K);
-  const TcTuning tune = tc_tuning_for(TC_KIND_ADJOINT, big, big);
-  const bool pair = tune.engine == 2;
   const int64_t tbm = pair ? 256 : TC_BM, tbn = pair ? 256 : TC_BN;
   TcParams prm;
   std::memset(&prm, 0, sizeof(prm));
-  prm.band = tune.band;
+  prm.band = sp.parts ? TC_SPLIT_BAND : tune.band;
   TcProblem& P = prm.prob[0];   // dA (M x K), contraction N
   P.M = M; P.N = K; P.K = N;
   P.tiles_m = static_cast<int32_t>((M + tbm - 1) / tbm);
@@ -305,8 +326,13 @@ int adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, co
     prm.c_tma = (tune.tma_store && make_c_tmap_f32(&tc0, dA, M, K, ldda) && make_c_tmap_f32(&tc1, dB, K, N, lddb))
                     ? 1 : 0;
     const int64_t ctas = 2 * static_cast<int64_t>(prm.total_tiles), cap = sms & ~1;
+    prm.split_first = sp.first;
+    prm.split_parts = sp.parts;
+    prm.split_ws = reinterpret_cast<float*>(w);
+    prm.split_count = counters;
     return tc_gemm_pair_launch(TC_EPI_F32, ta0, tb0h, &ta1, &tb1h, sched, prm,
-                               static_cast<int>(ctas < cap ? ctas : cap), GB_KERNEL_ADJOINT_MMA, s,
+                               sp.parts ? 2 * sp.clusters : static_cast<int>(ctas < cap ? ctas : cap),
+                               GB_KERNEL_ADJOINT_MMA, s,
                                prm.c_tma ? &tc0 : nullptr, prm.c_tma ? &tc1 : nullptr);
   }
   const int grid = prm.total_tiles < sms ? prm.total_tiles : sms;

@@ -27,14 +27,14 @@
 namespace gb {
 int measure_fma_peaks(int sms, double* fp64_tflops, double* fp32_tflops);
 int tc_autotune(int kind, int64_t M, int64_t N, int64_t K, int reps, TcTuning* out, float* best_ms, cudaStream_t s);
-size_t gemm_f32_tc_workspace_bytes(int64_t M, int64_t N, int64_t K, int nterms);
+size_t gemm_f32_tc_workspace_bytes(int64_t M, int64_t N, int64_t K, int nterms, int sms, bool split);
 int gemm_f32_tc(int ta, int tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A, int64_t lda,
-                const float* B, int64_t ldb, float beta, float* C, int64_t ldc, int nterms, void* ws, int sms,
-                DeviceStatus* status, uint64_t wait_limit_ns, cudaStream_t s);
-size_t adjoint_workspace_bytes(int64_t M, int64_t N, int64_t K);
+                const float* B, int64_t ldb, float beta, float* C, int64_t ldc, int nterms, void* ws, bool split,
+                int sms, DeviceStatus* status, uint64_t wait_limit_ns, cudaStream_t s);
+size_t adjoint_workspace_bytes(int64_t M, int64_t N, int64_t K, int sms, bool split);
 int adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B, int64_t ldb,
                 const float* dC, int64_t lddc, float* dA, int64_t ldda, float* dB, int64_t lddb, void* ws,
-                int sms, DeviceStatus* status, uint64_t wait_limit_ns, cudaStream_t s);
+                bool split, int sms, DeviceStatus* status, uint64_t wait_limit_ns, cudaStream_t s);
 }  // namespace gb
 
 static thread_local char g_last_detail[256];
@@ -1191,8 +1191,13 @@ int gb_gemm_f32_ex(int transA, int transB, int64_t M, int64_t N, int64_t K, floa
   if (tc_pair_tiles(M, N) > 0x7FFFFFFF / 2 || tc_tiles(M, N) > 0x7FFFFFFF / 2) return GB_ERR_UNSUPPORTED;
   const int nterms = (mode == GB_MODE_BF16X3) ? 2 : 3;
   void* ws = nullptr;
-  GB_CUDA_TRY(cudaMallocFromPoolAsync(&ws, gemm_f32_tc_workspace_bytes(M, N, K, nterms), dev->pool, s));
-  rc = gemm_f32_tc(transA, transB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, nterms, ws, dev->sms, dev->status,
+  bool split = true;   // without room for the partial sums no tile is cut
+  if (cudaMallocFromPoolAsync(&ws, gemm_f32_tc_workspace_bytes(M, N, K, nterms, dev->sms, true), dev->pool, s) != cudaSuccess) {
+    cudaGetLastError();
+    split = false;
+    GB_CUDA_TRY(cudaMallocFromPoolAsync(&ws, gemm_f32_tc_workspace_bytes(M, N, K, nterms, dev->sms, false), dev->pool, s));
+  }
+  rc = gemm_f32_tc(transA, transB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, nterms, ws, split, dev->sms, dev->status,
                    g_wait_limit_ns.load(), s);
   cudaFreeAsync(ws, s);
   return rc;
@@ -1246,8 +1251,13 @@ int gb_gemm_adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t
   if (!is_device_ptr(A) || !is_device_ptr(B) || !is_device_ptr(dC)) return GB_ERR_INVALID_VALUE;
   if (static_cast<int64_t>(tc_tiles(M, K)) + tc_tiles(K, N) > 0x7FFFFFFF) return GB_ERR_UNSUPPORTED;
   void* ws = nullptr;
-  GB_CUDA_TRY(cudaMallocFromPoolAsync(&ws, adjoint_workspace_bytes(M, N, K), dev->pool, s));
-  rc = adjoint_f32(M, N, K, A, lda, B, ldb, dC, lddc, dA, ldda, dB, lddb, ws, dev->sms, dev->status,
+  bool split = true;
+  if (cudaMallocFromPoolAsync(&ws, adjoint_workspace_bytes(M, N, K, dev->sms, true), dev->pool, s) != cudaSuccess) {
+    cudaGetLastError();
+    split = false;
+    GB_CUDA_TRY(cudaMallocFromPoolAsync(&ws, adjoint_workspace_bytes(M, N, K, dev->sms, false), dev->pool, s));
+  }
+  rc = adjoint_f32(M, N, K, A, lda, B, ldb, dC, lddc, dA, ldda, dB, lddb, ws, split, dev->sms, dev->status,
                    g_wait_limit_ns.load(), s);
   cudaFreeAsync(ws, s);
   return rc;

@@ -29,9 +29,16 @@ namespace gb {
 static inline int64_t pitch64_of(int64_t k) { return ((k + 63) / 64) * 64; }
 static inline size_t align_256(size_t x) { return (x + 255) & ~size_t(255); }
 
-size_t gemm_f32_tc_workspace_bytes(int64_t M, int64_t N, int64_t K, int nterms) {
+static TcSplit term_split(int64_t M, int64_t N, int64_t K, int nterms, int sms) {
+  const int64_t tiles = (M + 255) / 256 * ((N + 255) / 256);
+  return tc_split_plan({tiles, 0}, {(K + TC_BK - 1) / TC_BK, 0}, nterms * (nterms + 1) / 2, sms / 2);
+}
+
+size_t gemm_f32_tc_workspace_bytes(int64_t M, int64_t N, int64_t K, int nterms, int sms, bool split) {
   const size_t pk = static_cast<size_t>(pitch64_of(K));
-  return align_256(static_cast<size_t>(nterms) * M * pk * 2) + align_256(static_cast<size_t>(nterms) * N * pk * 2);
+  const TcSplit sp = split ? term_split(M, N, K, nterms, sms) : TcSplit();
+  return align_256(static_cast<size_t>(nterms) * M * pk * 2) + align_256(static_cast<size_t>(nterms) * N * pk * 2) +
+         sp.ws_bytes + sp.counters * sizeof(unsigned int);
 }
 
 // One group holding the kept term pairs, smallest contributions first.
@@ -52,7 +59,7 @@ static void term_schedule(SliceSchedule& S, int nterms, int kb_chunk) {
 }
 
 int gemm_f32_tc(int ta, int tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A, int64_t lda,
-                const float* B, int64_t ldb, float beta, float* C, int64_t ldc, int nterms, void* ws, int sms,
+                const float* B, int64_t ldb, float beta, float* C, int64_t ldc, int nterms, void* ws, bool split, int sms,
                 DeviceStatus* status, uint64_t wait_limit_ns, cudaStream_t s) {
   const int64_t pk = pitch64_of(K);
   __nv_bfloat16* PA = static_cast<__nv_bfloat16*>(ws);
@@ -61,10 +68,13 @@ int gemm_f32_tc(int ta, int tb, int64_t M, int64_t N, int64_t K, float alpha, co
   // op(A)[i, k] = ta ? A[k + i lda] : A[i + k lda];  op(B)[k, j] = tb ? B[j + k ldb] : B[k + j ldb]
   const SplitOperand ops[2] = {{A, M, K, ta ? lda : 1, ta ? 1 : lda, PA, pk, nullptr, 0},
                                {B, N, K, tb ? 1 : ldb, tb ? ldb : 1, PB, pk, nullptr, 0}};
-  int rc = split_bf16_terms(ops, 2, nterms, GB_KERNEL_F32_SPLIT, s);
-  if (rc) return rc;
   const TcTuning tune = tc_tuning_for(TC_KIND_F32, M, N);
   const bool pair = tune.engine == 2;
+  const TcSplit sp = pair && split ? term_split(M, N, K, nterms, sms) : TcSplit();
+  float* parts = reinterpret_cast<float*>(reinterpret_cast<char*>(PB) + align_256(static_cast<size_t>(nterms) * N * pk * 2));
+  unsigned int* counters = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(parts) + sp.ws_bytes);
+  int rc = split_bf16_terms(ops, 2, nterms, counters, sp.counters, GB_KERNEL_F32_SPLIT, s);
+  if (rc) return rc;
   CUtensorMap tmap_a, tmap_b;
   rc = make_plane_tmap(&tmap_a, PA, K, M, nterms, pk, TC_BM);
   if (!rc) rc = make_plane_tmap(&tmap_b, PB, K, N, nterms, pk, pair ? 128 : TC_BN);
@@ -72,7 +82,11 @@ int gemm_f32_tc(int ta, int tb, int64_t M, int64_t N, int64_t K, float alpha, co
   const int64_t tbm = pair ? 256 : TC_BM, tbn = pair ? 256 : TC_BN;
   TcParams prm;
   std::memset(&prm, 0, sizeof(prm));
-  prm.band = tune.band;
+  prm.band = sp.parts ? TC_SPLIT_BAND : tune.band;
+  prm.split_first = sp.first;
+  prm.split_parts = sp.parts;
+  prm.split_ws = parts;
+  prm.split_count = counters;
   TcProblem& P = prm.prob[0];
   P.M = M;
   P.N = N;
@@ -97,7 +111,7 @@ int gemm_f32_tc(int ta, int tb, int64_t M, int64_t N, int64_t K, float alpha, co
     prm.c_tma = (tune.tma_store && beta == 0.0f && make_c_tmap_f32(&tmap_c, C, M, N, ldc)) ? 1 : 0;
     const int64_t ctas = 2 * static_cast<int64_t>(prm.total_tiles), cap = sms & ~1;
     return tc_gemm_pair_launch(TC_EPI_F32, tmap_a, tmap_b, nullptr, nullptr, sched, prm,
-                               static_cast<int>(ctas < cap ? ctas : cap), GB_KERNEL_F32_MMA, s,
+                               sp.parts ? 2 * sp.clusters : static_cast<int>(ctas < cap ? ctas : cap), GB_KERNEL_F32_MMA, s,
                                prm.c_tma ? &tmap_c : nullptr, nullptr);
   }
   const int grid = prm.total_tiles < sms ? prm.total_tiles : sms;

@@ -18,7 +18,9 @@ struct SplitOperand {
 };
 constexpr int SPLIT_MAX_OPERANDS = 3;
 
-// Splits up to SPLIT_MAX_OPERANDS operands into nterms = 2 or 3 terms each in one launch, counted as `kind`.
-int split_bf16_terms(const SplitOperand* ops, int count, int nterms, int kind, cudaStream_t s);
+// Splits up to SPLIT_MAX_OPERANDS operands into nterms = 2 or 3 terms each in one launch, counted as
+// `kind`, which also writes zeros to zero[0 .. nzero - 1].
+int split_bf16_terms(const SplitOperand* ops, int count, int nterms, unsigned int* zero, int nzero, int kind,
+                     cudaStream_t s);
 
 }  // namespace gb

@@ -75,7 +75,27 @@ struct TcParams {
   float crt_psi[TC_MAX_MODULI][TC_MAX_MODULI];   // [n - 1][g]: multiplier of the final residue
   int32_t band;         // output-tile rows per band of the tile raster (L2 reuse of the A rows)
   int32_t c_tma;        // TC_EPI_F32: 1 = C written by TMA stores from shared memory (beta = 0)
+  // TC_EPI_F32, CTA pairs, when split_parts > 0: the tiles from split_first on are cut along K (TcSplit)
+  int32_t split_first;
+  int32_t split_parts;
+  float* split_ws;
+  unsigned int* split_count;
 };
+
+// How a launch of FP32 outputs on CTA pairs cuts its last tiles along K (tc_split_plan): `parts` pairs to
+// a tile, each with all term pairs of an equal share of its K panels.
+struct TcSplit {
+  int clusters = 0;          // CTA pairs to launch, when parts > 0
+  int first = 0;             // tiles before it are whole, dealt round robin
+  int parts = 0;             // 0: no tile is cut
+  size_t ws_bytes = 0;       // partial sums, and
+  int counters = 0;          // counters (zero on entry)
+};
+// tiles[p] tiles of panels[p] K panels each for one or two problems (tiles[1] = 0: one), `terms` term pairs,
+// `pairs` CTA pairs.
+TcSplit tc_split_plan(const int64_t (&tiles)[2], const int64_t (&panels)[2], int terms, int pairs);
+constexpr int TC_SPLIT_BAND = 8;   // the tile raster's band in a split launch (which tiles are cut is a
+                                   // matter of their order, and results do not depend on the tuning)
 
 // ---------------------------------------------------------------- tuning (pick_kernel_size)
 // Launch configuration of the engine per kind of product and output-size class, the

@@ -88,6 +88,72 @@ __device__ __forceinline__ int p2_problem_of(const TcParams& prm, int t) {
   return (prm.nprob == 2 && t >= prm.prob[1].tile_begin) ? 1 : 0;
 }
 
+// TC_EPI_F32: what a CTA pair works on in turn: its whole tiles, then its share of a cut tile, all term
+// pairs of K panels [begin, end) (TcSplit).
+struct P2Work {
+  int t, begin, end;         // tile, K panels of it
+  int part;                  // which part of a cut tile (the order of the sum), -1: whole
+  int next_tile, step;       // whole tiles
+  int first, cuts;           // first cut tile, number of them
+  int tile1;                 // first tile of problem 1
+  int parts, len0, len1;     // parts of a cut tile; K panels
+  int mine;                  // this pair's part of all the cut tiles', -1: none (any more)
+
+  __device__ __forceinline__ P2Work(const TcParams& prm, int cluster, int nclusters) {
+    len0 = prm.prob[0].kb_total;
+    len1 = prm.nprob == 2 ? prm.prob[1].kb_total : len0;
+    tile1 = prm.nprob == 2 ? prm.prob[1].tile_begin : prm.total_tiles;
+    parts = prm.split_parts;
+    first = parts ? prm.split_first : prm.total_tiles;
+    cuts = prm.total_tiles - first;
+    next_tile = cluster;
+    step = nclusters;
+    mine = cluster < parts * cuts ? cluster : -1;
+  }
+  __device__ __forceinline__ bool next() {
+    begin = 0;
+    if (next_tile < first) {
+      t = next_tile;
+      end = t < tile1 ? len0 : len1;
+      part = -1;
+      next_tile += step;
+      return true;
+    }
+    if (mine < 0) return false;
+    part = mine / cuts;   // pairs side by side take the same panels of neighbouring tiles
+    t = first + mine - part * cuts;
+    mine = -1;
+    const int len = t < tile1 ? len0 : len1;
+    begin = len * part / parts;
+    end = len * (part + 1) / parts;
+    return true;
+  }
+};
+
+// The units of a CTA pair in turn: tile t, groups [g0, g1) of it and, for FP32 outputs, a part of its panels.
+template <int EPI>
+struct P2Units {
+  int t, g0, g1, u, step, ntiles, G;
+  __device__ __forceinline__ P2Units(const TcParams& prm, int groups, int cluster, int nclusters)
+      : u(cluster), step(nclusters), ntiles(prm.total_tiles), G(groups) {}
+  __device__ __forceinline__ bool next() {
+    if (u >= (EPI == TC_EPI_CRT ? ntiles * G : ntiles)) return false;
+    p2_unit<EPI>(u, ntiles, G, t, g0, g1);
+    u += step;
+    return true;
+  }
+  static __device__ __forceinline__ int first_kb(int kb0) { return kb0; }
+  static __device__ __forceinline__ int last_kb(int kb1) { return kb1; }
+};
+template <>
+struct P2Units<TC_EPI_F32> : P2Work {
+  static constexpr int g0 = 0, g1 = 1;
+  __device__ __forceinline__ P2Units(const TcParams& prm, int, int cluster, int nclusters)
+      : P2Work(prm, cluster, nclusters) {}
+  __device__ __forceinline__ int first_kb(int) const { return begin; }
+  __device__ __forceinline__ int last_kb(int) const { return end; }
+};
+
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREADS, 1)
     tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_b0,
@@ -151,9 +217,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
       int issued_parity[P2_STAGES];
       for (int i = 0; i < P2_STAGES; ++i) issued_parity[i] = -1;
       bool ok = true;
-      for (int u = cluster; u < nunits && ok; u += nclusters) {
-        int t, g0, g1;
-        p2_unit<EPI>(u, ntiles, G, t, g0, g1);
+      P2Units<EPI> un(prm, G, cluster, nclusters);
+      while (ok && un.next()) {
+        const int t = un.t, g0 = un.g0, g1 = un.g1;
         const int pr = p2_problem_of(prm, t);
         const TcProblem& P = prm.prob[pr];
         const CUtensorMap* ta = pr ? &tmap_a1 : &tmap_a0;
@@ -169,7 +235,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
             for (int i = 0; i < sched.npairs[g] && ok; ++i) {
               const int pa = sched.pp[sched.pair_off[g] + i];
               const int pb = sched.pq[sched.pair_off[g] + i];
-              for (int kb = kb0; kb < kb1; ++kb) {
+              for (int kb = un.first_kb(kb0); kb < un.last_kb(kb1); ++kb) {
                 if (!mbar_wait_bounded(&empty[stage], phase ^ 1, prm.wait_limit_ns, abort_flag, prm.status, 1)) {
                   ok = false;
                   break;
@@ -211,10 +277,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
       uint32_t acc_phase = 0;
       bool ok = true;
       bool issued_any = false;
-      for (int u = cluster; u < nunits && ok; u += nclusters) {
-        int t, g0, g1;
-        p2_unit<EPI>(u, ntiles, G, t, g0, g1);
-        const TcProblem& P = prm.prob[p2_problem_of(prm, t)];
+      P2Units<EPI> un(prm, G, cluster, nclusters);
+      while (ok && un.next()) {
+        const int g0 = un.g0, g1 = un.g1;
+        const TcProblem& P = prm.prob[p2_problem_of(prm, un.t)];
         for (int g = g0; g < g1 && ok; ++g) {
           for (int c = 0; c < P.nchunks && ok; ++c) {
             const int kb0 = c * sched.kb_chunk;
@@ -229,7 +295,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
             // stored back into this buffer
             uint32_t accumulate = (EPI == TC_EPI_CRT && c >= 2) ? 1u : 0u;
             for (int i = 0; i < sched.npairs[g] && ok; ++i) {
-              for (int kb = kb0; kb < kb1; ++kb) {
+              for (int kb = un.first_kb(kb0); kb < un.last_kb(kb1); ++kb) {
                 if (!mbar_wait_bounded(&full[stage], phase, prm.wait_limit_ns, abort_flag, prm.status, 3)) {
                   ok = false;
                   break;
@@ -272,6 +338,146 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
     int buf = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    if constexpr (EPI == TC_EPI_F32) {
+      P2Work wk(prm, cluster, nclusters);
+      while (ok && wk.next()) {
+        ok = __all_sync(0xffffffffu,
+                        mbar_wait_bounded(&tfull[buf], acc_phase, prm.wait_limit_ns, abort_flag, prm.status, 4));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * TC_BN);
+        const int pr = p2_problem_of(prm, wk.t);
+        const TcProblem& P = prm.prob[pr];
+        int tm, tn;
+        p2_tile_coords(wk.t - P.tile_begin, P.tiles_m, P.tiles_n, prm.band, tm, tn);
+        const int64_t row = static_cast<int64_t>(tm) * 256 + 128 * static_cast<int>(rank) + row_l;
+        const int64_t n0 = static_cast<int64_t>(tn) * 256;
+        const float fa = static_cast<float>(P.alpha), fb = static_cast<float>(P.beta);
+        // Per 32 columns: the warp that brings a tile's last part adds the parts up, in order, and stores
+        // C.  A part whose others are all there is added from TMEM, any other first goes to its slot of
+        // the workspace.  Pairs that finish together so share the sums among them.
+        constexpr size_t SLOT = TC_BM * TC_BN;   // floats of a CTA's part
+        constexpr int NB = COLS / 32;            // blocks of 32 columns
+        constexpr unsigned int ALL = (1u << NB) - 1u;
+        auto slot_of = [&](int part) {
+          return prm.split_ws + (static_cast<size_t>((wk.t - wk.first) * wk.parts + part) * 2 + rank) * SLOT + row_l;
+        };
+        const int parts = wk.part < 0 ? 1 : wk.parts;
+        unsigned int direct = ALL, summed = 0;   // blocks stored from TMEM, from the workspace
+        if (parts > 1) {
+          const unsigned int others = static_cast<unsigned int>(parts - 1);
+          unsigned int* arrived =
+              prm.split_count +
+              (((wk.t - wk.first) * 2 + static_cast<int>(rank)) * P2Shape<EPI>::EPI_WARPS + (warp - 2)) * NB + lane;
+          const bool there = lane < NB && *static_cast<volatile unsigned int*>(arrived) == others;
+          direct = __ballot_sync(0xffffffffu, there);
+          if (direct != ALL) {
+#pragma unroll 1
+            for (int b = 0; b < NB; ++b) {
+              if (direct >> b & 1u) continue;
+              uint32_t v[32];
+              tmem_ld_32x32b_x32(taddr + col0 + 32 * b, v);
+              tc_wait_ld();
+              float* to = slot_of(wk.part) + (col0 + 32 * b) * TC_BM;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) __stcg(to + j * TC_BM, __uint_as_float(v[j]));
+            }
+            if (direct == 0) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(tempty_leader0 + static_cast<uint32_t>(buf) * 8u);
+            }
+            __threadfence();   // this lane's part is written
+            __syncwarp();
+            const bool last = lane < NB && !there && atomicAdd(arrived, 1u) == others;
+            summed = __ballot_sync(0xffffffffu, last);
+          }
+          __threadfence();   // everyone's parts are visible
+        }
+        {
+#pragma unroll 1
+          for (int b = 0; b < NB; ++b) {
+            const bool in_tmem = direct >> b & 1u;
+            if (!in_tmem && !(summed >> b & 1u)) continue;
+            const int cb = col0 + 32 * b;
+            uint32_t v[32];
+            float x[32];
+            auto fetch = [&](int c, float (&f)[32]) {
+              const float* from = slot_of(c) + cb * TC_BM;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) f[j] = __ldcg(from + j * TC_BM);
+            };
+            int c = 0;
+            if (in_tmem) {
+              // x: the sum of the parts before the own one; the one after it when there is none
+              const bool lead = wk.part <= 0;
+              if (parts > 1) fetch(lead ? 1 : 0, x);
+              tmem_ld_32x32b_x32(taddr + cb, v);
+              tc_wait_ld();
+              if (parts > 1) {
+                for (c = 1; c < wk.part; ++c) {
+                  float y[32];
+                  fetch(c, y);
+#pragma unroll
+                  for (int j = 0; j < 32; ++j) x[j] += y[j];
+                }
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + x[j]);
+                c = lead ? 1 : wk.part;
+              }
+            } else {
+              fetch(0, x);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(x[j]);
+            }
+#pragma unroll 2
+            for (++c; c < parts; ++c) {
+              fetch(c, x);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + x[j]);
+            }
+            const int64_t colb = n0 + cb;
+            if (prm.c_tma && fb == 0.0f && row - lane + 32 <= P.M && colb + 32 <= P.N) {
+              // C through shared memory and a TMA store of the warp's 32 x 32 box; boxes that
+              // reach past C's last row or column take the direct stores below (measured: a
+              // store box that crosses the last row was not clipped at the row but at the next
+              // 16-byte boundary, writing rows of the caller's padding).  The box buffer is
+              // reused once the previous store of this warp has read it.
+              float* cbuf = reinterpret_cast<float*>(smem + P2_CSTAGE_OFF + (warp - 2) * 4096);
+              if (lane == 0) bulk_wait_read_all();
+              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < 32; ++j) cbuf[j * 32 + lane] = fa * __uint_as_float(v[j]);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                tma_store_2d(pr ? &tmap_c1 : &tmap_c0, cbuf, static_cast<int>(row - lane), static_cast<int>(colb));
+                bulk_commit_group();
+              }
+            } else if (row < P.M) {
+              float* __restrict__ crow = static_cast<float*>(P.C) + row + colb * P.ldc;
+              float c0[32];
+              if (fb != 0.0f) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) c0[j] = (colb + j < P.N) ? crow[j * P.ldc] : 0.0f;
+              }
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                if (colb + j >= P.N) continue;
+                const float sj = __uint_as_float(v[j]);
+                crow[j * P.ldc] = (fb == 0.0f) ? fa * sj : fmaf(fa, sj, fb * c0[j]);
+              }
+            }
+          }
+          if (direct) {   // the whole warp has drained its columns: one arrival on the leader's tmem_empty
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(tempty_leader0 + static_cast<uint32_t>(buf) * 8u);
+          }
+        }
+        if (++buf == 2) { buf = 0; acc_phase ^= 1; }
+      }
+    } else
     for (int u = cluster; u < nunits && ok; u += nclusters) {
       int t, g0, g1;
       p2_unit<EPI>(u, ntiles, G, t, g0, g1);
@@ -373,44 +579,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
             tmem_ld_32x32b_x32(taddr + cb, v);
             tc_wait_ld();
             const int64_t colb = n0 + cb;
-            if (EPI == TC_EPI_F32) {
-              if (prm.c_tma && beta == 0.0 && row - lane + 32 <= P.M && colb + 32 <= P.N) {
-                // C through shared memory and a TMA store of the warp's 32 x 32 box; boxes that
-                // reach past C's last row or column take the direct stores below (measured: a
-                // store box that crosses the last row was not clipped at the row but at the next
-                // 16-byte boundary, writing rows of the caller's padding).  The box buffer is
-                // reused once the previous store of this warp has read it.
-                float* cbuf = reinterpret_cast<float*>(smem + P2_CSTAGE_OFF + (warp - 2) * 4096);
-                const float fa = static_cast<float>(alpha);
-                if (lane == 0) bulk_wait_read_all();
-                __syncwarp();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) cbuf[j * 32 + lane] = fa * __uint_as_float(v[j]);
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                  tma_store_2d(pr ? &tmap_c1 : &tmap_c0, cbuf, static_cast<int>(row - lane), static_cast<int>(colb));
-                  bulk_commit_group();
-                }
-                continue;
-              }
-              if (row_ok) {
-                float* __restrict__ crow = static_cast<float*>(P.C) + row + colb * P.ldc;
-                const float fa = static_cast<float>(alpha), fb = static_cast<float>(beta);
-                float c0[32];
-                if (fb != 0.0f) {
-#pragma unroll
-                  for (int j = 0; j < 32; ++j) c0[j] = (colb + j < P.N) ? crow[j * P.ldc] : 0.0f;
-                }
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                  if (colb + j >= P.N) continue;
-                  const float sj = __uint_as_float(v[j]);
-                  crow[j * P.ldc] = (fb == 0.0f) ? fa * sj : fmaf(fa, sj, fb * c0[j]);
-                }
-              }
-              continue;
-            }
             double* __restrict__ tcol = tws + static_cast<int64_t>(cb) * TC_BM + row_l;
             double tv[32];
             if (!first) {
@@ -469,6 +637,48 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, P2_TMEM_COLS);
   }
+}
+
+// The tiles left after the full rounds of a launch (all of them when there are fewer than pairs) take
+// a round of their own, however few they are.  Cut along K they occupy more pairs for their share of it,
+// at the price of partial sums.  Costs in K panels of a full round (0.335 us, the tensor cores' power
+// or operand bandwidth): with fewer pairs at work a panel takes less, down to three quarters from 57
+// pairs on; writing and adding the parts 32, and 2 for each beyond the second (512^3 x6 in four
+// parts would be 38 us, whole it is 34).  A part runs all term pairs of its K panels, so no sum in
+// TMEM is longer than before.  Tiles on more than half
+// of the pairs stay whole: the gain there is below the cost (cut in equal ranges of panels, or with the
+// idle pairs taking over a share, 2048^3 x6 went 84 -> 95 us and 3001 x 2503 x 2047 146 -> 143).
+// x6: 1024^3 (16 tiles) 47 -> 41 us, 1600 x 3328 x 1312 (91) 101 -> 87, 4096^3 (256) 529 -> 491,
+// 500 x 500 x 20000 (4) 551 -> 131.
+TcSplit tc_split_plan(const int64_t (&tiles)[2], const int64_t (&panels)[2], int terms, int pairs) {
+  constexpr double LEAST = 0.75, SUM = 32.0, PART = 2.0;
+  TcSplit sp;
+  const int64_t all = tiles[0] + tiles[1];
+  if (all <= 0 || pairs < 2 || panels[0] <= 0 || panels[0] > (1 << 24) || (tiles[1] > 0 && panels[1] <= 0) ||
+      panels[1] > (1 << 24))
+    return sp;
+  const int64_t cuts = all % pairs, first = all - cuts;
+  if (cuts == 0) return sp;
+  const int64_t longest = tiles[1] > 0 && (panels[1] > panels[0] || first >= tiles[0]) ? panels[1] : panels[0];
+  const int64_t shortest = tiles[1] > 0 && (panels[1] < panels[0] || first >= tiles[0]) ? panels[1] : panels[0];
+  auto share = [&](int64_t parts) {
+    const double busy = static_cast<double>(parts * cuts) / static_cast<double>(pairs);
+    return static_cast<double>(terms * ((longest + parts - 1) / parts)) * (busy < LEAST ? LEAST : busy);
+  };
+  double best = share(1);
+  for (int64_t parts = 2; parts * cuts <= pairs && parts <= shortest; ++parts) {
+    const double cost = share(parts) + SUM + PART * static_cast<double>(parts - 2);
+    if (cost < best) {
+      best = cost;
+      sp.parts = static_cast<int>(parts);
+    }
+  }
+  if (!sp.parts) return sp;
+  sp.clusters = static_cast<int>(first > 0 ? pairs : sp.parts * cuts);
+  sp.first = static_cast<int>(first);
+  sp.ws_bytes = static_cast<size_t>(cuts) * sp.parts * 2 * TC_BM * TC_BN * sizeof(float);
+  sp.counters = static_cast<int>(cuts) * 2 * P2Shape<TC_EPI_F32>::EPI_WARPS * (P2Shape<TC_EPI_F32>::COLS / 32);
+  return sp;
 }
 
 int tc_gemm_pair_launch(int epi, const CUtensorMap& ta0, const CUtensorMap& tb0, const CUtensorMap* ta1,
