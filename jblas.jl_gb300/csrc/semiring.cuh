@@ -2,9 +2,9 @@
 //
 // jBLAS keeps a tuple-SIMD Vec type (src/simd.jl) out of its module with the note that it
 // could serve "custom number types ... so it works with min-plus algebra" (src/jBLAS.jl:10).
-// Here the custom arithmetic is a policy of the register-blocked mainloop shared with the
-// native GEMM (simt_gemm.cuh): the accumulator starts at the identity of (+), each k folds
-// in one (x) product, and the epilogue folds in C when accumulating.
+// Here the custom arithmetic is a policy of the tiles (semiring4_tile.cuh and simt_gemm.cuh for 4-byte
+// elements, semiring_f64.cu for doubles): the accumulator starts at the identity of (+), each k
+// folds in one (x) product, and the epilogue folds in C when accumulating.
 //
 // (+) is min or max.  For floating point it ignores a NaN operand (fminf / fmaxf) and a
 // zero result is stored as +0.0: min and max are then associative and commutative on every
@@ -88,8 +88,6 @@ template <typename T, int SR>
 struct SemiringOp {
   using Ar = SrArith<T>;
   static constexpr bool kMinPlus = SR == GB_SEMIRING_MIN_PLUS || SR == GB_SEMIRING_MIN_MAX;
-  static constexpr bool kInitFromC = false;   // C is folded in by the epilogue instead
-  static constexpr bool kVecStore = false;
   static constexpr bool kPairs =
       Ar::kHas3 && (std::is_floating_point<T>::value || SR == GB_SEMIRING_MAX_MIN || SR == GB_SEMIRING_MIN_MAX);
   int accumulate;

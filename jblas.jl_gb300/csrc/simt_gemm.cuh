@@ -1,5 +1,4 @@
-// Register-blocked GEMM mainloop on the CUDA cores, shared by the FP32 grouped GEMM and the
-// semiring GEMM.
+// Register-blocked GEMM mainloop on the CUDA cores: float and int32 semirings with large outputs.
 //
 // Restates jBLAS's register-blocked driver (src/gemm.jl:244-348) for the GPU: each
 // thread owns a TM x TN register tile of C (the reference's rows x cols tile from
@@ -11,11 +10,6 @@
 //   Op::init()            the accumulator before k = 1
 //   Op::step(acc, a, b)   one contraction step, applied for k = 1..K in order
 //   op.store(c, acc)      the epilogue writing one element of C
-//   Op::kVecStore         when true (with op.value(c, acc), the value store writes, and
-//                         op.reads_c(), whether it reads C's old value) C is written with vector
-//                         stores or, when C is not aligned for them, through shared memory
-//   Op::kInitFromC        when true the accumulator starts from C's element instead of init()
-//                         (jBLAS's kernel!, which folds A*X onto D's value)
 //   Op::kPairs, Op::step2(acc, a0, b0, a1, b1)
 //                         when kPairs, two consecutive k are folded in by one call (for
 //                         associative, exact reductions such as min / max, whose result
@@ -31,13 +25,6 @@ template <typename T, int V>
 struct alignas(sizeof(T) * V) VecT {
   T v[V];
 };
-
-template <typename T>
-__device__ __forceinline__ T fma_t(T a, T b, T c);
-template <>
-__device__ __forceinline__ double fma_t<double>(double a, double b, double c) { return fma(a, b, c); }
-template <>
-__device__ __forceinline__ float fma_t<float>(float a, float b, float c) { return fmaf(a, b, c); }
 
 // Shared memory of one tile: double-buffered BK x BM and BK x BN panels, rows padded by 16
 // bytes (transposing stores hit distinct banks, vector reads stay aligned).
@@ -136,18 +123,9 @@ __device__ __forceinline__ void simt_tile(int64_t M, int64_t N, int64_t K, const
 
   T acc[TM][TN];
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int64_t m = m0 + (i < VM ? ty * VM + i : BM / 2 + ty * VM + (i - VM));
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      if constexpr (Op::kInitFromC) {
-        const int64_t n = n0 + (j < VN ? tx * VN + j : BN / 2 + tx * VN + (j - VN));
-        acc[i][j] = (m < M && n < N) ? C[m + n * ldc] : T(0);
-      } else {
-        acc[i][j] = Op::init();
-      }
-    }
-  }
+    for (int j = 0; j < TN; ++j) acc[i][j] = Op::init();
 
   auto load_k = [&](int buf, int kk, T (&a)[TM], T (&b)[TN]) {
     const VecT<T, VM> a0 = *reinterpret_cast<const VecT<T, VM>*>(&As[buf][kk][ty * VM]);
@@ -219,75 +197,17 @@ __device__ __forceinline__ void simt_tile(int64_t M, int64_t N, int64_t K, const
     }
   }
 
-  if constexpr (Op::kVecStore) {
-    // Epilogue for policies with kVecStore (and op.value / op.reads_c), where short K loops
-    // make the stores of C a large part of a tile.  The per-element stores of the general path
-    // write one element in each of 16 columns per warp instruction; instead:
-    //  - beta = 0 and C and ldc multiples of VM elements: a thread's VM consecutive rows of a
-    //    column go out as one vector store (whole 32-byte sectors);
-    //  - otherwise the tile goes through shared memory, half of its rows at a time, and a warp
-    //    writes 32 consecutive rows of one column per instruction.  The panels' shared memory
-    //    is reused: every warp has finished reading it first.
-    const bool rc = op.reads_c();
-    const bool vec_ok = VM > 1 && !rc && (reinterpret_cast<uintptr_t>(C) % (VM * sizeof(T))) == 0 &&
-                        (ldc % VM) == 0;   // the same for the whole CTA
-    if (vec_ok) {
+  // (Whole rows of four at a time, with C read ahead, 4096 x 4096 x 32 with C folded in takes 62 us
+  // instead of 154, but the int32 k loops then spill: (max, min) 2368 x 3008 x 1472 0.93 -> 1.09 ms.)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int64_t mb = m0 + h * (BM / 2) + ty * VM;   // first of this half's VM rows
+  for (int i = 0; i < TM; ++i) {
+    const int64_t m = m0 + (i < VM ? ty * VM + i : BM / 2 + ty * VM + (i - VM));
+    if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          const int64_t n = n0 + (j < VN ? tx * VN + j : BN / 2 + tx * VN + (j - VN));
-          if (n >= N) continue;
-          T* __restrict__ c = &C[mb + n * ldc];
-          if (mb + VM <= M) {
-            VecT<T, VM> v;
-#pragma unroll
-            for (int i = 0; i < VM; ++i) v.v[i] = op.value(T(0), acc[h * VM + i][j]);
-            *reinterpret_cast<VecT<T, VM>*>(c) = v;
-          } else {
-#pragma unroll
-            for (int i = 0; i < VM; ++i)
-              if (mb + i < M) c[i] = op.value(T(0), acc[h * VM + i][j]);
-          }
-        }
-      }
-    } else {
-      constexpr int HR = BM / 2;    // rows per half
-      constexpr int LDS = HR + 1;   // column stride: consecutive rows in consecutive banks
-      static_assert(BN * LDS <= SimtSmem<T, BM, BN, BK>::ELEMS, "staged epilogue does not fit");
-      __syncthreads();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          const int col = (j < VN ? tx * VN + j : BN / 2 + tx * VN + (j - VN));
-#pragma unroll
-          for (int i = 0; i < VM; ++i) smem[col * LDS + ty * VM + i] = acc[h * VM + i][j];
-        }
-        __syncthreads();
-        for (int e = tid; e < HR * BN; e += NT) {
-          const int r = e % HR, col = e / HR;
-          const int64_t m = m0 + h * HR + r, n = n0 + col;
-          if (m < M && n < N) {
-            T* c = &C[m + n * ldc];
-            *c = op.value(rc ? *c : T(0), smem[col * LDS + r]);
-          }
-        }
-        __syncthreads();
-      }
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int64_t m = m0 + (i < VM ? ty * VM + i : BM / 2 + ty * VM + (i - VM));
-      if (m >= M) continue;
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const int64_t n = n0 + (j < VN ? tx * VN + j : BN / 2 + tx * VN + (j - VN));
-        if (n >= N) continue;
-        op.store(&C[m + n * ldc], acc[i][j]);
-      }
+    for (int j = 0; j < TN; ++j) {
+      const int64_t n = n0 + (j < VN ? tx * VN + j : BN / 2 + tx * VN + (j - VN));
+      if (n >= N) continue;
+      op.store(&C[m + n * ldc], acc[i][j]);
     }
   }
 }
