@@ -7,7 +7,7 @@
 // Measured in alternation with 128 x 128 / 64 x 64 scalar register tiles (FFMA peak 78 TFLOP/s):
 // 256^3 16.6 -> 13 us a call, 1536^3 217 -> 172 us, 2048^3 404 -> 336 us, 4096^3 2.70 -> 2.31 ms,
 // 4097 x 4095 x 4001 2.67 -> 2.30, 8192 x 8192 x 4096 10.4 -> 8.66 (63 TFLOP/s), 16384 x 64 x 16384
-// 1.11 -> 0.91; kernel! at 2048^3 519 -> 369 us.
+// 1.11 -> 0.88; kernel! at 2048^3 519 -> 369 us.
 #include <algorithm>
 
 #include "gb_common.cuh"

@@ -642,8 +642,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
 // The tiles left after the full rounds of a launch (all of them when there are fewer than pairs) take
 // a round of their own, however few they are.  Cut along K they occupy more pairs for their share of it,
 // at the price of partial sums.  Costs in K panels of a full round (0.335 us, the tensor cores' power
-// or operand bandwidth): with fewer pairs at work a panel takes less, down to three quarters from 57
-// pairs on; writing and adding the parts 32, and 2 for each beyond the second (512^3 x6 in four
+// or operand bandwidth): with fewer pairs at work a panel takes less, down to three quarters at 57
+// pairs and fewer; writing and adding the parts 32, and 2 for each beyond the second (512^3 x6 in four
 // parts would be 38 us, whole it is 34).  A part runs all term pairs of its K panels, so no sum in
 // TMEM is longer than before.  Tiles on more than half
 // of the pairs stay whole: the gain there is below the cost (cut in equal ranges of panels, or with the
