@@ -689,21 +689,10 @@ __device__ __forceinline__ void crt_split8(const double (&x)[8], int e, int tbit
 #pragma unroll
     for (int l = 0; l < ND; ++l) d[l][j] = dj[l];
   }
-  // The moduli counts automatic plans pick for FP64 data (t = 52) run a straight loop whose
-  // table constants are immediate operands; other counts loop over the planes.
-  if (ND == 4) {
-    switch (nmod) {
-#define GB_CRT_SPLIT_CASE(n)                                                                          \
-  case n: {                                                                                           \
-    _Pragma("unroll") for (int g = 0; g < n; ++g)                                                     \
-        store_residues(out0 + g * plane_stride, crt_residues8<ND>(d, mod, g), nvalid);                \
-    return;                                                                                           \
-  }
-      GB_CRT_SPLIT_CASE(14) GB_CRT_SPLIT_CASE(15) GB_CRT_SPLIT_CASE(16)
-#undef GB_CRT_SPLIT_CASE
-      default: break;
-    }
-  }
+  // One modulus a turn, its constants read once for the 8 elements.  Written out for the 14 to 16 moduli of
+  // automatic plans, the constants were immediate operands, but the warps waited for instructions:
+  // 1531 x 1021 and 1999 x 1021 38 us, 34 so.
+#pragma unroll 1
   for (int g = 0; g < nmod; ++g) store_residues(out0 + g * plane_stride, crt_residues8<ND>(d, mod, g), nvalid);
 }
 
@@ -717,7 +706,7 @@ __device__ __forceinline__ void crt_split8(const double (&x)[8], int e, int tbit
 //                     columns); per modulus a warp stores 4 rows x 128 bytes of the plane, whole lines.
 // No shared memory and no barriers: the residue work of one modulus overlaps the stores of the
 // previous one.  A's blocks come first, then B's.  1531 x 1999 x 1021, both operands k-contiguous, 15
-// moduli: 27 + 31 us in two launches of a row to a block, 37 in one.
+// moduli: 27 + 31 us in two launches of a row to a block, 34 in one.
 struct CrtSplitPart {
   CrtSplitSide side;
   uint32_t gx;   // blocks along k (k contiguous) or along the rows (rows contiguous)
@@ -869,10 +858,12 @@ __device__ __forceinline__ void crt_combine_column(const uint8_t* __restrict__ b
   uint32_t words[NMOD];   // all loads in flight before any use
 #pragma unroll
   for (int g = 0; g < NMOD; ++g) words[g] = __ldg(reinterpret_cast<const uint32_t*>(base + g * res_plane));
-  double out[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {   // one element at a time: only its accumulators are live
-    if (i0 + q >= M) continue;
+  // One element a turn: only its accumulators are live, and the loop's code stays at 5 KB (four elements
+  // written out waited for instructions: 1531 x 1999 41 -> 36.5 us, 8192 x 1024 90 -> 82; two 38).
+#pragma unroll 1
+  for (int q = 0; q < 4; ++q) {
+    if (i0 + q >= M) break;
+    const int eaq = q < 2 ? (q ? eai[1] : eai[0]) : (q == 2 ? eai[2] : eai[3]);
     const uint32_t sel = 0x7540u + q;   // byte q of a word over 0x4B0000..: 2^23 + byte
     uint64_t acc0 = 0, acc1 = 0, acc2 = 0, acc3 = 0;
     float ks = rc.ks0;
@@ -906,35 +897,26 @@ __device__ __forceinline__ void crt_combine_column(const uint8_t* __restrict__ b
       c = v >> 32;
     }
     double val;
-    if (eai[q] == OZ_EXP_NONFINITE || ebj == OZ_EXP_NONFINITE) {
+    if (eaq == OZ_EXP_NONFINITE || ebj == OZ_EXP_NONFINITE) {
       val = __longlong_as_double(0x7FF8000000000000ll);
     } else {
       const uint64_t lo = (static_cast<uint64_t>(word[1]) << 32) | word[0];
       const uint64_t hi = (static_cast<uint64_t>(word[3]) << 32) | word[2];
-      val = i128_times_pow2(hi, lo, eai[q] + ebj - two_t);
+      val = i128_times_pow2(hi, lo, eaq + ebj - two_t);
     }
     if (ab == 1)
       val = alpha * val;
     else if (ab == 2)
       val = fma(alpha, val, beta * ccol[i0 + q]);
-    out[q] = val;
-  }
-  double* dst = ccol + i0;
-  if (i0 + 3 < M && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {   // two 16-byte stores
-    reinterpret_cast<double2*>(dst)[0] = make_double2(out[0], out[1]);
-    reinterpret_cast<double2*>(dst)[1] = make_double2(out[2], out[3]);
-  } else {
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (i0 + q < M) dst[q] = out[q];
+    ccol[i0 + q] = val;
   }
 }
 
 // 512 rows of a column to a block: 1531 rows are 383 threads' work, three blocks of 128 threads
-// (two of 256 left a quarter of the threads without any; 1531 x 1999 with alpha and beta 45 -> 42 us,
-// 13.7 ps an element).  Bound by the integer and FP32 instructions of the reconstruction, 11 ps an
-// element at 8192^2 with 16 moduli; handing the values over by shuffles for contiguous stores, or
-// reading C ahead, gained nothing.
+// (two of 256 left a quarter of the threads without any; 1531 x 1999 with alpha and beta 45 -> 42
+// us).  Bound by the integer and FP32 instructions of the reconstruction, 10 ps an element at 8192^2
+// with 16 moduli; handing the values over by shuffles for contiguous stores, or reading C ahead,
+// gained nothing.
 constexpr int CRT_COMBINE_THREADS = 128;
 
 __global__ void __launch_bounds__(CRT_COMBINE_THREADS) crt_combine_kernel(const uint8_t* __restrict__ res, int64_t res_ld,
