@@ -15,7 +15,7 @@
 // product is exact.  n moduli cost n BF16 GEMMs, against s(s+1)/2 for s digit slices
 // (ozaki.cu), which is why this is the faster FP64-accurate mode.
 //
-// Kernels: crt_split_kc_kernel / crt_split_rc_kernel (residue planes, [modulus][row][pitch]
+// Kernels: crt_split_kernel (residue planes, [modulus][row][pitch]
 // BF16, K-major, read by TMA like the digit planes; k-contiguous and row-contiguous operands), the CTA-pair slice-product kernel with the TC_EPI_CRT epilogue
 // (tc_gemm2.cu: one group per modulus, uint8 residue planes out), crt_combine_kernel
 // (reconstruction in 128-bit integer arithmetic, FP64 rounding by integer ops, alpha/beta).
