@@ -1,5 +1,5 @@
 """The FP64 semirings on element-dealt tiles and ordered integer keys, at the edges of both: tiles of 1 to
-64 rows, panels of 8 to 32 k, each orientation, padded leading dimensions, K = 0; NaNs of either sign,
+64 rows, panels of 8 to 32 k, each orientation, padded leading dimensions; NaNs of either sign,
 infinities, both zeros, subnormals and the largest numbers.  (+) is exact, so bit-identical to the oracle."""
 import numpy as np
 import pytest
