@@ -100,10 +100,10 @@ GB_API int gb_set_tc_engine(int engine);
  *              none, else two; 4: 2 x 2 blocks (column panels when M <= 256); at most one per
  *              256 columns.  The residue products of block b run on a high-priority stream of the
  *              library while the caller's stream splits the operand panels of block b + 1 and
- *              reconstructs block b - 1 (and, before the first products, B's statistics and
- *              first panel split run there beside A's).  Under stream capture a call uses one
- *              block.
- *              Results do not depend on it.
+ *              reconstructs block b - 1.  A call uses one block under stream capture and, as long
+ *              as its class's tuning has the default's values (gb_tc_default_tuning, whoever set
+ *              them), when its output has at most two rounds of 256 x 256 tiles over the SM pairs
+ *              and no host copies.  Results do not depend on it.
  * Size classes by max(M, N): 0 up to 2048, 1 up to 8192, 2 beyond.  gb_set_tc_engine, when set,
  * overrides the engine of every kind. */
 typedef enum { GB_TC_OZAKI_SLICES = 0, GB_TC_OZAKI_CRT = 1, GB_TC_F32 = 2, GB_TC_ADJOINT = 3, GB_TC_KINDS = 4 } gb_tc_kind_t;
@@ -419,7 +419,8 @@ GB_API int gb_plan_ozaki_crt(int64_t M, int64_t N, int64_t K, int moduli, gb_oza
  * pair at a time) and host_copies = 1 for a host-buffer call with a pinned C, the row
  * boundaries rows[0..*row_blocks] (at most 2 blocks) and column boundaries
  * cols[0..*col_blocks] (at most 4) of the blocks, multiples of 256 but the last.  A call under
- * stream capture runs one block whatever this returns. */
+ * stream capture, and a small one under a default tuning (gb_tc_tuning_t.panels), runs one block
+ * whatever this returns. */
 GB_API int gb_crt_blocks(int64_t M, int64_t N, int panels, int sms, int host_copies, int64_t* rows, int* row_blocks,
                          int64_t* cols, int* col_blocks);
 /* The plan of the most recent OZAKI (BF16 or CRT) gb_gemm_f64 call made by the calling

@@ -681,10 +681,11 @@ static int crt_gemm(DeviceInfo* dev, int ta, int tb, int64_t M, int64_t N, int64
   // sequence on this stream) when the tuning asks for one and under stream capture; at most
   // one block column per 256 columns.
   const TcTuning tune = tc_tuning_for(TC_KIND_CRT, M, N);
-  // Up to two rounds of tiles a block by default: with both operands split in one launch, halves hide
+  // A default tuning runs up to two rounds of tiles as one block: with both operands split in one launch, halves hide
   // less than their shorter rounds and extra launches cost (8192 x 512 x 8192 1477 -> 1365 us,
   // 8000 x 500 x 3000 645 -> 580, 3000^3 840 -> 832; 2560^3 and 4096^3 the same).
-  const bool small = tc_pair_tiles(M, N) <= (dev->sms & ~1) && !sink && tc_tuning_is_default(TC_KIND_CRT, M, N);
+  const bool small = tc_pair_tiles(M, N) <= (dev->sms & ~1) && !sink &&
+                     tc_tuning_is_default(TC_KIND_CRT, tc_tune_class(M, N), tune);
   const CrtBlocks blocks = crt_blocks(M, N, small ? 1 : tune.panels, dev->sms, sink != nullptr);
   const int panels = blocks.prow * blocks.pcol;
   cudaStreamCaptureStatus cap_status = cudaStreamCaptureStatusNone;

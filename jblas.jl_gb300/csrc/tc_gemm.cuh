@@ -115,10 +115,11 @@ int tc_tune_class(int64_t M, int64_t N);
 constexpr int TC_MAX_PANELS = 4;   // CRT column panels
 TcTuning tc_default_tuning(int kind, int cls);
 int tc_validate_tuning(int kind, const TcTuning& t);
+// Whether `t` has the default's values, whoever set it: a tuning read and written back, or put back
+// after an autotuner's run, means what it meant.
+bool tc_tuning_is_default(int kind, int cls, const TcTuning& t);
 // The tuning a call of this kind and output size uses (gb_set_tc_engine, when set, overrides
 // the engine).
-// Whether no caller has set the tuning that tc_tuning_for gives.
-bool tc_tuning_is_default(int kind, int64_t M, int64_t N);
 TcTuning tc_tuning_for(int kind, int64_t M, int64_t N);
 int tc_set_tuning(int kind, int cls, const TcTuning* t);   // t = nullptr: the default
 TcTuning tc_get_tuning(int kind, int cls);

@@ -14,7 +14,6 @@ namespace {
 std::mutex g_tune_mu;
 bool g_tune_init = false;
 TcTuning g_tune[TC_KINDS][TC_TUNE_CLASSES];
-bool g_tune_set[TC_KINDS][TC_TUNE_CLASSES];   // by a caller, not the defaults
 
 void init_locked() {
   if (g_tune_init) return;
@@ -75,9 +74,9 @@ TcTuning tc_tuning_for(int kind, int64_t M, int64_t N) {
   return t;
 }
 
-bool tc_tuning_is_default(int kind, int64_t M, int64_t N) {
-  std::lock_guard<std::mutex> lk(g_tune_mu);
-  return !g_tune_set[kind][tc_tune_class(M, N)];
+bool tc_tuning_is_default(int kind, int cls, const TcTuning& t) {
+  const TcTuning d = tc_default_tuning(kind, cls);
+  return t.engine == d.engine && t.band == d.band && t.tma_store == d.tma_store && t.panels == d.panels;
 }
 
 int tc_set_tuning(int kind, int cls, const TcTuning* t) {
@@ -88,7 +87,6 @@ int tc_set_tuning(int kind, int cls, const TcTuning* t) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   init_locked();
   g_tune[kind][cls] = v;
-  g_tune_set[kind][cls] = t != nullptr;
   return GB_OK;
 }
 
