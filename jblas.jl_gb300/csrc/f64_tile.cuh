@@ -107,22 +107,31 @@ struct F64Loader {
 
 // The policy of the FMA chains:
 //   ONTO = false   the chain starts at -0.0 (fma(a1, x1, -0.0) is the rounded product a1 x1) and
-//                  C = alpha * chain [+ beta * C], written without a multiply when unit (alpha = 1,
-//                  beta = 0: the multiply would run on the FP64 pipe)
+//                  C = alpha * chain [+ beta * C]; `out` (f64_out) says which of the terms there are, so
+//                  that the epilogue issues no other FP64 instruction, comparisons of alpha and beta
+//                  included: each costs an element as much as one k
 //   ONTO = true    the chain starts at C's value and is stored as it is (jBLAS's kernel!)
+enum { F64_CHAIN, F64_SCALED, F64_WITH_C };
+// On the bits: 1.0 is the only double with its pattern, and a shift drops the sign of zero.
+__host__ __device__ inline int f64_out(long long alpha_bits, long long beta_bits) {
+  return (static_cast<unsigned long long>(beta_bits) << 1) != 0 ? F64_WITH_C
+       : alpha_bits != 0x3FF0000000000000ll ? F64_SCALED : F64_CHAIN;
+}
 template <bool ONTO>
 struct F64Chain {
   using Elem = double;   // an element in shared memory, and
   using Acc = double;    // what a lane keeps for an element of C
   static constexpr bool ENCODE = false;   // no rewriting of the panels
+  static constexpr int AHEAD = 4;         // old values of C in flight (8: the same, and more spilled)
   double alpha, beta;
-  bool unit;
+  int out;
   __device__ __forceinline__ double init(const double* c, bool in) const { return (ONTO && in) ? *c : -0.0; }
   static __device__ __forceinline__ double step(double acc, double a, double b) { return fma(a, b, acc); }
-  __device__ __forceinline__ void store(double* c, double acc) const {
-    if (ONTO || unit) *c = acc;
-    else *c = (beta == 0.0) ? alpha * acc : fma(alpha, acc, beta * *c);
-  }
+  __device__ __forceinline__ bool reads_c() const { return !ONTO && out == F64_WITH_C; }
+  __device__ __forceinline__ double value(double c, double acc) const { return fma(alpha, acc, beta * c); }
+  __device__ __forceinline__ bool plain() const { return ONTO || out == F64_CHAIN; }
+  static __device__ __forceinline__ double raw(double acc) { return acc; }
+  __device__ __forceinline__ double value(double acc) const { return alpha * acc; }
 };
 
 // NU chains per lane over the kc k of one panel; off[i] holds the byte offsets of the lane's row
@@ -250,12 +259,34 @@ __device__ __forceinline__ void f64_tile(int r, int c, int64_t K, const double* 
   }
   cp_async_wait<0>();   // (only empty groups are left)
 
+  // C's old values, where the epilogue reads them, are requested AHEAD at a time before the first is
+  // used; the three ways are written out, so that none issues another's FP64 instructions: with one
+  // expression for all and a value at a time, 4096 x 4096 x 8 with alpha and beta took 372 us instead of
+  // 312 (alpha = 1, beta = 0: 231).  (The addresses are opaque before this point: computed ahead
+  // and kept through the k loop, they spilled.)
+  if constexpr (Op::AHEAD > 1) asm volatile("" : "+l"(C), "+l"(ldc));
+  auto at = [&](int i) { return C + (off[i] & 0xFFFFu) / 8 + static_cast<int64_t>(off[i] >> 19) * ldc; };
+  constexpr int AHEAD = MAXU < Op::AHEAD ? MAXU : Op::AHEAD;
+  const int mine = elems - v * 32 - lane;   // element i is the lane's when i * F64_THREADS < mine
+  if (op.reads_c()) {
 #pragma unroll
-  for (int i = 0; i < MAXU; ++i) {
-    if (i >= nu) break;
-    if (v * 32 + lane + i * F64_THREADS < elems) {
-      op.store(C + (off[i] & 0xFFFFu) / 8 + static_cast<int64_t>(off[i] >> 19) * ldc, acc[i]);
+    for (int i0 = 0; i0 < MAXU; i0 += AHEAD) {
+      double old[AHEAD];
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i)
+        if ((i0 + i) * F64_THREADS < mine) old[i] = *at(i0 + i);
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i)
+        if ((i0 + i) * F64_THREADS < mine) *at(i0 + i) = op.value(old[i], acc[i0 + i]);
     }
+  } else if (op.plain()) {
+#pragma unroll
+    for (int i = 0; i < MAXU; ++i)
+      if (i * F64_THREADS < mine) *at(i) = Op::raw(acc[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < MAXU; ++i)
+      if (i * F64_THREADS < mine) *at(i) = op.value(acc[i]);
   }
 }
 

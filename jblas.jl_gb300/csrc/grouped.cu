@@ -316,8 +316,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64_CTAS)
       scale_tile<double>(p, m0, n0, r, c, threadIdx.x, F64_THREADS);
       return;
     }
-    const bool unit = __double_as_longlong(p.alpha) == 0x3FF0000000000000ll && __double_as_longlong(p.beta) == 0ll;
-    const F64Chain<false> chain{p.alpha, p.beta, unit};
+    const F64Chain<false> chain{p.alpha, p.beta, f64_out(__double_as_longlong(p.alpha), __double_as_longlong(p.beta))};
     const int cols = min(32, F64_MAX_ELEMS / r);   // larger tiles run in column strips
     for (int j0 = 0; j0 < c; j0 += cols) {
       if (j0) __syncthreads();   // the strip reuses the shared panels

@@ -6,6 +6,8 @@
 // that the first step fma(a1, x1, -0.0) equals the rounded product a1*x1 bit for bit,
 // signed zeros included; the K tail is handled with an exact trip count (no zero
 // padding, which would turn -0 into +0 and Inf*0 into NaN).
+#include <cstring>
+
 #include "f64_gemm.cuh"
 #include "gb_common.cuh"
 #include "native_gemm.cuh"
@@ -44,7 +46,7 @@ int native_scale_f32(int64_t M, int64_t N, float beta, float* C, int64_t ldc, cu
 int native_kernel_onto_f64(int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B,
                            int64_t ldb, double* C, int64_t ldc, int sms, cudaStream_t s) {
   if (M == 0 || N == 0 || K == 0) return GB_OK;   // an empty chain leaves D as it is
-  return launch_f64_gemm(GB_KERNEL_NATIVE_GEMM, F64Chain<true>{1.0, 0.0, true}, M, N, K, A, 1, lda, B, 1, ldb, C, ldc,
+  return launch_f64_gemm(GB_KERNEL_NATIVE_GEMM, F64Chain<true>{1.0, 0.0, F64_CHAIN}, M, N, K, A, 1, lda, B, 1, ldb, C, ldc,
                          sms, s);
 }
 
@@ -53,7 +55,10 @@ int native_gemm_f64(int ta, int tb, int64_t M, int64_t N, int64_t K, double alph
                     cudaStream_t s) {
   if (M == 0 || N == 0) return GB_OK;
   if (alpha == 0.0 || K == 0) return launch_scale<double>(M, N, beta, C, ldc, s);
-  return launch_f64_gemm(GB_KERNEL_NATIVE_GEMM, F64Chain<false>{alpha, beta, alpha == 1.0 && beta == 0.0}, M, N, K, A,
+  long long ab[2];
+  std::memcpy(&ab[0], &alpha, 8);
+  std::memcpy(&ab[1], &beta, 8);
+  return launch_f64_gemm(GB_KERNEL_NATIVE_GEMM, F64Chain<false>{alpha, beta, f64_out(ab[0], ab[1])}, M, N, K, A,
                          ta ? lda : 1, ta ? 1 : lda, B, tb ? ldb : 1, tb ? 1 : ldb, C, ldc, sms, s);
 }
 
