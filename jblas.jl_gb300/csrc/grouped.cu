@@ -275,10 +275,16 @@ __device__ __forceinline__ bool alpha_is_zero(const gb_problem_t& p) {
   return (__double_as_longlong(p.alpha) & 0x7FFFFFFFFFFFFFFFll) == 0;
 }
 
-// Persistent tile loop: CTA b takes tile b of the schedule, then the next one that no CTA has taken (a
+constexpr int GROUPED_CTAS = 4;   // resident CTAs an SM, both element types
+static_assert(GROUPED_CTAS == F64_CTAS, "grid of the grouped kernels");
+
+// Persistent tile loop: each CTA takes a tile of the schedule, then the next one that no CTA has taken (a
 // counter in offsets[0]; its answer is fetched while the tile runs).  Against a fixed stride, where
-// the busiest SM of 4096 log-uniform problems gets 3.5% more than its share.  run(tile, index) may leave
-// its shared memory without a barrier: one follows.
+// the busiest SM of 4096 log-uniform problems gets 3.5% more than its share.  The first tiles go to the
+// CTAs from the second quarter of the grid on, which are one to an SM; with the grid's first CTAs, which
+// put three on each of four SMs, calls of less than a grid of tiles were slower (f32, 16 problems of
+// 300^3 47 -> 40 us, one of 1000^3 96 -> 75, 64 of 128^3 23 -> 19; f64, 100 of 64^3 78 -> 62).
+// run(tile, index) may leave its shared memory without a barrier: one follows.
 template <class Run>
 __device__ __forceinline__ void grouped_loop(const gb_problem_t* __restrict__ probs, int count,
                                              const gb_grouped_tuning_t& tuning, bool f32, long long* __restrict__ ws,
@@ -288,7 +294,8 @@ __device__ __forceinline__ void grouped_loop(const gb_problem_t* __restrict__ pr
   const int* order = reinterpret_cast<const int*>(grouped_order_words(ws, count));
   const long long total = offsets[count];
   int lo = 0, slot = 0;
-  for (long long w = blockIdx.x; w < total; slot ^= 1) {
+  const unsigned skip = gridDim.x / GROUPED_CTAS;
+  for (long long w = blockIdx.x + (blockIdx.x < skip ? gridDim.x : 0) - skip; w < total; slot ^= 1) {
     long long next = 0;
     if (threadIdx.x == 0)
       next = gridDim.x + static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(ws), 1ull));
@@ -334,8 +341,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64_CTAS)
 // tiles three quarters of their time was waiting for instructions (4096 log-uniform problems 1.1 to
 // 1.8 ms; 32 x 32 tiles 0.85 ms, bound by their 4-byte copies).
 using GroupedPiece = S4Shape<8, 4, 2, 2>;
-constexpr int GROUPED_F32_CTAS = 4;
-__global__ void __launch_bounds__(GroupedPiece::THREADS, GROUPED_F32_CTAS)
+__global__ void __launch_bounds__(GroupedPiece::THREADS, GROUPED_CTAS)
     grouped_f32_kernel(const gb_problem_t* __restrict__ probs, int count, gb_grouped_tuning_t tuning,
                        long long* __restrict__ ws) {
   __shared__ __align__(16) uint32_t smem[GroupedPiece::SMEM_BYTES / 4];
@@ -381,11 +387,11 @@ int grouped_validate_tuning(int dtype_bytes, const gb_grouped_tuning_t& t) {
 }
 
 // 64 x 64 pieces from which FP32's per-problem choice takes them (auto_config_f32): three a CTA.
-static int f32_enough(int sms) { return 3 * GROUPED_F32_CTAS * sms; }
+static int f32_enough(int sms) { return 3 * GROUPED_CTAS * sms; }
 
 static int launch_f64_tiles(const gb_problem_t* d_probs, int count, const gb_grouped_tuning_t& tuning, long long* ws,
                             int sms, cudaStream_t s) {
-  grouped_f64_kernel<<<sms * F64_CTAS, F64_THREADS, 0, s>>>(d_probs, count, tuning, ws);
+  grouped_f64_kernel<<<sms * GROUPED_CTAS, F64_THREADS, 0, s>>>(d_probs, count, tuning, ws);
   return GB_OK;
 }
 
@@ -395,7 +401,7 @@ static int launch_tiles(int dtype_bytes, const gb_problem_t* d_probs, int count,
     GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s, launch_f64_tiles(d_probs, count, tuning, d_ws, sms, s));
   else
     GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
-              (grouped_f32_kernel<<<sms * GROUPED_F32_CTAS, GroupedPiece::THREADS, 0, s>>>(d_probs, count, tuning,
+              (grouped_f32_kernel<<<sms * GROUPED_CTAS, GroupedPiece::THREADS, 0, s>>>(d_probs, count, tuning,
                                                                                            d_ws)));
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
