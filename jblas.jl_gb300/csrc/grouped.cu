@@ -53,9 +53,14 @@ __host__ __device__ inline int size_class(int64_t m, int64_t n) {
   return d <= 16 ? 0 : d <= 32 ? 1 : d <= 64 ? 2 : d <= 128 ? 3 : d <= 256 ? 4 : 5;
 }
 
-// Per-problem choice (GB_GROUPED_AUTO) in FP32: 64 x 64 pieces, or 32 x 32 ones where all problems
-// together have too few of the larger for every CTA of the grid to take several.
+// GB_GROUPED_AUTO in FP32, one choice for the whole table: 64 x 64 pieces, or 32 x 32 ones (one warp at
+// work on each) where the outputs together have fewer elements than three quarters of such a piece an
+// SM.  Measured, 32 x 32 and 64 x 64: 50 problems of 65 x 65 x 100 15.4 and 18.1 us, 10 of 200 x 200 x 64
+// 14.1 and 14.8, one of 512^3 31.8 and 30.1, 32 of 128^3 17.4 and 15.7, 64 of 128^3 26 and 19, 16 of
+// 300^3 61 and 40, 4 of 1000 x 1000 x 200 98 and 63 (with the line at three pieces a CTA all of these took
+// the former).
 __host__ __device__ inline int auto_config_f32(bool large) { return large ? 3 : 1; }
+static int64_t f32_large_elems(int sms) { return static_cast<int64_t>(sms) * (64 * 64 * 3 / 4); }
 
 // Extents of an FP64 problem's tiles under a configuration: equal tiles as large as the
 // configuration allows (33 rows on 32-row tiles: 17 + 16, not 32 + 1).
@@ -118,7 +123,7 @@ __device__ __forceinline__ void scale_tile(const gb_problem_t& p, int64_t m0, in
   }
 }
 
-// The configuration one problem runs under: the table's, or the per-problem choice (`large`: auto_config_f32).
+// The configuration one problem runs under: the table's, or the library's choice (`large`: auto_config_f32).
 __device__ __forceinline__ int prologue_config(const gb_grouped_tuning_t& tuning, const gb_problem_t& p, bool f32,
                                                bool large) {
   const int c = config_of(tuning, size_class(p.m, p.n));
@@ -144,7 +149,7 @@ __host__ __device__ inline int grouped_order_entry(int i, int cfg, int count) {
 // independent).
 __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_problem_t* __restrict__ probs, int count,
                                                               gb_grouped_tuning_t tuning, bool f32,
-                                                              int enough, long long* __restrict__ ws) {
+                                                              long long large_elems, long long* __restrict__ ws) {
   __shared__ long long part[1024];
   __shared__ int hist[32], start[32];
   long long* offsets = ws;
@@ -153,18 +158,16 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   if (t < 32) hist[t] = 0;
   bool large = true;   // (a table too long to pack keeps the larger tiles)
   if (f32 && count <= GROUPED_PACK_LIMIT) {
-    int pieces = 0;   // 64 x 64 pieces of all problems, up to the threshold
-    for (int i = t; i < count && pieces < enough; i += 1024) {
-      const gb_problem_t& p = probs[i];
-      if (p.m > 0 && p.n > 0) pieces += static_cast<int>(min(static_cast<int64_t>(enough), ((p.m + 63) / 64) * ((p.n + 63) / 64)));
-    }
-    part[t] = pieces;
+    long long elems = 0;   // of all outputs, up to the line
+    for (int i = t; i < count && elems < large_elems; i += 1024)
+      if (probs[i].m > 0 && probs[i].n > 0) elems += probs[i].m * probs[i].n;
+    part[t] = elems;
     __syncthreads();
     for (int off = 512; off > 0; off >>= 1) {
       if (t < off) part[t] += part[t + off];
       __syncthreads();
     }
-    large = part[0] >= enough;
+    large = part[0] >= large_elems;
   }
   __syncthreads();
   auto bucket_of = [&](const gb_problem_t& p, int cfg) {
@@ -370,8 +373,7 @@ gb_grouped_tuning_t grouped_default_tuning(int dtype_bytes) {
   gb_grouped_tuning_t t;
   std::memset(&t, 0, sizeof(t));
   // classes: <=16, <=32, <=64, <=128, <=256, >256
-  // The per-problem choice in every class (rectangular FP32 tiles for tall and wide problems; the
-  // FP64 tiles that pad least).
+  // The library's choice in every class (auto_config_f32, auto_config_f64).
   (void)dtype_bytes;
   for (int c = 0; c < GB_GROUPED_CLASSES; ++c) t.config[c] = GB_GROUPED_AUTO;
   return t;
@@ -385,9 +387,6 @@ int grouped_validate_tuning(int dtype_bytes, const gb_grouped_tuning_t& t) {
       return GB_ERR_INVALID_VALUE;
   return GB_OK;
 }
-
-// 64 x 64 pieces from which FP32's per-problem choice takes them (auto_config_f32): three a CTA.
-static int f32_enough(int sms) { return 3 * GROUPED_CTAS * sms; }
 
 static int launch_f64_tiles(const gb_problem_t* d_probs, int count, const gb_grouped_tuning_t& tuning, long long* ws,
                             int sms, cudaStream_t s) {
@@ -411,8 +410,8 @@ int grouped_launch(int dtype_bytes, const gb_problem_t* d_probs, int count, cons
                    long long* d_offsets, int sms, cudaStream_t s) {
   if (count <= 0) return GB_OK;
   GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
-            (grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, tuning, dtype_bytes == 4, f32_enough(sms),
-                                                      d_offsets)));
+            (grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, tuning, dtype_bytes == 4,
+                                                      f32_large_elems(sms), d_offsets)));
   GB_CUDA_TRY(cudaGetLastError());
   return launch_tiles(dtype_bytes, d_probs, count, tuning, d_offsets, sms, s);
 }
@@ -604,8 +603,9 @@ int grouped_strided_launch(int dtype_bytes, gb_problem_t* d_probs, long long* d_
   int cfg = -1;
   long long tiles = 0;
   if (count <= GROUPED_PACK_LIMIT) {
-    const int64_t pieces = ((M + 63) / 64) * ((N + 63) / 64);
-    cfg = dtype_bytes == 8 ? auto_config_f64(M, N, K) : auto_config_f32(pieces >= f32_enough(sms) / count + 1);
+    // (M N count >= the line, without the product)
+    const bool large = M * N >= (f32_large_elems(sms) + count - 1) / count;
+    cfg = dtype_bytes == 8 ? auto_config_f64(M, N, K) : auto_config_f32(large);
     const TileCfg c = tile_cfg(cfg);
     tiles = ((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
   }
