@@ -32,7 +32,7 @@ struct TileCfg {
   int bm, bn;
 };
 // 0-3 serve both element types; 4-9, the larger and rectangular tiles, are FP32 only.  FP64 takes bm
-// and bn as the largest extents of its tiles (f64_tile.cuh); FP32 runs a tile in pieces of 64 x 64.
+// and bn as the largest extents of its tiles (f64_tiles); FP32 runs a tile in pieces of 64 x 64.
 __host__ __device__ constexpr TileCfg tile_cfg(int c) {
   return c == 0 ? TileCfg{16, 16}
        : c == 1 ? TileCfg{32, 32}
@@ -63,38 +63,68 @@ __host__ __device__ inline int auto_config_f32(bool large) { return large ? 3 : 
 static int64_t f32_large_elems(int sms) { return static_cast<int64_t>(sms) * (64 * 64 * 3 / 4); }
 
 // Extents of an FP64 problem's tiles under a configuration: equal tiles as large as the
-// configuration allows (33 rows on 32-row tiles: 17 + 16, not 32 + 1).
+// configuration, 32 columns and F64_MAX_ELEMS allow (33 rows on 32-row tiles: 17 + 16, not 32 + 1).
+// In 32-bit arithmetic: a 64-bit division is some hundred instructions, of which the one-block prologue
+// would make a dozen per problem; beyond it tiles are not made equal.
 struct F64Tiles {
   int tm, tn, fm, fn;
 };
 __host__ __device__ inline F64Tiles f64_tiles(const TileCfg& c, int64_t m, int64_t n) {
-  F64Tiles t;
-  t.tm = static_cast<int>((m + c.bm - 1) / c.bm);
-  t.tn = static_cast<int>((n + c.bn - 1) / c.bn);
-  t.fm = t.tm > 0 ? static_cast<int>((m + t.tm - 1) / t.tm) : 0;
-  t.fn = t.tn > 0 ? static_cast<int>((n + t.tn - 1) / t.tn) : 0;
-  return t;
+  if (m <= 0 || n <= 0) return F64Tiles{0, 0, 0, 0};
+  if (m > 0x7FFFFFFF - 64 || n > 0x7FFFFFFF - 64)
+    return F64Tiles{static_cast<int>((m + c.bm - 1) / c.bm), static_cast<int>((n + 15) / 16), c.bm, 16};
+  const uint32_t m32 = static_cast<uint32_t>(m), n32 = static_cast<uint32_t>(n);
+  const uint32_t tm = (m32 + c.bm - 1) / c.bm, fm = (m32 + tm - 1) / tm;
+  const uint32_t room = F64_MAX_ELEMS / fm, most = c.bn < 32 ? c.bn : 32, width = room < most ? room : most;
+  const uint32_t tn = (n32 + width - 1) / width, fn = (n32 + tn - 1) / tn;
+  return F64Tiles{static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(fm), static_cast<int>(fn)};
 }
 
-// The same in FP64, where the DFMA pipe bounds everything (f64_tile.cuh): the configuration with
-// the fewest units of 32 elements, a tile's barriers, first loads and stores counting as 26 unit-k
-// (measured on 8192 problems of 32 x 32 x 64: 1.01 ms on 16 x 16 tiles, 0.96 on 32 x 32), among those
-// whose tiles hold at most F64_MAX_ELEMS (larger ones run in strips and re-read A).
-__host__ __device__ inline int auto_config_f64(int64_t m, int64_t n, int64_t k) {
-  float best = 3.4e38f;
+// GB_GROUPED_AUTO in FP64, where the DFMA pipe bounds everything (f64_tile.cuh).  A tile costs its units
+// of 32 elements times k and, for its barriers, first loads and stores, 26 unit-k (measured on 8192
+// problems of 32 x 32 x 64: 1.01 ms on 16 x 16 tiles, 0.96 on 32 x 32).  A call takes the sum of these
+// over the SM partitions, or the longest tile's time on one of the four warps if that is longer.
+struct F64Load {
+  long long total = 0, longest = 0;
+  __host__ __device__ void add(const F64Tiles& t, int64_t k, long long problems = 1) {
+    const long long kk = k > 1 ? k : 1, units = (t.fm * t.fn + 31) / 32;
+    const long long one = ((units + 3) / 4) * kk;
+    total += problems * t.tm * t.tn * (units * kk + 26);
+    longest = one > longest ? one : longest;
+  }
+  __host__ __device__ long long time(int sms) const {   // times 4 sms
+    const long long l = longest * 4 * sms;
+    return total > l ? total : l;
+  }
+};
+// Per problem the configuration with the smallest total (0-2; 3 has 2's tiles), among those whose tiles
+// F64_MAX_ELEMS does not cut (64 of 100^3 on cut 64 x 32 tiles, 10 a problem: 199 us, on 32 x 32 141), or, if a
+// call has too little work for that, 16 x 16 for all: one problem of 100^3 32 -> 18 us, 10 of 64^3 31 -> 17,
+// one of 64 x 64 x 200 78 -> 27; 16 of 100^3 stay (45 us, 63 on 16 x 16).
+__host__ __device__ inline int auto_config_f64(int64_t m, int64_t n, int64_t k, F64Tiles* tiles) {
+  *tiles = f64_tiles(tile_cfg(0), m, n);
+  if (m <= 16 && n <= 16) return 0;   // one tile under any of them
+  F64Load first;
+  first.add(*tiles, k);
+  long long best = first.total;
   int arg = 0;
-  for (int c = 0; c < GROUPED_CONFIGS_F64; ++c) {
+  for (int c = 1; c < 3; ++c) {
     const F64Tiles t = f64_tiles(tile_cfg(c), m, n);
-    if (t.fm * t.fn > F64_MAX_ELEMS) continue;
-    const float units = static_cast<float>((t.fm * t.fn + 31) / 32);
-    const float cost = static_cast<float>(t.tm) * static_cast<float>(t.tn) *
-                       (units * static_cast<float>(k > 1 ? k : 1) + 26.0f);
-    if (cost < best) {
-      best = cost;
+    if (c == 2 && t.tn > (n + 31) / 32) continue;
+    F64Load l;
+    l.add(t, k);
+    if (l.total < best) {
+      best = l.total;
       arg = c;
+      *tiles = t;
     }
   }
   return arg;
+}
+// (From eight problems an SM the first choice stands, which saves the prologue the second.)
+__host__ __device__ inline bool f64_may_be_small(int count, int sms) { return count < 8 * sms; }
+__host__ __device__ inline bool f64_small(const F64Load& chosen, const F64Load& small, int sms) {
+  return small.time(sms) < chosen.time(sms);
 }
 
 // tuning.config[cls] without a dynamically indexed (local-memory) array
@@ -123,14 +153,6 @@ __device__ __forceinline__ void scale_tile(const gb_problem_t& p, int64_t m0, in
   }
 }
 
-// The configuration one problem runs under: the table's, or the library's choice (`large`: auto_config_f32).
-__device__ __forceinline__ int prologue_config(const gb_grouped_tuning_t& tuning, const gb_problem_t& p, bool f32,
-                                               bool large) {
-  const int c = config_of(tuning, size_class(p.m, p.n));
-  if (c != GB_GROUPED_AUTO) return c;
-  return f32 ? auto_config_f32(large) : auto_config_f64(p.m, p.n, p.k);
-}
-
 // Workspace of a call over `count` problems (int64 words): the tile prefix sums in schedule
 // order offsets[0..count], then the schedule order (count int32 entries: the problem index,
 // and for count <= 2^24 its tile configuration in bits 24-30, so the tile loop need not
@@ -142,48 +164,111 @@ __host__ __device__ inline int grouped_order_entry(int i, int cfg, int count) {
   return count <= GROUPED_PACK_LIMIT ? (i | (cfg << 24)) : i;
 }
 
+// The configuration of a problem of a table too long for packed order entries.
+__device__ __forceinline__ int unpacked_config(const gb_grouped_tuning_t& tuning, const gb_problem_t& p, bool f32) {
+  const int c = config_of(tuning, size_class(p.m, p.n));
+  F64Tiles t;
+  return c != GB_GROUPED_AUTO ? c : f32 ? auto_config_f32(true) : auto_config_f64(p.m, p.n, p.k, &t);
+}
+
+__device__ __forceinline__ long long tile_count(const gb_problem_t& p, const TileCfg& c, bool f32) {
+  if (p.m <= 0 || p.n <= 0) return 0;
+  if (f32) return ((p.m + c.bm - 1) / c.bm) * ((p.n + c.bn - 1) / c.bn);
+  const F64Tiles t = f64_tiles(c, p.m, p.n);
+  return static_cast<long long>(t.tm) * t.tn;
+}
+
+// What the prologue decides for a problem: its configuration under the table, with the library's choice
+// for a table of enough work or for a small one (auto_config_f32, f64_small), and the bucket of the
+// schedule each puts it in.  Kept in the workspace's prefix sums until these are written.
+__device__ __forceinline__ int choice_word(int cfg, int bucket, int cfg_small, int bucket_small) {
+  return cfg | bucket << 5 | cfg_small << 10 | bucket_small << 15;
+}
+__device__ __forceinline__ int choice_config(int word, bool small) { return word >> (small ? 10 : 0) & 31; }
+__device__ __forceinline__ int choice_bucket(int word, bool small) { return word >> (small ? 15 : 5) & 31; }
+
 // Prologue (one block): the schedule orders the problems by the work of one of their tiles
 // (rows x columns x k of what a tile holds, in 32 power-of-two buckets, heaviest first), so that the
-// CTAs take tiles of similar length side by side and the short ones fill the tail; it writes the order and the exclusive prefix sums of the tiles in that order.
+// CTAs take tiles of similar length side by side and the short ones fill the tail; it writes the order and
+// the exclusive prefix sums of the tiles in that order.
 // The order inside a bucket depends on timing, which changes no result (each tile is
-// independent).
+// independent).  Each problem's choice is made once: made again for the histogram, the order and with
+// 64-bit divisions it was a third of a call on 4000 FP64 problems of 8^3 (65 us, now 45).
 __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_problem_t* __restrict__ probs, int count,
-                                                              gb_grouped_tuning_t tuning, bool f32,
+                                                              gb_grouped_tuning_t tuning, bool f32, int sms,
                                                               long long large_elems, long long* __restrict__ ws) {
   __shared__ long long part[1024];
+  __shared__ long long sums[4][32];
   __shared__ int hist[32], start[32];
   long long* offsets = ws;
+  int* words = reinterpret_cast<int*>(ws);
   int* order = reinterpret_cast<int*>(grouped_order_words(ws, count));
   const int t = threadIdx.x;
+  const bool packed = count <= GROUPED_PACK_LIMIT;   // (a longer table keeps the choice for enough work)
   if (t < 32) hist[t] = 0;
-  bool large = true;   // (a table too long to pack keeps the larger tiles)
-  if (f32 && count <= GROUPED_PACK_LIMIT) {
-    long long elems = 0;   // of all outputs, up to the line
-    for (int i = t; i < count && elems < large_elems; i += 1024)
-      if (probs[i].m > 0 && probs[i].n > 0) elems += probs[i].m * probs[i].n;
-    part[t] = elems;
-    __syncthreads();
-    for (int off = 512; off > 0; off >>= 1) {
-      if (t < off) part[t] += part[t + off];
-      __syncthreads();
-    }
-    large = part[0] >= large_elems;
-  }
-  __syncthreads();
-  auto bucket_of = [&](const gb_problem_t& p, int cfg) {
-    const long long k = p.k > 1 ? p.k : 1;
-    const TileCfg c = tile_cfg(cfg);
-    const F64Tiles t = f64_tiles(c, p.m, p.n);
-    const long long held = f32 ? min(p.m, static_cast<int64_t>(c.bm)) * min(p.n, static_cast<int64_t>(c.bn))
-                               : static_cast<long long>(t.fm) * t.fn;
-    const long long w = held * k;
+  auto bucket = [](long long held, int64_t k) {
+    const long long w = held * (k > 1 ? k : 1);
     const int lg = 63 - __clzll(w > 1 ? w : 1);
     return 31 - (lg > 31 ? 31 : lg);                 // heavy first
   };
+  auto held_f32 = [](const gb_problem_t& p, int cfg) {
+    const TileCfg c = tile_cfg(cfg);
+    return min(p.m, static_cast<int64_t>(c.bm)) * min(p.n, static_cast<int64_t>(c.bn));
+  };
+  const bool may_be_small = f32 ? packed : f64_may_be_small(count, sms);
+  F64Load chosen, least;
   for (int i = t; i < count; i += 1024) {
     const gb_problem_t& p = probs[i];
-    atomicAdd(&hist[bucket_of(p, prologue_config(tuning, p, f32, large))], 1);
+    const int c = config_of(tuning, size_class(p.m, p.n));
+    if (f32) {
+      const int a = c == GB_GROUPED_AUTO ? auto_config_f32(true) : c, b = c == GB_GROUPED_AUTO ? auto_config_f32(false) : c;
+      if (p.m > 0 && p.n > 0) chosen.total += p.m * p.n;   // elements of C
+      words[i] = choice_word(a, bucket(held_f32(p, a), p.k), b, bucket(held_f32(p, b), p.k));
+    } else {
+      F64Tiles ta;
+      int a = c, b = c, bucket_b = 0;
+      if (c == GB_GROUPED_AUTO) a = auto_config_f64(p.m, p.n, p.k, &ta);
+      else ta = f64_tiles(tile_cfg(c), p.m, p.n);
+      if (may_be_small) {
+        F64Tiles tb = ta;
+        if (c == GB_GROUPED_AUTO) {
+          b = 0;
+          tb = f64_tiles(tile_cfg(0), p.m, p.n);
+        }
+        chosen.add(ta, p.k);
+        least.add(tb, p.k);
+        bucket_b = bucket(tb.fm * tb.fn, p.k);
+      }
+      words[i] = choice_word(a, bucket(ta.fm * ta.fn, p.k), b, bucket_b);
+    }
   }
+  auto combine = [](F64Load& l, int off) {
+    l.total += __shfl_xor_sync(0xffffffffu, l.total, off);
+    l.longest = max(l.longest, __shfl_xor_sync(0xffffffffu, l.longest, off));
+  };
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    combine(chosen, off);
+    combine(least, off);
+  }
+  if ((t & 31) == 0) {
+    sums[0][t >> 5] = chosen.total;
+    sums[1][t >> 5] = chosen.longest;
+    sums[2][t >> 5] = least.total;
+    sums[3][t >> 5] = least.longest;
+  }
+  __syncthreads();
+  chosen.total = sums[0][t & 31];
+  chosen.longest = sums[1][t & 31];
+  least.total = sums[2][t & 31];
+  least.longest = sums[3][t & 31];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    combine(chosen, off);
+    combine(least, off);
+  }
+  const bool small = may_be_small && (f32 ? chosen.total < large_elems : f64_small(chosen, least, sms));
+  for (int i = t; i < count; i += 1024) atomicAdd(&hist[choice_bucket(words[i], small)], 1);
   __syncthreads();
   if (t == 0) {
     int run = 0;
@@ -194,19 +279,16 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   }
   __syncthreads();
   for (int i = t; i < count; i += 1024) {
-    const gb_problem_t& p = probs[i];
-    const int cfg = prologue_config(tuning, p, f32, large);
-    order[atomicAdd(&start[bucket_of(p, cfg)], 1)] = grouped_order_entry(i, cfg, count);
+    const int w = words[i];
+    order[atomicAdd(&start[choice_bucket(w, small)], 1)] = grouped_order_entry(i, choice_config(w, small), count);
   }
   __syncthreads();
   const int per = (count + 1023) / 1024;
   const int b = t * per, e = min(count, b + per);
-  const bool packed = count <= GROUPED_PACK_LIMIT;
   auto tiles_of = [&](int pos) -> long long {
     const int e = order[pos];
     const gb_problem_t& p = probs[packed ? (e & 0xFFFFFF) : e];
-    const TileCfg c = tile_cfg(packed ? (e >> 24) : prologue_config(tuning, p, f32, large));
-    return (p.m <= 0 || p.n <= 0) ? 0 : ((p.m + c.bm - 1) / c.bm) * ((p.n + c.bn - 1) / c.bn);
+    return tile_count(p, tile_cfg(packed ? (e >> 24) : unpacked_config(tuning, p, f32)), f32);
   };
   long long sum = 0;
   for (int i = b; i < e; ++i) sum += tiles_of(i);
@@ -266,7 +348,7 @@ __device__ __forceinline__ void grouped_find(const gb_problem_t* __restrict__ pr
   const int e = order[lo];
   const bool packed = count <= GROUPED_PACK_LIMIT;
   t.p = probs[packed ? (e & 0xFFFFFF) : e];
-  t.c = tile_cfg(packed ? (e >> 24) : prologue_config(tuning, t.p, f32, true));
+  t.c = tile_cfg(packed ? (e >> 24) : unpacked_config(tuning, t.p, f32));
   // in 32-bit arithmetic (a problem's tile count is below 2^31); the first problem's tiles start at 0
   const int local = static_cast<int>(lo ? w - offsets[lo] : w);
   const int tiles_m = static_cast<int>((t.p.m + t.c.bm - 1) / t.c.bm);
@@ -327,13 +409,8 @@ __global__ void __launch_bounds__(F64_THREADS, F64_CTAS)
       return;
     }
     const F64Chain<false> chain{p.alpha, p.beta, f64_out(__double_as_longlong(p.alpha), __double_as_longlong(p.beta))};
-    const int cols = min(32, F64_MAX_ELEMS / r);   // larger tiles run in column strips
-    for (int j0 = 0; j0 < c; j0 += cols) {
-      if (j0) __syncthreads();   // the strip reuses the shared panels
-      f64_tile_any(r, min(cols, c - j0), p.k, static_cast<const double*>(p.A) + m0, 1, p.lda,
-                   static_cast<const double*>(p.B) + (n0 + j0) * p.ldb, 1, p.ldb, chain,
-                   static_cast<double*>(p.C) + m0 + (n0 + j0) * p.ldc, p.ldc, static_cast<int>(w ^ (w >> 2)), smem);
-    }
+    f64_tile_any(r, c, p.k, static_cast<const double*>(p.A) + m0, 1, p.lda, static_cast<const double*>(p.B) + n0 * p.ldb, 1,
+                 p.ldb, chain, static_cast<double*>(p.C) + m0 + n0 * p.ldc, p.ldc, static_cast<int>(w ^ (w >> 2)), smem);
   });
 }
 
@@ -410,7 +487,7 @@ int grouped_launch(int dtype_bytes, const gb_problem_t* d_probs, int count, cons
                    long long* d_offsets, int sms, cudaStream_t s) {
   if (count <= 0) return GB_OK;
   GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
-            (grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, tuning, dtype_bytes == 4,
+            (grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, tuning, dtype_bytes == 4, sms,
                                                       f32_large_elems(sms), d_offsets)));
   GB_CUDA_TRY(cudaGetLastError());
   return launch_tiles(dtype_bytes, d_probs, count, tuning, d_offsets, sms, s);
@@ -552,7 +629,7 @@ int grouped_f64_noalloc(const gb_problem_t* d_probs, int count, const gb_grouped
   // clearing.
   // Launched directly, not through the timing hooks (which create CUDA events while profiling
   // is on); gb_launch_counts still counts both launches.
-  grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, t, false, 0, offsets);
+  grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, t, false, sms, 0, offsets);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return gb_set_cuda_error(e, "grouped prologue launch");
   prof_count(GB_KERNEL_GROUPED_GEMM);
@@ -605,9 +682,23 @@ int grouped_strided_launch(int dtype_bytes, gb_problem_t* d_probs, long long* d_
   if (count <= GROUPED_PACK_LIMIT) {
     // (M N count >= the line, without the product)
     const bool large = M * N >= (f32_large_elems(sms) + count - 1) / count;
-    cfg = dtype_bytes == 8 ? auto_config_f64(M, N, K) : auto_config_f32(large);
-    const TileCfg c = tile_cfg(cfg);
-    tiles = ((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
+    if (dtype_bytes == 8) {
+      F64Tiles t;
+      cfg = auto_config_f64(M, N, K, &t);
+      const F64Tiles t0 = f64_tiles(tile_cfg(0), M, N);
+      F64Load chosen, least;
+      chosen.add(t, K, count);
+      least.add(t0, K, count);
+      if (f64_may_be_small(count, sms) && f64_small(chosen, least, sms)) {
+        cfg = 0;
+        t = t0;
+      }
+      tiles = static_cast<long long>(t.tm) * t.tn;
+    } else {
+      cfg = auto_config_f32(large);
+      const TileCfg c = tile_cfg(cfg);
+      tiles = ((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
+    }
   }
   const int blocks = (count + 255) / 256;
   grouped_fill_strided_kernel<<<blocks, 256, 0, s>>>(d_probs, count, M, N, K, lda, ldb, ldc,
