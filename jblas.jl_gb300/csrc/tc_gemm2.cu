@@ -644,14 +644,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2Shape<EPI>::THREAD
 // at the price of partial sums.  Costs in K panels of a full round (0.335 us, the tensor cores' power
 // or operand bandwidth): with fewer pairs at work a panel takes less, down to three quarters at 57
 // pairs and fewer; writing and adding the parts 32, and 2 for each beyond the second (512^3 x6 in four
-// parts would be 38 us, whole it is 34).  A part runs all term pairs of its K panels, so no sum in
+// parts would be 38 us, whole it is 34).  After whole tiles, whose epilogues the cut tiles' first panels
+// overlap either way, a panel of few pairs takes four fifths, and the parts cost 20 and 7 (fitted to
+// every number of parts at 77 to 320 tiles and 4 to 64 panels; within 0.7% of the best, while the other
+// costs lost up to 10% to whole tiles: 20224 x 256 x 704 x6 with C folded in 87 us whole, 96 in six
+// parts).  A part runs all term pairs of its K panels, so no sum in
 // TMEM is longer than before.  Tiles on more than half
 // of the pairs stay whole: the gain there is below the cost (cut in equal ranges of panels, or with the
 // idle pairs taking over a share, 2048^3 x6 went 84 -> 95 us and 3001 x 2503 x 2047 146 -> 143).
 // x6: 1024^3 (16 tiles) 47 -> 41 us, 1600 x 3328 x 1312 (91) 101 -> 87, 4096^3 (256) 529 -> 491,
 // 500 x 500 x 20000 (4) 551 -> 131.
 TcSplit tc_split_plan(const int64_t (&tiles)[2], const int64_t (&panels)[2], int terms, int pairs) {
-  constexpr double LEAST = 0.75, SUM = 32.0, PART = 2.0;
   TcSplit sp;
   const int64_t all = tiles[0] + tiles[1];
   if (all <= 0 || pairs < 2 || panels[0] <= 0 || panels[0] > (1 << 24) || (tiles[1] > 0 && panels[1] <= 0) ||
@@ -659,6 +662,7 @@ TcSplit tc_split_plan(const int64_t (&tiles)[2], const int64_t (&panels)[2], int
     return sp;
   const int64_t cuts = all % pairs, first = all - cuts;
   if (cuts == 0) return sp;
+  const double LEAST = first ? 0.8 : 0.75, SUM = first ? 20.0 : 32.0, PART = first ? 7.0 : 2.0;
   const int64_t longest = tiles[1] > 0 && (panels[1] > panels[0] || first >= tiles[0]) ? panels[1] : panels[0];
   const int64_t shortest = tiles[1] > 0 && (panels[1] < panels[0] || first >= tiles[0]) ? panels[1] : panels[0];
   auto share = [&](int64_t parts) {
