@@ -41,7 +41,6 @@ struct SrArith<float> {
   static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
   static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
   static __device__ __forceinline__ float canon(float v) { return v == 0.0f ? 0.0f : v; }
-  static constexpr bool kHas3 = true;
   static __device__ __forceinline__ float min3(float a, float b, float c) {
     float r;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -55,15 +54,12 @@ struct SrArith<float> {
 };
 
 template <>
-struct SrArith<double> {
-  static __device__ __forceinline__ double lo() { return __longlong_as_double(0xfff0000000000000ll); }
-  static __device__ __forceinline__ double hi() { return __longlong_as_double(0x7ff0000000000000ll); }
+struct SrArith<double> {   // (identities and the steps of a chain: semiring_f64.cu)
   static __device__ __forceinline__ double min(double a, double b) { return fmin(a, b); }
   static __device__ __forceinline__ double max(double a, double b) { return fmax(a, b); }
   static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
   static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
   static __device__ __forceinline__ double canon(double v) { return v == 0.0 ? 0.0 : v; }
-  static constexpr bool kHas3 = false;
 };
 
 template <>
@@ -79,7 +75,6 @@ struct SrArith<int32_t> {
     return static_cast<int32_t>(static_cast<uint32_t>(a) * static_cast<uint32_t>(b));
   }
   static __device__ __forceinline__ int32_t canon(int32_t v) { return v; }
-  static constexpr bool kHas3 = true;
   static __device__ __forceinline__ int32_t min3(int32_t a, int32_t b, int32_t c) { return __vimin3_s32(a, b, c); }
   static __device__ __forceinline__ int32_t max3(int32_t a, int32_t b, int32_t c) { return __vimax3_s32(a, b, c); }
 };
@@ -89,7 +84,7 @@ struct SemiringOp {
   using Ar = SrArith<T>;
   static constexpr bool kMinPlus = SR == GB_SEMIRING_MIN_PLUS || SR == GB_SEMIRING_MIN_MAX;
   static constexpr bool kPairs =
-      Ar::kHas3 && (std::is_floating_point<T>::value || SR == GB_SEMIRING_MAX_MIN || SR == GB_SEMIRING_MIN_MAX);
+      std::is_floating_point<T>::value || SR == GB_SEMIRING_MAX_MIN || SR == GB_SEMIRING_MIN_MAX;
   int accumulate;
 
   static __device__ __forceinline__ T oplus(T x, T y) { return kMinPlus ? Ar::min(x, y) : Ar::max(x, y); }

@@ -30,21 +30,20 @@ struct SrShape {
 // XF the lanes along x, KF the lanes along k.
 template <int X, int LD>
 struct SrLoader {
+  static_assert(X == 32, "a lane per x");
   static constexpr int KP = 0, XF = 1, KF = 2;
-  static constexpr int FX = X < 32 ? X : 32, FNX = X / FX;
   const uint32_t* p;
-  int64_t str, adv, xstep;
+  int64_t str, adv;
   uint32_t dst;
   int way, x, k;
 
   __device__ __forceinline__ void init(const uint32_t* src, int64_t xs, int64_t ks) {
     const int lane = threadIdx.x & 31;
     way = (ks == 1 && xs != 1) ? ((reinterpret_cast<uintptr_t>(src) & 7) == 0 && (xs & 1) == 0 ? KP : KF) : XF;
-    x = way == KP ? lane / 4 : way == XF ? lane % FX : lane / 8;
-    k = way == KP ? lane % 4 * 2 : way == XF ? lane / FX : lane % 8;
+    x = way == KP ? lane / 4 : way == XF ? lane : lane / 8;
+    k = way == KP ? lane % 4 * 2 : way == XF ? 0 : lane % 8;
     p = src + x * xs + k * ks;
-    str = way == KP ? 8 * xs : way == XF ? 32 / FX * ks : 4 * xs;
-    xstep = FX * xs;
+    str = way == KP ? 8 * xs : way == XF ? ks : 4 * xs;
     adv = S4_BK * ks;
     dst = static_cast<uint32_t>(k / 2 * LD + 2 * x + k % 2) * 4u;
   }
@@ -61,15 +60,9 @@ struct SrLoader {
           else if (x + l * 8 < extent && k + h < kc) cp_async_4(to, q + h);
         }
     } else if (way == XF) {
-      static_assert(FX == 32 || FX == 16, "x extents");
 #pragma unroll 8
-      for (int l = 0; l < S4_BK * FX / 32; ++l, q += str) {
-        constexpr int FK = 32 / FX;   // k step; FK = 2 keeps k's parity, FK = 1 alternates it
-        const uint32_t to = d + (FK == 2 ? l * LD : l / 2 * LD + l % 2) * 4;
-#pragma unroll
-        for (int h = 0; h < FNX; ++h)
-          if (!CHECK || (x + h * FX < extent && k + l * FK < kc)) cp_async_4(to + h * FX * 8, q + h * xstep);
-      }
+      for (int l = 0; l < S4_BK; ++l, q += str)
+        if (!CHECK || (x < extent && l < kc)) cp_async_4(d + (l / 2 * LD + l % 2) * 4, q);
     } else {
 #pragma unroll 8
       for (int l = 0; l < X / 4; ++l, q += str)

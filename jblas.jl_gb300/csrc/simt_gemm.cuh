@@ -13,7 +13,7 @@
 //   Op::kPairs, Op::step2(acc, a0, b0, a1, b1)
 //                         when kPairs, two consecutive k are folded in by one call (for
 //                         associative, exact reductions such as min / max, whose result
-//                         does not depend on the grouping; the FMA chain keeps kPairs false)
+//                         does not depend on the grouping; int32 sums and products keep it false)
 // The K tail is handled with an exact trip count: no padded k is ever folded in.
 #pragma once
 #include <cuda_runtime.h>
@@ -213,10 +213,9 @@ __device__ __forceinline__ void simt_tile(int64_t M, int64_t N, int64_t K, const
 }
 
 // The tile above as a kernel: CTA (x, y) computes the tile at (x BM, y BN).
-// 4-byte elements: two CTAs per SM (at most 128 registers a thread for 256 threads);
-// 8-byte elements: no residency bound (0), which leaves ptxas its own register choice.
+// Two CTAs per SM: at most 128 registers a thread for 256 threads.
 template <typename T, typename Op, int BM, int BN, int BK, int TM, int TN, bool TA, bool TB>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), sizeof(T) == 4 ? 2 : 0)
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), 2)
     simt_gemm_kernel(int64_t M, int64_t N, int64_t K, Op op, const T* __restrict__ A, int64_t lda,
                      const T* __restrict__ B, int64_t ldb, T* __restrict__ C, int64_t ldc) {
   __shared__ __align__(16) T smem[SimtSmem<T, BM, BN, BK>::ELEMS];
