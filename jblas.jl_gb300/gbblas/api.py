@@ -29,9 +29,14 @@ class DimensionMismatch(ValueError):
 # launch.  So the calls below pass integers straight to the C signatures (which convert them), take the
 # current stream as an integer (a torch.cuda.Stream object per call costs 2 us) and read each shape
 # once: 7.0 us.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)   # not a public name: torch may drop it
+
+
 def _stream_of(t):
     """The current stream of t's device (an integer); t is a CUDA tensor."""
-    return torch._C._cuda_getCurrentRawStream(t.get_device())
+    if _raw_stream is None:
+        return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.get_device())
 
 
 def _storage(X, name, allow_copy):
