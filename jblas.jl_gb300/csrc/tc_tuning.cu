@@ -166,6 +166,17 @@ int tc_autotune(int kind, int64_t M, int64_t N, int64_t K, int reps, TcTuning* o
   };
   // the adjoint writes dA over D as well as dB: both outputs share D's storage here, which only
   // the timing sees (the operands stay A, B, C)
+  // A launch of FP32 outputs on pairs that cuts tiles has a band of its own: one candidate for all of them.
+  int device = 0, sms = 0;
+  GB_CUDA_TRY(cudaGetDevice(&device));
+  GB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  auto t256 = [](int64_t x) { return (x + 255) / 256; };
+  auto kp = [](int64_t x) { return (x + TC_BK - 1) / TC_BK; };
+  const bool cut = kind == TC_KIND_F32
+                       ? tc_split_plan({t256(M) * t256(N), 0}, {kp(K), 0}, 3, sms / 2).parts > 0
+                   : kind == TC_KIND_ADJOINT
+                       ? tc_split_plan({t256(M) * t256(K), t256(K) * t256(N)}, {kp(N), kp(M)}, 3, sms / 2).parts > 0
+                       : false;
   const int cls = tc_tune_class(M, N);
   const TcTuning saved = tc_get_tuning(kind, cls);
   const int saved_engine = tc_engine_setting();
@@ -179,6 +190,7 @@ int tc_autotune(int kind, int64_t M, int64_t N, int64_t K, int reps, TcTuning* o
     if (kind == TC_KIND_CRT && engine == 1) continue;
     for (int bi = 0; bi < 5 && !rc; ++bi) {
       const int band = (engine == 2 ? 2 : 4) << bi;   // 2..32 pair tiles, 4..64 single tiles
+      if (cut && engine == 2 && band != TC_SPLIT_BAND) continue;
       // the second option: TMA stores of C (FP32 outputs on pairs) or column panels (CRT: 1..4)
       const int nopt = (kind == TC_KIND_CRT) ? TC_MAX_PANELS
                        : (engine == 2 && (kind == TC_KIND_F32 || kind == TC_KIND_ADJOINT)) ? 2 : 1;
