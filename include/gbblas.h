@@ -90,7 +90,9 @@ GB_API int gb_set_tc_engine(int engine);
  *              2 = a CTA pair per 256 x 256 tile (cta_group::2, each SM loads half of B);
  *              the CRT mode runs on pairs only
  *   band       output-tile rows per band of the tile raster (1..64; tiles of a band share their
- *              A rows in L2)
+ *              A rows in L2); without effect where a launch of GB_TC_F32 or GB_TC_ADJOINT on pairs
+ *              cuts tiles along K (which tiles these are goes by the raster, and results do not
+ *              depend on the tuning's band): there it is 8, and gb_autotune_tc times that alone
  *   tma_store  FP32 outputs (GB_TC_F32, GB_TC_ADJOINT) on the pair engine: 1 = C staged in
  *              shared memory and written by TMA stores (beta = 0), 0 = direct stores
  *   panels     GB_TC_OZAKI_CRT only (0 elsewhere): C in blocks — 0 or 1: one; 2: two equal
@@ -233,6 +235,11 @@ GB_API int gb_gemm_f64(int transA, int transB, int64_t M, int64_t N, int64_t K, 
                 const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                 double* C, int64_t ldc, int mode, int slices, double* err_bound_out,
                 void* stream);
+/* gb_gemm_f32 (and gb_jmul_f32, gb_kernel_f32) first copies operands that are k-contiguous or not
+ * 16-byte aligned to rows-contiguous ones where that is sooner (from about 1000 rows and columns up):
+ * up to 4 K (M + N) bytes, rows padded to a multiple of 128, from the library pool, which keeps the
+ * memory (gb_release_workspace).  Under stream capture, or when the memory cannot be had, it
+ * reads them as they are; the bits are the same. */
 GB_API int gb_gemm_f32(int transA, int transB, int64_t M, int64_t N, int64_t K, float alpha,
                 const float* A, int64_t lda, const float* B, int64_t ldb, float beta,
                 float* C, int64_t ldc, void* stream);
@@ -245,7 +252,11 @@ GB_API int gb_gemm_f32(int transA, int transB, int64_t M, int64_t N, int64_t K, 
  *                   (2^-15 + K 2^-24) |alpha| (|op(A)| |op(B)|)_ij  (+ beta C rounding)
  *   GB_MODE_BF16X6  3 terms, 6 products; about (2^-21 + K 2^-24) |alpha| (|op(A)| |op(B)|)_ij,
  *                   FP32-level accuracy
- * Workspace (the term planes, (terms) x (M + N) x K BF16) comes from the library pool.  Other
+ * Workspace (the term planes, (terms) x (M + N) x K BF16, and, where the last tiles are cut along K
+ * over several CTA pairs, up to 19 MiB of partial sums) comes from the library pool.  Repeated
+ * calls give the same bits, with two exceptions where tiles are cut (their sums are rounded in
+ * another order, within the bounds above): the two engines (gb_set_tc_engine) differ, and so does a
+ * call that finds memory for the planes but not for the partial sums, which cuts nothing.  Other
  * modes give GB_ERR_INVALID_VALUE.  Arguments, transposes, alpha/beta rules as gb_gemm_f32. */
 GB_API int gb_gemm_f32_ex(int transA, int transB, int64_t M, int64_t N, int64_t K, float alpha,
                           const float* A, int64_t lda, const float* B, int64_t ldb, float beta,
@@ -286,12 +297,14 @@ typedef struct {
 
 /* Tile configuration per size class.  Classes by max(m, n): <=16, <=32, <=64, <=128,
  * <=256, >256.  Configurations (rows x cols of a C tile; f64: the largest extents of a problem's
- * equal tiles):
+ * equal tiles, of at most 32 columns and 1024 elements; f32: runs in pieces of at most 64 x 64, so
+ * that 4, 5 and 7 are 3's pieces in another order):
  *   0: 16x16  1: 32x32  2: 64x32  3: 64x64                     (f64 and f32)
  *   4: 128x64  5: 128x128  6: 32x64  7: 64x128  8: 128x32  9: 32x128   (f32 only)
- *   GB_GROUPED_AUTO: chosen per problem from its m, n and k by a cost model (f32: padding of the
- *   tiles against the FMA efficiency of their register tiles; f64: DFMA work and a cost per tile);
- *   the default
+ *   GB_GROUPED_AUTO, the default: f64, 0, 1 or 2 per problem from its m, n and k (DFMA work and a cost
+ *   per tile), or 0 for all problems of a table with too little work for that; f32, one choice for
+ *   the table, 64 x 64 pieces, or 32 x 32 where the outputs together are smaller than three quarters of
+ *   such a piece an SM
  * This replaces jBLAS's fixed BLASOptions(m_k, p_k) (src/blas_options.jl:2-7). */
 #define GB_GROUPED_CLASSES 6
 #define GB_GROUPED_CONFIGS 10
@@ -381,7 +394,9 @@ GB_API int gb_gemm_semiring_i32(int semiring, int transA, int transB, int64_t M,
 /* Autotuner: times every configuration per size class on the given problems (HOST copy
  * of the table; their C buffers are left untouched, results go to scratch) with `reps`
  * timed repetitions and writes the fastest configuration per class; class_ms (may be
- * NULL) receives the best time per class in ms.  Synchronises `stream`.
+ * NULL) receives the best time per class in ms.  A class is timed by itself, and GB_GROUPED_AUTO,
+ * one of the candidates, looks at the table it runs in: for a small class of a large table it can be
+ * timed with one choice and run with the other.  Synchronises `stream`.
  * Reference: pick_kernel_size / blocking_structure, src/kernel_structure.jl:76-99,
  * src/memory_management.jl:78-177. */
 GB_API int gb_autotune_grouped(int dtype_bytes, const gb_problem_t* host_problems, int count, int reps,
@@ -393,7 +408,8 @@ GB_API int gb_autotune_grouped(int dtype_bytes, const gb_problem_t* host_problem
  * in one tensor-core launch.  No reference counterpart: it is the rrule of jBLAS's
  * jmul!/gemm! (src/gemm.jl:244).  Products use the 3xBF16 split (x = hi + lo, the
  * lo*lo term dropped) with FP32 accumulation: per element |error| <= about
- * 2^-15 (|dC||B|^T)_ik plus FP32 summation error.  dC is read from memory once. */
+ * 2^-15 (|dC||B|^T)_ik plus FP32 summation error.  dC is read from memory once.  Workspace and
+ * repeatability as gb_gemm_f32_ex. */
 GB_API int gb_gemm_adjoint_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B,
                         int64_t ldb, const float* dC, int64_t lddc, float* dA, int64_t ldda, float* dB,
                         int64_t lddb, void* stream);
