@@ -61,26 +61,56 @@ __global__ void __launch_bounds__(32 * WARPS, 1) f32_gemm_kernel(const F32Args g
   }
 }
 
-// The tile shapes, with what a rule on them needs: the cycles one k of a tile takes on an SM filled
-// with such tiles, the least it takes alone, how slowly few tiles reach the full rate, and what an
-// operand that is not x-contiguous and aligned costs (measured at 2 GHz on 256^3 to 4096^3).
+// How an operand's panels are copied: 16 bytes at a time, 4 bytes along x (unaligned), or 4 along k.
+enum F32Copy { COPY_16, COPY_4_X, COPY_4_K };
+static F32Copy copy_of(const void* p, int64_t xs, int64_t ks) {
+  if (xs != 1) return COPY_4_K;
+  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ks & 3) == 0 ? COPY_16 : COPY_4_X;
+}
+
+// The tile shapes and a time model of a product on each (cycles at 2 GHz), with n tiles on the fullest SM
+// and so ceil(n / 4) warps on its fullest partition:
+//   a k    max(alone, warp0 + warp ceil(n / 4)) and, with operands in 4-byte copies, their sum of copy n and
+//          COPY_LATENCY more
+//   once   fixed + tile n, where a tile's stores depend on whether C's rows are contiguous for the tile
+//          (not with the operands' roles exchanged) and C is read
+// Fitted to the times of 860 products on every shape, both ways round, packed and not (up to 4e10
+// multiply-adds, an eighth of them in vectors of 8 to 128): the choice is within 2% of the best one on
+// average, 5% faster than that of a model of full tiles and one cost per tile, whose misses were short K
+// (256 x 4672 x 32 12.4 us on 64 x 64 tiles, 8.4 on 32 x 32) and long products with both operands in
+// 4-byte copies (112 x 9081 x 3103 276 us, packed 230).  On 660 other products: 254 faster by more than 2%,
+// 34 slower (at most 16%), 4.7% faster on average; 11 slower than on the register tiles of 4 x 4 to 8 x 8
+// elements a thread that came before (at most 9%; 31, at most 19%, under that model).
 enum F32Tile { T64X64, T32X32, T32X16 };
 struct F32TileInfo {
   int bm, bn;
-  double full, alone, few;
-  double unpacked;   // share by which one operand in 4-byte copies slows the product
+  double alone, warp0, warp;
+  double copy[3];       // by F32Copy
+  double fixed, tile[2][2];   // [roles exchanged][C read]
 };
 static const F32TileInfo kF32Tile[] = {
-    {64, 64, 41.5, 196.0, 1.0, 0.06}, {32, 32, 12.6, 79.0, 1.5, 0.16}, {32, 16, 8.2, 60.0, 1.5, 0.16}};
+    {64, 64, 172, 0, 113, {0.0, 5.3, 10}, 6900, {{5500, 1100}, {5000, 9000}}},
+    {32, 32, 93, 21, 39.7, {0.0, 1.5, 3.1}, 740, {{1100, 760}, {480, 4000}}},
+    {32, 16, 52.6, 15.6, 26.5, {0.0, 1, 1.6}, 545, {{400, 760}, {210, 1470}}}};
+constexpr double COPY_LATENCY = 13.4;
+// The 32 x 16 tile with the longer side of C along its 16 columns reads that side's operand in half the
+// width (36 x 8672 x 10813 520 us, the other way round 415).
+constexpr double SHORT_ROWS = 1.107;
+// Packing copies of `x` rows of K elements: read and write, and one more launch and the buffer's
+// allocation, as much on the host as on the device.
+constexpr double PACK_BYTES_PER_CYCLE = 1950, PACK_LAUNCH = 16500;
 
-// Time model (cycles) of an M x N x K product on one shape: n tiles on the busiest SM take
-// max(alone, n full (1 + few / (n + 1))) cycles a k, and each some 600 for its first loads and stores.
-static double f32_cost(F32Tile t, int64_t M, int64_t N, int64_t K, int sms) {
+// The cost of a choice; of the tile's own time alone with packed operands.
+static double f32_cost(F32Tile t, bool exchanged, int64_t M, int64_t N, int64_t K, F32Copy a, F32Copy b, bool reads_c,
+                       int sms) {
   const F32TileInfo& i = kF32Tile[t];
   const int64_t tiles = ((M + i.bm - 1) / i.bm) * ((N + i.bn - 1) / i.bn);
-  const double n = static_cast<double>((tiles + sms - 1) / sms);
-  const double per_k = std::max(i.alone, n * i.full * (1.0 + i.few / (n + 1.0)));
-  return static_cast<double>(K) * per_k + 600.0 * n;
+  const int64_t n = (tiles + sms - 1) / sms;
+  const double copies = i.copy[a] + i.copy[b], nd = static_cast<double>(n);
+  const double per_k = std::max(i.alone, i.warp0 + i.warp * static_cast<double>((n + 3) / 4)) *
+                           (t == T32X16 && M < N ? SHORT_ROWS : 1.0) +
+                       (copies > 0.0 ? copies * nd + COPY_LATENCY : 0.0);
+  return static_cast<double>(K) * per_k + i.fixed + i.tile[exchanged][reads_c] * nd;
 }
 
 template <class S, bool ANY, int WARPS, class Op>
@@ -142,85 +172,75 @@ __global__ void __launch_bounds__(256) f32_pack_kernel(const PackJob j0, const P
   }
 }
 
-static bool x_aligned(const void* p, int64_t xs, int64_t ks) {
-  return xs == 1 && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ks & 3) == 0;
+// C^T = B^T A^T: the same chain (fma commutes), with the tile's rows along the columns of C.
+static void exchange_roles(F32Args* g) {
+  std::swap(g->M, g->N);
+  std::swap(g->a, g->b);
+  std::swap(g->ars, g->bcs);
+  std::swap(g->aks, g->bks);
+  std::swap(g->crs, g->ccs);
 }
 
-// Estimated cost in cycles of packing `x` rows of K elements: read and write at about 4 TB/s.
-static double pack_cost(int64_t x, int64_t K) { return 8.0 * static_cast<double>(x) * static_cast<double>(K) / 4e12 * 2e9; }
-// One more launch and the buffer's allocation, as much on the host as on the device.
-constexpr double PACK_LAUNCH = 9e-6 * 2e9;
-
+// Direct, on 4-byte copies of the operands that need them, or packed; either way round; on the shape that the
+// model finds soonest.  Packing needs a buffer: under capture (no allocation in the graph), or when it
+// cannot be had, the call takes the best direct choice.
 template <class Op>
-static int f32_run(F32Args g, const Op& op, int sms, cudaMemPool_t pool, cudaStream_t s) {
-  const int64_t M = g.M, N = g.N, K = g.K;
-  // The 32 x 16 tile is taller than wide: a product of few rows runs with the operands' roles
-  // exchanged, C^T = B^T A^T (the same chain; fma commutes), where that is cheaper.
-  auto best_of = [&](int64_t m, int64_t n, F32Tile* t) {
-    double best = 1e300;
-    for (F32Tile c : {T64X64, T32X32, T32X16}) {
-      const double cost = f32_cost(c, m, n, K, sms);
-      if (cost < best) best = cost, *t = c;
+static int f32_run(F32Args g, const Op& op, bool reads_c, int sms, cudaMemPool_t pool, cudaStream_t s) {
+  const int64_t K = g.K;
+  struct Choice {
+    double cost = 1e300;
+    F32Tile tile = T32X32;
+    bool exchanged = false;
+  } direct, packed;
+  const F32Copy ca = copy_of(g.a, g.ars, g.aks), cb = copy_of(g.b, g.bcs, g.bks);
+  const double pack = PACK_LAUNCH + 8.0 / PACK_BYTES_PER_CYCLE * static_cast<double>(K) *
+                                        static_cast<double>((ca != COPY_16 ? g.M : 0) + (cb != COPY_16 ? g.N : 0));
+  for (int x = 0; x < 2; ++x) {
+    for (F32Tile t : {T64X64, T32X32, T32X16}) {
+      auto offer = [&](Choice* c, F32Copy a, F32Copy b, double more) {
+        const double cost = (f32_cost(t, x, x ? g.N : g.M, x ? g.M : g.N, K, x ? b : a, x ? a : b, reads_c, sms) + more) *
+                            (x ? 1.01 : 1.0);
+        if (cost < c->cost) *c = Choice{cost, t, x != 0};
+      };
+      offer(&direct, ca, cb, 0.0);
+      if (ca != COPY_16 || cb != COPY_16) offer(&packed, COPY_16, COPY_16, pack);
     }
-    return best;
-  };
-  F32Tile tile = T32X32, tile_x = T32X32;
-  double direct = best_of(M, N, &tile);
-  const double exchanged = best_of(N, M, &tile_x);
-  if (exchanged < 0.97 * direct) {
-    std::swap(g.M, g.N);
-    std::swap(g.a, g.b);
-    std::swap(g.ars, g.bcs);
-    std::swap(g.aks, g.bks);
-    std::swap(g.crs, g.ccs);
-    direct = exchanged;
-    tile = tile_x;
   }
-  // Direct, on 4-byte copies of an operand that needs them, or packed, whichever the model finds
-  // cheaper: packing costs two passes over an operand and a launch, and pays from about 800 rows and
-  // columns up (4097 x 4095 x 4001 2.77 -> 2.40 ms; 1024^3 with both k-contiguous 77 -> 69 us).
-  const bool va = x_aligned(g.a, g.ars, g.aks), vb = x_aligned(g.b, g.bcs, g.bks);
-  const double penalty = kF32Tile[tile].unpacked * ((va ? 0 : 1) + (vb ? 0 : 1));
-  if (tile != T32X16 &&
-      (va && vb ? 0.0 : PACK_LAUNCH + pack_cost((va ? 0 : g.M) + (vb ? 0 : g.N), K)) <= penalty * direct) {
+  if (packed.cost < direct.cost && pool && (K + PACK - 1) / PACK <= 65535) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    F32Args p = g;
+    if (packed.exchanged) exchange_roles(&p);
+    const bool pa = copy_of(p.a, p.ars, p.aks) != COPY_16, pb = copy_of(p.b, p.bcs, p.bks) != COPY_16;
+    const int64_t la = pa ? (p.M + 127) / 128 * 128 : 0, lb = pb ? (p.N + 127) / 128 * 128 : 0;
     uint32_t* ws = nullptr;
-    const int64_t la = va ? 0 : (g.M + 127) / 128 * 128, lb = vb ? 0 : (g.N + 127) / 128 * 128;
-    bool ready = va && vb;
-    if (!ready && pool && (K + PACK - 1) / PACK <= 65535) {
-      // under capture the call keeps to the direct path (no allocation in the graph); so it does when
-      // the workspace cannot be had
-      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
-          cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(la + lb) * K * 4, pool, s) ==
-              cudaSuccess) {
-        PackJob jobs[2];
-        int n = 0;
-        int64_t most = 0;
-        auto pack = [&](const uint32_t*& p, int64_t& xs, int64_t& ks, int64_t X, uint32_t* dst, int64_t ld, int& pad) {
-          jobs[n++] = PackJob{p, xs, ks, X, dst, ld};
-          most = std::max(most, X);
-          p = dst;
-          xs = 1;
-          ks = ld;
-          pad = 1;
-        };
-        if (!va) pack(g.a, g.ars, g.aks, g.M, ws, la, g.pad_a);
-        if (!vb) pack(g.b, g.bcs, g.bks, g.N, ws + la * K, lb, g.pad_b);
-        const dim3 grid(static_cast<unsigned>((most + PACK - 1) / PACK), static_cast<unsigned>((K + PACK - 1) / PACK),
-                        static_cast<unsigned>(n));
-        GB_LAUNCH(GB_KERNEL_NATIVE_GEMM, s, (f32_pack_kernel<<<grid, 256, 0, s>>>(jobs[0], jobs[n - 1], K)));
-        ready = true;
-      } else {
-        cudaGetLastError();
-      }
-    }
-    if (ready) {
-      const int rc = launch_tile<false>(tile, g, op, sms, s);
-      if (ws) cudaFreeAsync(ws, s);
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+        cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(la + lb) * K * 4, pool, s) ==
+            cudaSuccess) {
+      PackJob jobs[2];
+      int n = 0;
+      int64_t most = 0;
+      auto job = [&](const uint32_t*& src, int64_t& xs, int64_t& ks, int64_t X, uint32_t* dst, int64_t ld, int& pad) {
+        jobs[n++] = PackJob{src, xs, ks, X, dst, ld};
+        most = std::max(most, X);
+        src = dst;
+        xs = 1;
+        ks = ld;
+        pad = 1;
+      };
+      if (pa) job(p.a, p.ars, p.aks, p.M, ws, la, p.pad_a);
+      if (pb) job(p.b, p.bcs, p.bks, p.N, ws + la * K, lb, p.pad_b);
+      const dim3 grid(static_cast<unsigned>((most + PACK - 1) / PACK), static_cast<unsigned>((K + PACK - 1) / PACK),
+                      static_cast<unsigned>(n));
+      GB_LAUNCH(GB_KERNEL_NATIVE_GEMM, s, (f32_pack_kernel<<<grid, 256, 0, s>>>(jobs[0], jobs[n - 1], K)));
+      const int rc = launch_tile<false>(packed.tile, p, op, sms, s);
+      cudaFreeAsync(ws, s);
       return rc;
     }
+    cudaGetLastError();
   }
-  return launch_tile<true>(tile, g, op, sms, s);
+  if (direct.exchanged) exchange_roles(&g);
+  return ca == COPY_16 && cb == COPY_16 ? launch_tile<false>(direct.tile, g, op, sms, s)
+                                        : launch_tile<true>(direct.tile, g, op, sms, s);
 }
 
 int native_gemm_f32(int ta, int tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A, int64_t lda,
@@ -232,7 +252,7 @@ int native_gemm_f32(int ta, int tb, int64_t M, int64_t N, int64_t K, float alpha
   const F32Args g{M, N, K, reinterpret_cast<const uint32_t*>(A), ta ? lda : 1, ta ? 1 : lda,
                   reinterpret_cast<const uint32_t*>(B), tb ? ldb : 1, tb ? 1 : ldb, reinterpret_cast<uint32_t*>(C), 1,
                   ldc, 0, 0};
-  return f32_run(g, F32Chain{alpha, beta}, sms, pool, s);
+  return f32_run(g, F32Chain{alpha, beta}, beta != 0.0f, sms, pool, s);
 }
 
 int native_kernel_onto_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B, int64_t ldb,
@@ -241,7 +261,7 @@ int native_kernel_onto_f32(int64_t M, int64_t N, int64_t K, const float* A, int6
   if ((M + 63) / 64 > 0x7FFFFFFF || (N + 63) / 64 > 65535) return GB_ERR_UNSUPPORTED;
   const F32Args g{M, N, K, reinterpret_cast<const uint32_t*>(A), 1, lda, reinterpret_cast<const uint32_t*>(B), 1, ldb,
                   reinterpret_cast<uint32_t*>(C), 1, ldc, 0, 0};
-  return f32_run(g, F32Onto{}, sms, pool, s);
+  return f32_run(g, F32Onto{}, true, sms, pool, s);
 }
 
 }  // namespace gb
