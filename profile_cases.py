@@ -17,7 +17,7 @@ cases:
   ozaki_crt_1panel, ozaki_crt_auto_1panel
                  the same in one panel: every kernel once per call, on the caller's stream
   grouped_f64    gb_gemm_grouped_f64, 4096 problems with m, n, k log-uniform in [8, 512]
-  grouped_f32    the same problems in FP32 (default configuration: tiles chosen per problem)
+  grouped_f32    the same problems in FP32 (default configuration)
   adjoint        gb_gemm_adjoint_f32, A 4096 x 2048, B 2048 x 4096
   semiring_f32   gb_gemm_semiring_f32 (min, +), 4096^3
   f32_bf16x3     gb_gemm_f32_ex BF16X3 (term split, 3 term products), 4096^3
