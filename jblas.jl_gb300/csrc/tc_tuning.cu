@@ -166,6 +166,7 @@ int tc_autotune(int kind, int64_t M, int64_t N, int64_t K, int reps, TcTuning* o
   };
   // the adjoint writes dA over D as well as dB: both outputs share D's storage here, which only
   // the timing sees (the operands stay A, B, C)
+
   // A launch of FP32 outputs on pairs that cuts tiles has a band of its own: one candidate for all of them.
   int device = 0, sms = 0;
   GB_CUDA_TRY(cudaGetDevice(&device));
