@@ -45,6 +45,14 @@ __host__ __device__ constexpr TileCfg tile_cfg(int c) {
        : c == 8 ? TileCfg{128, 32}
                 : TileCfg{32, 128};
 }
+// ceil(x / d) for a tile extent, a power of two: without the division of 64 bits.
+__host__ __device__ inline int64_t tiles_along(int64_t x, int d) {
+#ifdef __CUDA_ARCH__
+  return (x + d - 1) >> (31 - __clz(d));
+#else
+  return (x + d - 1) / d;
+#endif
+}
 constexpr int GROUPED_CONFIGS_F64 = 4;
 constexpr int GROUPED_CONFIGS_F32 = 10;
 
@@ -72,9 +80,9 @@ struct F64Tiles {
 __host__ __device__ inline F64Tiles f64_tiles(const TileCfg& c, int64_t m, int64_t n) {
   if (m <= 0 || n <= 0) return F64Tiles{0, 0, 0, 0};
   if (m > 0x7FFFFFFF - 64 || n > 0x7FFFFFFF - 64)
-    return F64Tiles{static_cast<int>((m + c.bm - 1) / c.bm), static_cast<int>((n + 15) / 16), c.bm, 16};
+    return F64Tiles{static_cast<int>(tiles_along(m, c.bm)), static_cast<int>((n + 15) / 16), c.bm, 16};
   const uint32_t m32 = static_cast<uint32_t>(m), n32 = static_cast<uint32_t>(n);
-  const uint32_t tm = (m32 + c.bm - 1) / c.bm, fm = (m32 + tm - 1) / tm;
+  const uint32_t tm = static_cast<uint32_t>(tiles_along(m, c.bm)), fm = (m32 + tm - 1) / tm;
   const uint32_t room = F64_MAX_ELEMS / fm, most = c.bn < 32 ? c.bn : 32, width = room < most ? room : most;
   const uint32_t tn = (n32 + width - 1) / width, fn = (n32 + tn - 1) / tn;
   return F64Tiles{static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(fm), static_cast<int>(fn)};
@@ -173,7 +181,7 @@ __device__ __forceinline__ int unpacked_config(const gb_grouped_tuning_t& tuning
 
 __device__ __forceinline__ long long tile_count(const gb_problem_t& p, const TileCfg& c, bool f32) {
   if (p.m <= 0 || p.n <= 0) return 0;
-  if (f32) return ((p.m + c.bm - 1) / c.bm) * ((p.n + c.bn - 1) / c.bn);
+  if (f32) return tiles_along(p.m, c.bm) * tiles_along(p.n, c.bn);
   const F64Tiles t = f64_tiles(c, p.m, p.n);
   return static_cast<long long>(t.tm) * t.tn;
 }
@@ -194,6 +202,13 @@ __device__ __forceinline__ int choice_bucket(int word, bool small) { return word
 // The order inside a bucket depends on timing, which changes no result (each tile is
 // independent).  Each problem's choice is made once: made again for the histogram, the order and with
 // 64-bit divisions it was a third of a call on 4000 FP64 problems of 8^3 (65 us, now 45).
+// The block has a thread per problem, up to 1024 (grouped_prefix_threads): the sums and the scan take every
+// warp through their shuffles and barriers, which is most of the time of a small table.
+static int grouped_prefix_threads(int count) {
+  int threads = 32;
+  while (threads < count && threads < 1024) threads *= 2;
+  return threads;
+}
 __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_problem_t* __restrict__ probs, int count,
                                                               gb_grouped_tuning_t tuning, bool f32, int sms,
                                                               long long large_elems, long long* __restrict__ ws) {
@@ -203,7 +218,7 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   long long* offsets = ws;
   int* words = reinterpret_cast<int*>(ws);
   int* order = reinterpret_cast<int*>(grouped_order_words(ws, count));
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, threads = static_cast<int>(blockDim.x);
   const bool packed = count <= GROUPED_PACK_LIMIT;   // (a longer table keeps the choice for enough work)
   if (t < 32) hist[t] = 0;
   auto bucket = [](long long held, int64_t k) {
@@ -217,7 +232,7 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   };
   const bool may_be_small = f32 ? packed : f64_may_be_small(count, sms);
   F64Load chosen, least;
-  for (int i = t; i < count; i += 1024) {
+  for (int i = t; i < count; i += threads) {
     const gb_problem_t& p = probs[i];
     const int c = config_of(tuning, size_class(p.m, p.n));
     if (f32) {
@@ -258,32 +273,37 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
     sums[3][t >> 5] = least.longest;
   }
   __syncthreads();
-  chosen.total = sums[0][t & 31];
-  chosen.longest = sums[1][t & 31];
-  least.total = sums[2][t & 31];
-  least.longest = sums[3][t & 31];
+  if (threads > 32) {
+    const bool there = (t & 31) < threads / 32;
+    chosen.total = there ? sums[0][t & 31] : 0;
+    chosen.longest = there ? sums[1][t & 31] : 0;
+    least.total = there ? sums[2][t & 31] : 0;
+    least.longest = there ? sums[3][t & 31] : 0;
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    combine(chosen, off);
-    combine(least, off);
-  }
-  const bool small = may_be_small && (f32 ? chosen.total < large_elems : f64_small(chosen, least, sms));
-  for (int i = t; i < count; i += 1024) atomicAdd(&hist[choice_bucket(words[i], small)], 1);
-  __syncthreads();
-  if (t == 0) {
-    int run = 0;
-    for (int b = 0; b < 32; ++b) {
-      start[b] = run;
-      run += hist[b];
+    for (int off = 16; off > 0; off >>= 1) {
+      combine(chosen, off);
+      combine(least, off);
     }
   }
+  const bool small = may_be_small && (f32 ? chosen.total < large_elems : f64_small(chosen, least, sms));
+  for (int i = t; i < count; i += threads) atomicAdd(&hist[choice_bucket(words[i], small)], 1);
   __syncthreads();
-  for (int i = t; i < count; i += 1024) {
+  if (t < 32) {   // exclusive prefix sums over the 32 buckets
+    int run = hist[t];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, run, off);
+      if (t >= off) run += v;
+    }
+    start[t] = run - hist[t];
+  }
+  __syncthreads();
+  for (int i = t; i < count; i += threads) {
     const int w = words[i];
     order[atomicAdd(&start[choice_bucket(w, small)], 1)] = grouped_order_entry(i, choice_config(w, small), count);
   }
   __syncthreads();
-  const int per = (count + 1023) / 1024;
+  const int per = (count + threads - 1) / threads;
   const int b = t * per, e = min(count, b + per);
   auto tiles_of = [&](int pos) -> long long {
     const int e = order[pos];
@@ -294,7 +314,7 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   for (int i = b; i < e; ++i) sum += tiles_of(i);
   part[t] = sum;
   __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {   // inclusive Hillis-Steele scan of the parts
+  for (int off = 1; off < threads; off <<= 1) {   // inclusive Hillis-Steele scan of the parts
     const long long v = (t >= off) ? part[t - off] : 0;
     __syncthreads();
     part[t] += v;
@@ -303,9 +323,9 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   long long run = (t == 0) ? 0 : part[t - 1];
   for (int i = b; i < e; ++i) {
     offsets[i] = run;   // offsets[0] = 0: the tile counter's start
-    run += tiles_of(i);
+    if (i + 1 < e) run += tiles_of(i);
   }
-  if (t == 1023) offsets[count] = part[1023];
+  if (t == threads - 1) offsets[count] = part[t];
 }
 
 // The schedule position of tile w: the last pos with offsets[pos] <= w (problems without
@@ -351,7 +371,7 @@ __device__ __forceinline__ void grouped_find(const gb_problem_t* __restrict__ pr
   t.c = tile_cfg(packed ? (e >> 24) : unpacked_config(tuning, t.p, f32));
   // in 32-bit arithmetic (a problem's tile count is below 2^31); the first problem's tiles start at 0
   const int local = static_cast<int>(lo ? w - offsets[lo] : w);
-  const int tiles_m = static_cast<int>((t.p.m + t.c.bm - 1) / t.c.bm);
+  const int tiles_m = static_cast<int>(tiles_along(t.p.m, t.c.bm));
   const int tn = local / tiles_m;
   t.tm = local - tn * tiles_m;
   t.tn = tn;
@@ -380,13 +400,15 @@ __device__ __forceinline__ void grouped_loop(const gb_problem_t* __restrict__ pr
   const long long total = offsets[count];
   int lo = 0, slot = 0;
   const unsigned skip = gridDim.x / GROUPED_CTAS;
+  const bool one_each = total <= gridDim.x;   // nothing to hand out
   for (long long w = blockIdx.x + (blockIdx.x < skip ? gridDim.x : 0) - skip; w < total; slot ^= 1) {
     long long next = 0;
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0 && !one_each)
       next = gridDim.x + static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(ws), 1ull));
     GroupedTile t;
     grouped_find(probs, count, tuning, f32, offsets, order, w, lo, t);
     run(t, w);
+    if (one_each) return;
     if (threadIdx.x == 0) next_tile[slot] = next;
     __syncthreads();
     w = next_tile[slot];
@@ -487,7 +509,7 @@ int grouped_launch(int dtype_bytes, const gb_problem_t* d_probs, int count, cons
                    long long* d_offsets, int sms, cudaStream_t s) {
   if (count <= 0) return GB_OK;
   GB_LAUNCH(GB_KERNEL_GROUPED_GEMM, s,
-            (grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, tuning, dtype_bytes == 4, sms,
+            (grouped_prefix_kernel<<<1, grouped_prefix_threads(count), 0, s>>>(d_probs, count, tuning, dtype_bytes == 4, sms,
                                                       f32_large_elems(sms), d_offsets)));
   GB_CUDA_TRY(cudaGetLastError());
   return launch_tiles(dtype_bytes, d_probs, count, tuning, d_offsets, sms, s);
@@ -629,7 +651,7 @@ int grouped_f64_noalloc(const gb_problem_t* d_probs, int count, const gb_grouped
   // clearing.
   // Launched directly, not through the timing hooks (which create CUDA events while profiling
   // is on); gb_launch_counts still counts both launches.
-  grouped_prefix_kernel<<<1, 1024, 0, s>>>(d_probs, count, t, false, sms, 0, offsets);
+  grouped_prefix_kernel<<<1, grouped_prefix_threads(count), 0, s>>>(d_probs, count, t, false, sms, 0, offsets);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return gb_set_cuda_error(e, "grouped prologue launch");
   prof_count(GB_KERNEL_GROUPED_GEMM);
