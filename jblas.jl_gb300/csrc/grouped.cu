@@ -203,7 +203,9 @@ __device__ __forceinline__ int choice_bucket(int word, bool small) { return word
 // independent).  Each problem's choice is made once: made again for the histogram, the order and with
 // 64-bit divisions it was a third of a call on 4000 FP64 problems of 8^3 (65 us, now 45).
 // The block has a thread per problem, up to 1024 (grouped_prefix_threads): the sums and the scan take every
-// warp through their shuffles and barriers, which is most of the time of a small table.
+// warp through their shuffles and barriers, which was most of the time of a small table (10 FP64 problems
+// 8.8 us with 1024 threads, 6.1 with 32; a whole call 17.4, 14.5).  What is left there is latency: table
+// loads, the choices' 32-bit divisions, two rounds of atomics.
 static int grouped_prefix_threads(int count) {
   int threads = 32;
   while (threads < count && threads < 1024) threads *= 2;
@@ -212,8 +214,8 @@ static int grouped_prefix_threads(int count) {
 __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_problem_t* __restrict__ probs, int count,
                                                               gb_grouped_tuning_t tuning, bool f32, int sms,
                                                               long long large_elems, long long* __restrict__ ws) {
-  __shared__ long long part[1024];
   __shared__ long long sums[4][32];
+  __shared__ bool small_table;
   __shared__ int hist[32], start[32];
   long long* offsets = ws;
   int* words = reinterpret_cast<int*>(ws);
@@ -257,35 +259,38 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
       words[i] = choice_word(a, bucket(ta.fm * ta.fn, p.k), b, bucket_b);
     }
   }
-  auto combine = [](F64Load& l, int off) {
-    l.total += __shfl_xor_sync(0xffffffffu, l.total, off);
-    l.longest = max(l.longest, __shfl_xor_sync(0xffffffffu, l.longest, off));
-  };
+  // The sums over the block, where the choice needs them, in two steps: a warp each, then the first warp.
+  bool small = false;
+  if (may_be_small) {
+    auto combine = [](F64Load& l) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    combine(chosen, off);
-    combine(least, off);
-  }
-  if ((t & 31) == 0) {
-    sums[0][t >> 5] = chosen.total;
-    sums[1][t >> 5] = chosen.longest;
-    sums[2][t >> 5] = least.total;
-    sums[3][t >> 5] = least.longest;
-  }
-  __syncthreads();
-  if (threads > 32) {
-    const bool there = (t & 31) < threads / 32;
-    chosen.total = there ? sums[0][t & 31] : 0;
-    chosen.longest = there ? sums[1][t & 31] : 0;
-    least.total = there ? sums[2][t & 31] : 0;
-    least.longest = there ? sums[3][t & 31] : 0;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      combine(chosen, off);
-      combine(least, off);
+      for (int off = 16; off > 0; off >>= 1) {
+        l.total += __shfl_xor_sync(0xffffffffu, l.total, off);
+        l.longest = max(l.longest, __shfl_xor_sync(0xffffffffu, l.longest, off));
+      }
+    };
+    combine(chosen);
+    if (!f32) combine(least);
+    if ((t & 31) == 0) {
+      sums[0][t >> 5] = chosen.total;
+      sums[1][t >> 5] = chosen.longest;
+      sums[2][t >> 5] = least.total;
+      sums[3][t >> 5] = least.longest;
+    }
+    __syncthreads();
+    if (t < 32) {
+      const bool there = t < threads / 32;
+      chosen.total = there ? sums[0][t] : 0;
+      chosen.longest = there ? sums[1][t] : 0;
+      least.total = there ? sums[2][t] : 0;
+      least.longest = there ? sums[3][t] : 0;
+      combine(chosen);
+      if (!f32) combine(least);
+      if (t == 0) small_table = f32 ? chosen.total < large_elems : f64_small(chosen, least, sms);
     }
   }
-  const bool small = may_be_small && (f32 ? chosen.total < large_elems : f64_small(chosen, least, sms));
+  __syncthreads();
+  if (may_be_small) small = small_table;
   for (int i = t; i < count; i += threads) atomicAdd(&hist[choice_bucket(words[i], small)], 1);
   __syncthreads();
   if (t < 32) {   // exclusive prefix sums over the 32 buckets
@@ -312,20 +317,27 @@ __global__ void __launch_bounds__(1024, 1) grouped_prefix_kernel(const gb_proble
   };
   long long sum = 0;
   for (int i = b; i < e; ++i) sum += tiles_of(i);
-  part[t] = sum;
+  // inclusive scan over the block: inside each warp, then over the warps' totals
+  auto scan = [&](long long v) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const long long u = __shfl_up_sync(0xffffffffu, v, off);
+      if ((t & 31) >= off) v += u;
+    }
+    return v;
+  };
+  const long long in_warp = scan(sum);
+  if ((t & 31) == 31) sums[0][t >> 5] = in_warp;
   __syncthreads();
-  for (int off = 1; off < threads; off <<= 1) {   // inclusive Hillis-Steele scan of the parts
-    const long long v = (t >= off) ? part[t - off] : 0;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  long long run = (t == 0) ? 0 : part[t - 1];
+  if (t < 32) sums[1][t] = scan(t < threads / 32 ? sums[0][t] : 0);
+  __syncthreads();
+  const long long end = in_warp + (t >= 32 ? sums[1][(t >> 5) - 1] : 0);
+  long long run = end - sum;
   for (int i = b; i < e; ++i) {
     offsets[i] = run;   // offsets[0] = 0: the tile counter's start
     if (i + 1 < e) run += tiles_of(i);
   }
-  if (t == threads - 1) offsets[count] = part[t];
+  if (t == threads - 1) offsets[count] = end;
 }
 
 // The schedule position of tile w: the last pos with offsets[pos] <= w (problems without
